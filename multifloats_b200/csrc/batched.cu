@@ -110,8 +110,7 @@ __global__ void __launch_bounds__(256, 2)
     if (w >= nitems) break;
     const PItem it = items[w];
     const PProb p = probs[it.prob];
-    gtile::cgemm_tile<ALIGNED>(p.A, p.B, p.C, p.m, p.k, p.n, ri, (int64_t)it.tm * gtile::kCBM,
-                               (int64_t)it.tn * gtile::kCBN, sm);
+    gtile::cgemm_tile<2, 2, ALIGNED>(p.A, p.B, p.C, p.m, p.k, p.n, ri, (int64_t)it.tm * 32, (int64_t)it.tn * 32, sm);
   }
 }
 
@@ -679,7 +678,7 @@ static int create_plain(const mfcuda_gemm_desc *d, int64_t count, int64_t ri, co
     probs[p] = {static_cast<const double *>(d[p].a), static_cast<const double *>(d[p].b),
                 static_cast<double *>(d[p].c), d[p].m, d[p].k, d[p].n};
   for (int64_t p : order) {
-    const int e = complex ? gtile::kCBM : cfg_edge(cfg[p]);
+    const int e = complex ? 32 : cfg_edge(cfg[p]);
     for (int64_t tn = 0; tn < (d[p].n + e - 1) / e; ++tn)
       for (int64_t tm = 0; tm < (d[p].m + e - 1) / e; ++tm)
         items.push_back({(int)p, complex ? 1 : cfg[p], (int)tm, (int)tn});

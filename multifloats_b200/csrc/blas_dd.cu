@@ -159,7 +159,11 @@ int launch_scale(double *C, int64_t ldc, int64_t M, int64_t N, dd beta, int zero
 // ---- wgemm tile kernel ---------------------------------------------------------
 constexpr int kWThreads = 256;
 constexpr int kWTile = 64;  // 16 x 4 outputs per tile edge
-constexpr int kWK = gtile::kBK;
+constexpr int kWK = 8;
+struct WgemmSmem {
+  double2 A[2][kWK][64];
+  double2 B[2][kWK][64];
+};
 enum { BETA_ZERO = 0, BETA_ONE = 1, BETA_OTHER = 2 };
 
 // The 16 accumulator chains of a thread use the branch-free operator forms so
@@ -171,7 +175,7 @@ __global__ void __launch_bounds__(kWThreads, TA ? 1 : 2)
     wgemm_kernel(const double *__restrict__ A, int64_t lda, const double *__restrict__ B,
                  int64_t ldb, double *__restrict__ C, int64_t ldc, int64_t M, int64_t N, int64_t K,
                  dd alpha, dd beta, int beta_mode) {
-  __shared__ __align__(16) gtile::Smem sm;
+  __shared__ __align__(16) WgemmSmem sm;
   const int t = threadIdx.x, tx = t % 16, ty = t / 16;
   const int64_t m0 = (int64_t)blockIdx.x * kWTile, n0 = (int64_t)blockIdx.y * kWTile;
 

@@ -12,11 +12,12 @@
 // rr, ii, ri, ir accumulated side by side, then re = rr - ii, im = ri + ir with
 // the DD operators.
 //
-// Tiling: a 256-thread CTA owns a BM x BN output tile; each thread owns a
-// TM x TN register tile of (s_hi, s_lo) accumulators.  A and B k-slices of
-// depth BK are staged in shared memory with cp.async (16-byte copies,
-// zero-filled past the matrix edge) in a two-stage ring.  Bound: FP64 pipe,
-// 13 FP64 instructions per MAC plus 6 per renormalisation.
+// Tiling: a 256-thread CTA owns a square output tile of edge 64, 32 or 16 (32
+// or 16 complex); each thread owns a register tile of (s_hi, s_lo)
+// accumulators.  A and B k-slices are staged in shared memory with cp.async
+// (16-byte copies, zero-filled past the matrix edge) in a two-stage ring.
+// Bound: FP64 pipe, 13 FP64 instructions per MAC plus 6 per renormalisation.
+// Which tiles a product is cut into is decided by pick_tiles.
 #include <mutex>
 
 #include "common.cuh"
@@ -30,32 +31,140 @@ using gtile::cp_async_commit;
 using gtile::cp_async_wait_all;
 
 // ---------------------------------------------------------------------------
-// Real GEMM: one 64 x 64 tile per CTA (4 x 4 outputs per thread).
+// Cutting a product into tiles.  The k loop of an output cannot be split (the
+// MAC order is fixed), so a product fills the chip only by its output tiles,
+// and the SM that gets one tile more than the others sets the time.  A tile
+// of edge E costs (start + n per_tile) k for the n tiles of the busiest SM,
+// measured at k = 1024 on 148 SMs (in units of 0.1 ns per step: real tiles
+// of 64 / 32 / 16: 300 + 5000 n, 150 + 1320 n, 110 + 385 n; complex tiles of
+// 32 / 16: 300 + 5100 n, 270 + 1335 n): a small tile loses 5-20 % per MAC but
+// quantises better.  Candidates: every tile of one edge, or the largest edge
+// for the whole rounds over the SMs and the remaining tiles cut into 4 or 16
+// (run at the large tile's two CTAs per SM: 1390 / 433, complex 1460).  The
+// cheapest one is launched.  256^3: 16 tiles of 64 took 180 us, 256 of 16
+// take 25 us; 1531 x 977 x 1203: 456 tiles of 64 took 2.34 ms, 444 of them and
+// 192 of 16 take 1.56 ms.
 // ---------------------------------------------------------------------------
 constexpr int kThreads = gtile::kThreads;
-constexpr int kTM = 4, kTN = 4;
-constexpr int kBM = 16 * kTM, kBN = 16 * kTN;
 
-template <bool ALIGNED>
-__global__ void __launch_bounds__(kThreads, 2)
-    gemm_dd_kernel(const double *__restrict__ A, const double *__restrict__ B,
-                   double *__restrict__ C, int64_t M, int64_t K, int64_t N, int64_t ri) {
-  __shared__ gtile::Smem sm;
-  gtile::gemm_tile<kTM, kTN, ALIGNED>(A, B, C, M, K, N, ri, (int64_t)blockIdx.x * kBM,
-                                      (int64_t)blockIdx.y * kBN, sm);
+struct TilePick {
+  int edge;        // of the uniform tiles, or of the whole ones
+  int64_t blocks;  // grid
+  int64_t whole;   // mixed: this many whole tiles, then the rest cut into `cut` pieces
+  int cut;         // 0: uniform
+};
+struct TileCost {
+  int64_t start, per_tile;
+};
+// Tiles of the edges 16 TMAX, 8 TMAX, ... 16 with their costs, largest first.
+static TilePick pick_tiles(int64_t m, int64_t n, const TileCost *cost, int nedges, const int64_t *cut_cost) {
+  const int64_t sms = sm_count();
+  auto tiles = [&](int e) { return ((m + e - 1) / e) * ((n + e - 1) / e); };
+  const int top = 16 << (nedges - 1);
+  TilePick best = {0, 0, 0, 0};
+  int64_t best_cost = INT64_MAX;
+  for (int i = 0; i < nedges; ++i) {
+    const int64_t t = tiles(top >> i), c = cost[i].start + (t + sms - 1) / sms * cost[i].per_tile;
+    if (c < best_cost && t <= INT32_MAX) {
+      best_cost = c;
+      best = {top >> i, t, 0, 0};
+    }
+  }
+  const int64_t t = tiles(top), rounds = t / sms, rest = t % sms;
+  for (int i = 1; i < nedges && rounds > 0 && rest > 0; ++i) {
+    const int64_t pieces = rest << (2 * i);
+    const int64_t c = cost[0].start + rounds * cost[0].per_tile + (pieces + sms - 1) / sms * cut_cost[i - 1];
+    if (c < best_cost && t <= INT32_MAX) {
+      best_cost = c;
+      best = {top, rounds * sms + pieces, rounds * sms, 1 << (2 * i)};
+    }
+  }
+  return best;
+}
+constexpr TileCost kRealCost[3] = {{300, 5000}, {150, 1320}, {110, 385}};
+constexpr int64_t kRealCutCost[2] = {1390, 433};
+constexpr TileCost kCplxCost[2] = {{300, 5100}, {270, 1335}};
+constexpr int64_t kCplxCutCost[1] = {1460};
+
+// Origin of block b's tile among tiles of edge E, gx of them along M.
+__device__ __forceinline__ void tile_origin(int64_t b, int64_t gx, int E, int64_t &m0, int64_t &n0) {
+  m0 = b % gx * E;
+  n0 = b / gx * E;
+}
+// Piece q of the tile at (m0, n0) cut into side x side pieces of edge E.
+__device__ __forceinline__ void piece_origin(int q, int side, int E, int64_t &m0, int64_t &n0) {
+  m0 += q % side * E;
+  n0 += q / side * E;
 }
 
 // ---------------------------------------------------------------------------
-// Complex GEMM: one 32 x 32 tile per CTA (gtile::cgemm_tile).
+// Real GEMM.  Mixed: blocks 0 .. whole - 1 own a 64 x 64 tile (4 x 4 outputs
+// per thread), the others a piece of the tiles after those.
 // ---------------------------------------------------------------------------
-constexpr int kCBM = gtile::kCBM, kCBN = gtile::kCBN;
+template <bool ALIGNED>
+__global__ void __launch_bounds__(kThreads, 2)
+    gemm_dd_kernel(const double *__restrict__ A, const double *__restrict__ B,
+                   double *__restrict__ C, int64_t M, int64_t K, int64_t N, int64_t ri,
+                   int64_t whole, int cut) {
+  __shared__ gtile::Smem sm;
+  const int64_t gx = (M + 63) / 64;
+  int64_t b = blockIdx.x, m0, n0;
+  if (b < whole) {
+    tile_origin(b, gx, 64, m0, n0);
+    gtile::gemm_tile<4, 4, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+    return;
+  }
+  b -= whole;
+  const int q = (int)(b % cut);
+  tile_origin(whole + b / cut, gx, 64, m0, n0);
+  if (cut == 4) {
+    piece_origin(q, 2, 32, m0, n0);
+    if (m0 < M && n0 < N) gtile::gemm_tile<2, 2, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+  } else {
+    piece_origin(q, 4, 16, m0, n0);
+    if (m0 < M && n0 < N) gtile::gemm_tile<1, 1, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+  }
+}
+// Uniform tiles of edge 16 T (three CTAs of edge 32 per SM, four of edge 16).
+template <int T, bool ALIGNED>
+__global__ void __launch_bounds__(kThreads, T == 2 ? 3 : 4)
+    gemm_dd_small_kernel(const double *__restrict__ A, const double *__restrict__ B,
+                         double *__restrict__ C, int64_t M, int64_t K, int64_t N, int64_t ri) {
+  __shared__ gtile::Smem sm;
+  int64_t m0, n0;
+  tile_origin(blockIdx.x, (M + 16 * T - 1) / (16 * T), 16 * T, m0, n0);
+  gtile::gemm_tile<T, T, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+}
 
+// ---------------------------------------------------------------------------
+// Complex GEMM (gtile::cgemm_tile): the same with tiles of 32 and 16.
+// ---------------------------------------------------------------------------
 template <bool ALIGNED>
 __global__ void __launch_bounds__(kThreads, 2)
     cgemm_dd_kernel(const double *__restrict__ A, const double *__restrict__ B,
-                    double *__restrict__ C, int64_t M, int64_t K, int64_t N, int64_t ri) {
+                    double *__restrict__ C, int64_t M, int64_t K, int64_t N, int64_t ri,
+                    int64_t whole, int cut) {
   __shared__ gtile::CSmem sm;
-  gtile::cgemm_tile<ALIGNED>(A, B, C, M, K, N, ri, (int64_t)blockIdx.x * kCBM, (int64_t)blockIdx.y * kCBN, sm);
+  const int64_t gx = (M + 31) / 32;
+  int64_t b = blockIdx.x, m0, n0;
+  if (b < whole) {
+    tile_origin(b, gx, 32, m0, n0);
+    gtile::cgemm_tile<2, 2, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+    return;
+  }
+  b -= whole;
+  tile_origin(whole + b / cut, gx, 32, m0, n0);
+  piece_origin((int)(b % cut), 2, 16, m0, n0);
+  if (m0 < M && n0 < N) gtile::cgemm_tile<1, 1, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+}
+template <bool ALIGNED>
+__global__ void __launch_bounds__(kThreads, 4)
+    cgemm_dd_small_kernel(const double *__restrict__ A, const double *__restrict__ B,
+                          double *__restrict__ C, int64_t M, int64_t K, int64_t N, int64_t ri) {
+  __shared__ gtile::CSmem sm;
+  int64_t m0, n0;
+  tile_origin(blockIdx.x, (M + 15) / 16, 16, m0, n0);
+  gtile::cgemm_tile<1, 1, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -321,6 +430,27 @@ static int zero_fill(double *p, int64_t ndoubles, cudaStream_t s) {
   return MFCUDA_OK;
 }
 
+template <bool ALIGNED>
+static void launch_gemm(const TilePick &p, const double *A, const double *B, double *C, int64_t m, int64_t k,
+                        int64_t n, int64_t ri, cudaStream_t s) {
+  const unsigned g = (unsigned)p.blocks;
+  if (p.edge == 64)
+    gemm_dd_kernel<ALIGNED><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri, p.cut ? p.whole : p.blocks, p.cut);
+  else if (p.edge == 32)
+    gemm_dd_small_kernel<2, ALIGNED><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
+  else
+    gemm_dd_small_kernel<1, ALIGNED><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
+}
+template <bool ALIGNED>
+static void launch_cgemm(const TilePick &p, const double *A, const double *B, double *C, int64_t m, int64_t k,
+                         int64_t n, int64_t ri, cudaStream_t s) {
+  const unsigned g = (unsigned)p.blocks;
+  if (p.edge == 32)
+    cgemm_dd_kernel<ALIGNED><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri, p.cut ? p.whole : p.blocks, p.cut);
+  else
+    cgemm_dd_small_kernel<ALIGNED><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
+}
+
 int gemm_dev(const float64x2 *a, const float64x2 *b, float64x2 *c, int64_t m, int64_t k,
              int64_t n, int64_t ri, cudaStream_t s) {
   if (!shape_ok(m, k, n, sizeof(float64x2))) return MFCUDA_ERR_INVALID_ARG;
@@ -331,13 +461,13 @@ int gemm_dev(const float64x2 *a, const float64x2 *b, float64x2 *c, int64_t m, in
   if (k == 0) return zero_fill(C, 2 * m * n, s);
   const double *A = reinterpret_cast<const double *>(a);
   const double *B = reinterpret_cast<const double *>(b);
-  int64_t gx = (m + kBM - 1) / kBM, gy = (n + kBN - 1) / kBN;
-  if (gy > 65535) return MFCUDA_ERR_UNSUPPORTED;
-  dim3 grid((unsigned)gx, (unsigned)gy);
+  if ((n + 63) / 64 > 65535) return MFCUDA_ERR_UNSUPPORTED;
+  const TilePick p = pick_tiles(m, n, kRealCost, 3, kRealCutCost);
+  if (p.blocks <= 0 || p.blocks > INT32_MAX) return MFCUDA_ERR_UNSUPPORTED;
   if (aligned16(a, b, c))
-    gemm_dd_kernel<true><<<grid, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
+    launch_gemm<true>(p, A, B, C, m, k, n, ri, s);
   else
-    gemm_dd_kernel<false><<<grid, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
+    launch_gemm<false>(p, A, B, C, m, k, n, ri, s);
   MF_TRY_CUDA(cudaGetLastError());
   return MFCUDA_OK;
 }
@@ -352,13 +482,13 @@ int cgemm_dev(const complex64x2 *a, const complex64x2 *b, complex64x2 *c, int64_
   if (k == 0) return zero_fill(C, 4 * m * n, s);
   const double *A = reinterpret_cast<const double *>(a);
   const double *B = reinterpret_cast<const double *>(b);
-  int64_t gx = (m + kCBM - 1) / kCBM, gy = (n + kCBN - 1) / kCBN;
-  if (gy > 65535) return MFCUDA_ERR_UNSUPPORTED;
-  dim3 grid((unsigned)gx, (unsigned)gy);
+  if ((n + 31) / 32 > 65535) return MFCUDA_ERR_UNSUPPORTED;
+  const TilePick p = pick_tiles(m, n, kCplxCost, 2, kCplxCutCost);
+  if (p.blocks <= 0 || p.blocks > INT32_MAX) return MFCUDA_ERR_UNSUPPORTED;
   if (aligned16(a, b, c))
-    cgemm_dd_kernel<true><<<grid, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
+    launch_cgemm<true>(p, A, B, C, m, k, n, ri, s);
   else
-    cgemm_dd_kernel<false><<<grid, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
+    launch_cgemm<false>(p, A, B, C, m, k, n, ri, s);
   MF_TRY_CUDA(cudaGetLastError());
   return MFCUDA_OK;
 }

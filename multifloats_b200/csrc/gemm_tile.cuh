@@ -5,8 +5,18 @@
 //
 // A 256-thread CTA owns a (16 TM) x (16 TN) tile; thread t owns rows
 // tx + 16 i (i < TM) and columns ty + 16 j (j < TN), tx = t % 16, ty = t / 16.
-// A and B k-slices of depth 8 go through a two-stage cp.async ring in shared
-// memory (zero-filled past the edges).
+// A and B k-slices go through a two-stage cp.async ring in shared memory
+// (zero-filled past the edges), deeper for smaller tiles (8, 16 or 32 steps),
+// so that a stage always holds about the same bytes and the small tiles do
+// not meet a barrier every few MACs.
+//
+// Bound: FP64 pipe, 13 instructions per MAC plus 6 per renormalisation, two
+// issue cycles each.  The steps run in branch-free groups of eight: with the
+// chunk counter tested after every step the accumulators had to sit in fixed
+// registers at each merge, and the moves that took (8 of 26 issue cycles per
+// MAC) were paid on top of the FP64 issue -- 4096^3 66.6 -> 56.8 ms, FP64 pipe
+// 88 % busy.  An interval that is not a multiple of eight runs from chunk end
+// to chunk end in a counted loop.
 #pragma once
 #include "dd_device.cuh"
 
@@ -44,20 +54,43 @@ __device__ __forceinline__ void load_dd(double2 *dst, const double *src, bool va
 
 
 constexpr int kThreads = 256;
-constexpr int kBK = 8;
-constexpr int kBMax = 64;  // largest tile edge (TM, TN <= 4)
+constexpr int kGroup = 8;  // steps of a branch-free group
 
-// Shared staging of the largest tile; smaller tiles use the first rows.
+// Depth of a stage for a tile of edge e: 8 steps of 64, 16 of 32, 32 of 16.
+__host__ __device__ constexpr int depth(int edge) { return 512 / edge; }
+// A row of the B stage is one entry longer than the tile: the threads of a
+// copy run along k, and without it eight of them meet in the same banks.
+__host__ __device__ constexpr int b_pitch(int bn) { return bn + 1; }
+
+// Staging of any tile (edges 16, 32, 64).
 struct Smem {
-  double2 A[2][kBK][kBMax];
-  double2 B[2][kBK][kBMax];
+  double2 A[2][512];
+  double2 B[2][depth(16) * b_pitch(16)];
+};
+
+// The renormalisation cadence: where the chunks of `ri` steps end.
+struct Cadence {
+  int64_t ri, cnt;   // interval (<= 0: no renormalisation), steps since the last one
+  bool grouped;      // the interval is none or a multiple of kGroup
+  __device__ __forceinline__ explicit Cadence(int64_t r) : ri(r), cnt(0), grouped(r <= 0 || r % kGroup == 0) {}
+  // steps until the chunk's end, at most `left`
+  __device__ __forceinline__ int run(int left) const {
+    return ri > 0 && ri - cnt < left ? (int)(ri - cnt) : left;
+  }
+  // `steps` more MACs done (never past a chunk's end): does a chunk end here?
+  __device__ __forceinline__ bool ends(int steps) {
+    if (ri <= 0 || (cnt += steps) != ri) return false;
+    cnt = 0;
+    return true;
+  }
 };
 
 template <int TM, int TN, bool ALIGNED>
 __device__ __forceinline__ void gemm_tile(const double *__restrict__ A, const double *__restrict__ B,
                                           double *__restrict__ C, int64_t M, int64_t K, int64_t N,
                                           int64_t ri, int64_t m0, int64_t n0, Smem &sm) {
-  constexpr int BM = 16 * TM, BN = 16 * TN;
+  constexpr int BM = 16 * TM, BN = 16 * TN, BK = depth(BM > BN ? BM : BN), PB = b_pitch(BN);
+  static_assert(BK * BM <= 512 && BK * PB <= depth(16) * b_pitch(16), "stage fits Smem");
   const int t = threadIdx.x;
   const int tx = t % 16, ty = t / 16;
 
@@ -69,64 +102,72 @@ __device__ __forceinline__ void gemm_tile(const double *__restrict__ A, const do
 
   auto issue = [&](int stage, int64_t k0) {
 #pragma unroll
-    for (int idx = t; idx < kBK * BM; idx += kThreads) {
+    for (int idx = t; idx < BK * BM; idx += kThreads) {
       int row = idx % BM, kk = idx / BM;
       int64_t gi = m0 + row, gk = k0 + kk;
       bool v = gi < M && gk < K;
-      load_dd<ALIGNED>(&sm.A[stage][kk][row], A + 2 * (gk * M + gi), v, A);
+      load_dd<ALIGNED>(&sm.A[stage][kk * BM + row], A + 2 * (gk * M + gi), v, A);
     }
 #pragma unroll
-    for (int idx = t; idx < kBK * BN; idx += kThreads) {
-      int kk = idx % kBK, col = idx / kBK;
+    for (int idx = t; idx < BK * BN; idx += kThreads) {
+      int kk = idx % BK, col = idx / BK;
       int64_t gj = n0 + col, gk = k0 + kk;
       bool v = gj < N && gk < K;
-      load_dd<ALIGNED>(&sm.B[stage][kk][col], B + 2 * (gj * K + gk), v, B);
+      load_dd<ALIGNED>(&sm.B[stage][kk * PB + col], B + 2 * (gj * K + gk), v, B);
     }
     cp_async_commit();
   };
+  auto step = [&](const double2 *as, const double2 *bs) {
+    double ah[TM], al[TM], bh[TN], bl[TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      double2 v = as[16 * i];
+      ah[i] = v.x;
+      al[i] = v.y;
+    }
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      double2 v = bs[16 * j];
+      bh[j] = v.x;
+      bl[j] = v.y;
+    }
+#pragma unroll
+    for (int j = 0; j < TN; ++j)
+#pragma unroll
+      for (int i = 0; i < TM; ++i) mfdev::mac(ah[i], al[i], bh[j], bl[j], s_hi[i][j], s_lo[i][j]);
+  };
+  auto renorm_all = [&]() {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) mfdev::renorm(s_hi[i][j], s_lo[i][j]);
+  };
 
-  const int64_t ntiles = (K + kBK - 1) / kBK;
-  int64_t cnt = 0;
+  const int64_t ntiles = (K + BK - 1) / BK;
+  Cadence cad(ri);
   if (ntiles > 0) issue(0, 0);
   for (int64_t kt = 0; kt < ntiles; ++kt) {
     const int stage = (int)(kt & 1);
     cp_async_wait_all();
     __syncthreads();
-    if (kt + 1 < ntiles) issue(stage ^ 1, (kt + 1) * kBK);
-    const int64_t k0 = kt * kBK;
-    const int kmax = (K - k0) < kBK ? (int)(K - k0) : kBK;
+    if (kt + 1 < ntiles) issue(stage ^ 1, (kt + 1) * BK);
+    const int64_t k0 = kt * BK;
+    const int kmax = (K - k0) < BK ? (int)(K - k0) : BK;
+    const double2 *as = sm.A[stage] + tx, *bs = sm.B[stage] + ty;
+    int kk = 0;
+    if (cad.grouped) {
+#pragma unroll 1
+      for (; kk + kGroup <= kmax; kk += kGroup) {
 #pragma unroll
-    for (int kk = 0; kk < kBK; ++kk) {
-      if (kk < kmax) {
-        double ah[TM], al[TM], bh[TN], bl[TN];
-#pragma unroll
-        for (int i = 0; i < TM; ++i) {
-          double2 v = sm.A[stage][kk][tx + 16 * i];
-          ah[i] = v.x;
-          al[i] = v.y;
-        }
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          double2 v = sm.B[stage][kk][ty + 16 * j];
-          bh[j] = v.x;
-          bl[j] = v.y;
-        }
-#pragma unroll
-        for (int j = 0; j < TN; ++j)
-#pragma unroll
-          for (int i = 0; i < TM; ++i) mfdev::mac(ah[i], al[i], bh[j], bl[j], s_hi[i][j], s_lo[i][j]);
-        if (ri > 0) {
-          if (++cnt == ri) {
-            cnt = 0;
-            if (k0 + kk + 1 < K) {
-#pragma unroll
-              for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) mfdev::renorm(s_hi[i][j], s_lo[i][j]);
-            }
-          }
-        }
+        for (int u = 0; u < kGroup; ++u) step(as + (kk + u) * BM, bs + (kk + u) * PB);
+        if (cad.ends(kGroup) && k0 + kk + kGroup < K) renorm_all();
       }
+    }
+    while (kk < kmax) {  // the steps up to the next chunk's end
+      const int end = kk + cad.run(kmax - kk), from = kk;
+#pragma unroll(TM * TN >= 16 ? 1 : 4)
+      for (; kk < end; ++kk) step(as + kk * BM, bs + kk * PB);
+      if (cad.ends(kk - from) && k0 + kk < K) renorm_all();
     }
     __syncthreads();
   }
@@ -153,116 +194,119 @@ __device__ __forceinline__ void gemm_tile(const double *__restrict__ A, const do
 
 
 // ---------------------------------------------------------------------------
-// One 32 x 32 output tile of the complex product (the Fortran cdd_matmul_mm
-// composition, fsrc/multifloats.fypp:2609-2621): each thread owns a 2 x 2
-// complex tile with four real accumulators per output (rr, ii, ri, ir), each
-// run with the real MAC and renorm cadence, then re = rr - ii, im = ri + ir
-// with the DD operators.
+// One (16 TM) x (16 TN) output tile of the complex product (the Fortran
+// cdd_matmul_mm composition, fsrc/multifloats.fypp:2609-2621): each thread owns
+// TM x TN complex outputs with four real accumulators each (rr, ii, ri, ir),
+// each run with the real MAC and renorm cadence, then re = rr - ii,
+// im = ri + ir with the DD operators.
 // ---------------------------------------------------------------------------
-constexpr int kCTM = 2, kCTN = 2;
-constexpr int kCBM = 16 * kCTM, kCBN = 16 * kCTN, kCBK = kBK;
-
+// Staging of any complex tile (edges 16, 32): real and imaginary part adjacent.
 struct CSmem {
-  double2 A[2][kCBK][kCBM][2];
-  double2 B[2][kCBK][kCBN][2];
+  double2 A[2][512];
+  double2 B[2][2 * depth(32) * b_pitch(16)];
 };
 
-template <bool ALIGNED>
+template <int TM, int TN, bool ALIGNED>
 __device__ __forceinline__ void cgemm_tile(const double *__restrict__ A, const double *__restrict__ B,
                                            double *__restrict__ C, int64_t M, int64_t K, int64_t N,
                                            int64_t ri, int64_t m0, int64_t n0, CSmem &sm) {
   // complex element = 4 doubles = two double2 (re, im)
-  auto &As = sm.A;
-  auto &Bs = sm.B;
+  constexpr int BM = 16 * TM, BN = 16 * TN, BK = depth(2 * (BM > BN ? BM : BN)), PB = b_pitch(BN);
+  static_assert(2 * BK * BM <= 512 && BK * PB <= depth(32) * b_pitch(16), "stage fits CSmem");
   const int t = threadIdx.x;
   const int tx = t % 16, ty = t / 16;
 
-  double s_hi[kCTM][kCTN][4], s_lo[kCTM][kCTN][4];
+  double s_hi[TM][TN][4], s_lo[TM][TN][4];
 #pragma unroll
-  for (int i = 0; i < kCTM; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < kCTN; ++j)
+    for (int j = 0; j < TN; ++j)
 #pragma unroll
       for (int q = 0; q < 4; ++q) s_hi[i][j][q] = s_lo[i][j][q] = 0.0;
 
   auto issue = [&](int stage, int64_t k0) {
-    // A: kCBK x kCBM complex = 256 complex = 512 DD; each thread copies 2 DD.
 #pragma unroll
-    for (int r = 0; r < (kCBK * kCBM * 2) / kThreads; ++r) {
-      int idx = t + r * kThreads;
+    for (int idx = t; idx < 2 * BK * BM; idx += kThreads) {
       int part = idx & 1, e = idx >> 1;
-      int row = e % kCBM, kk = e / kCBM;
+      int row = e % BM, kk = e / BM;
       int64_t gi = m0 + row, gk = k0 + kk;
       bool v = gi < M && gk < K;
-      load_dd<ALIGNED>(&As[stage][kk][row][part], A + 4 * (gk * M + gi) + 2 * part, v, A);
+      load_dd<ALIGNED>(&sm.A[stage][2 * (kk * BM + row) + part], A + 4 * (gk * M + gi) + 2 * part, v, A);
     }
 #pragma unroll
-    for (int r = 0; r < (kCBK * kCBN * 2) / kThreads; ++r) {
-      int idx = t + r * kThreads;
+    for (int idx = t; idx < 2 * BK * BN; idx += kThreads) {
       int part = idx & 1, e = idx >> 1;
-      int kk = e % kCBK, col = e / kCBK;
+      int kk = e % BK, col = e / BK;
       int64_t gj = n0 + col, gk = k0 + kk;
       bool v = gj < N && gk < K;
-      load_dd<ALIGNED>(&Bs[stage][kk][col][part], B + 4 * (gj * K + gk) + 2 * part, v, B);
+      load_dd<ALIGNED>(&sm.B[stage][2 * (kk * PB + col) + part], B + 4 * (gj * K + gk) + 2 * part, v, B);
     }
     cp_async_commit();
   };
+  auto step = [&](const double2 *as, const double2 *bs) {
+    double2 ar[TM], ai[TM], br[TN], bi[TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      ar[i] = as[32 * i];
+      ai[i] = as[32 * i + 1];
+    }
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      br[j] = bs[32 * j];
+      bi[j] = bs[32 * j + 1];
+    }
+#pragma unroll
+    for (int j = 0; j < TN; ++j)
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        mfdev::mac(ar[i].x, ar[i].y, br[j].x, br[j].y, s_hi[i][j][0], s_lo[i][j][0]);
+        mfdev::mac(ai[i].x, ai[i].y, bi[j].x, bi[j].y, s_hi[i][j][1], s_lo[i][j][1]);
+        mfdev::mac(ar[i].x, ar[i].y, bi[j].x, bi[j].y, s_hi[i][j][2], s_lo[i][j][2]);
+        mfdev::mac(ai[i].x, ai[i].y, br[j].x, br[j].y, s_hi[i][j][3], s_lo[i][j][3]);
+      }
+  };
+  auto renorm_all = [&]() {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) mfdev::renorm(s_hi[i][j][q], s_lo[i][j][q]);
+  };
 
-  const int64_t ntiles = (K + kCBK - 1) / kCBK;
-  int64_t cnt = 0;
+  const int64_t ntiles = (K + BK - 1) / BK;
+  Cadence cad(ri);
   if (ntiles > 0) issue(0, 0);
   for (int64_t kt = 0; kt < ntiles; ++kt) {
     const int stage = (int)(kt & 1);
     cp_async_wait_all();
     __syncthreads();
-    if (kt + 1 < ntiles) issue(stage ^ 1, (kt + 1) * kCBK);
-    const int64_t k0 = kt * kCBK;
-    const int kmax = (K - k0) < kCBK ? (int)(K - k0) : kCBK;
+    if (kt + 1 < ntiles) issue(stage ^ 1, (kt + 1) * BK);
+    const int64_t k0 = kt * BK;
+    const int kmax = (K - k0) < BK ? (int)(K - k0) : BK;
+    const double2 *as = sm.A[stage] + 2 * tx, *bs = sm.B[stage] + 2 * ty;
+    int kk = 0;
+    if (cad.grouped) {
+#pragma unroll 1
+      for (; kk + kGroup <= kmax; kk += kGroup) {
 #pragma unroll
-    for (int kk = 0; kk < kCBK; ++kk) {
-      if (kk < kmax) {
-        double2 ar[kCTM], ai[kCTM], br[kCTN], bi[kCTN];
-#pragma unroll
-        for (int i = 0; i < kCTM; ++i) {
-          ar[i] = As[stage][kk][tx + 16 * i][0];
-          ai[i] = As[stage][kk][tx + 16 * i][1];
-        }
-#pragma unroll
-        for (int j = 0; j < kCTN; ++j) {
-          br[j] = Bs[stage][kk][ty + 16 * j][0];
-          bi[j] = Bs[stage][kk][ty + 16 * j][1];
-        }
-#pragma unroll
-        for (int j = 0; j < kCTN; ++j)
-#pragma unroll
-          for (int i = 0; i < kCTM; ++i) {
-            mfdev::mac(ar[i].x, ar[i].y, br[j].x, br[j].y, s_hi[i][j][0], s_lo[i][j][0]);
-            mfdev::mac(ai[i].x, ai[i].y, bi[j].x, bi[j].y, s_hi[i][j][1], s_lo[i][j][1]);
-            mfdev::mac(ar[i].x, ar[i].y, bi[j].x, bi[j].y, s_hi[i][j][2], s_lo[i][j][2]);
-            mfdev::mac(ai[i].x, ai[i].y, br[j].x, br[j].y, s_hi[i][j][3], s_lo[i][j][3]);
-          }
-        if (ri > 0) {
-          if (++cnt == ri) {
-            cnt = 0;
-            if (k0 + kk + 1 < K) {
-#pragma unroll
-              for (int i = 0; i < kCTM; ++i)
-#pragma unroll
-                for (int j = 0; j < kCTN; ++j)
-#pragma unroll
-                  for (int q = 0; q < 4; ++q) mfdev::renorm(s_hi[i][j][q], s_lo[i][j][q]);
-            }
-          }
-        }
+        for (int u = 0; u < kGroup; ++u) step(as + 2 * (kk + u) * BM, bs + 2 * (kk + u) * PB);
+        if (cad.ends(kGroup) && k0 + kk + kGroup < K) renorm_all();
       }
+    }
+    while (kk < kmax) {  // the steps up to the next chunk's end
+      const int end = kk + cad.run(kmax - kk), from = kk;
+#pragma unroll(TM * TN >= 4 ? 1 : 4)
+      for (; kk < end; ++kk) step(as + 2 * kk * BM, bs + 2 * kk * PB);
+      if (cad.ends(kk - from) && k0 + kk < K) renorm_all();
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int j = 0; j < kCTN; ++j) {
+  for (int j = 0; j < TN; ++j) {
     int64_t gj = n0 + ty + 16 * j;
 #pragma unroll
-    for (int i = 0; i < kCTM; ++i) {
+    for (int i = 0; i < TM; ++i) {
       int64_t gi = m0 + tx + 16 * i;
       mfdev::dd p[4];
 #pragma unroll
