@@ -38,6 +38,15 @@ __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e
   e = add(sub(a, ap), sub(b, bp));
   s = ss;
 }
+// two_sum for operands in known order (the exponent of a at least that of b):
+// the error is exact after two more additions instead of five.  Written
+// (a - s) + b, an exact sum gives +0 whatever the signs of its zeros, as
+// two_sum does (fast_two_sum gives -0 for b = -0).
+__device__ __forceinline__ void two_sum_ord(double a, double b, double& s, double& e) {
+  double ss = add(a, b);
+  e = add(sub(a, ss), b);
+  s = ss;
+}
 __device__ __forceinline__ void fast_two_sum(double a, double b, double& s, double& e) {
   double ss = add(a, b);
   double bp = sub(ss, a);
@@ -114,6 +123,47 @@ __device__ __forceinline__ dd dd_div(dd x, dd y) {
   double q2 = div_(rh, y.hi);
   dd r;
   fast_two_sum(q1, q2, r.hi, r.lo);
+  return r;
+}
+
+// ---- the operators' general paths, for operands known to take them -----------
+// dd_add / dd_sub / dd_mul without the short-circuit tests: bit-identical where
+// the leading sum or product is finite and (addition) the two high limbs are
+// not both zero.  dd_add_ord needs |x.hi| >= |y.hi| besides: 17 FP64
+// instructions instead of 20.  The polynomial kernels of exp, log, sin and cos
+// run on these behind one test of their argument; the tests and branches of
+// the operators cost them a fifth of their time (they end a basic block after
+// every operation).
+__device__ __forceinline__ dd dd_add_tail(double a, double b, double c, double d) {
+  dd r;
+  fast_two_sum(a, c, a, c);
+  b = add(b, d);
+  b = add(b, c);
+  fast_two_sum(a, b, r.hi, r.lo);
+  return r;
+}
+__device__ __forceinline__ dd dd_add_gen(dd x, dd y) {
+  double a, b, c, d;
+  two_sum(x.hi, y.hi, a, b);
+  two_sum(x.lo, y.lo, c, d);
+  return dd_add_tail(a, b, c, d);
+}
+__device__ __forceinline__ dd dd_sub_gen(dd x, dd y) { return dd_add_gen(x, neg(y)); }
+__device__ __forceinline__ dd dd_add_ord(dd x, dd y) {
+  double a, b, c, d;
+  two_sum_ord(x.hi, y.hi, a, b);
+  two_sum(x.lo, y.lo, c, d);
+  return dd_add_tail(a, b, c, d);
+}
+__device__ __forceinline__ dd dd_mul_gen(dd x, dd y) {
+  double p00, e00;
+  two_prod(x.hi, y.hi, p00, e00);
+  double p01 = mul(x.hi, y.lo);
+  double p10 = mul(x.lo, y.hi);
+  p01 = add(p01, p10);
+  e00 = add(e00, p01);
+  dd r;
+  fast_two_sum(p00, e00, r.hi, r.lo);
   return r;
 }
 
@@ -213,70 +263,114 @@ __device__ __forceinline__ dd dd_sqrt(dd x) {
   return r;
 }
 
+// Exact power of two 2^e for -1022 <= e <= 1023.
+__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+// x 2^e, correctly rounded like ldexp: a multiplication by an exact power of
+// two when 2^e is a normal double, ldexp otherwise.
+__device__ __forceinline__ double scale2(double x, int e) {
+  return (e >= -1022 && e <= 1023) ? mul(x, pow2(e)) : ldexp(x, e);
+}
+
 // ---- polynomial evaluators (src/float64x2/poly.inc) ------------------------
-// horner: n = coefficient count (poly.inc:9-16).
-__device__ __forceinline__ dd horner(dd y, const double* hi, const double* lo, int n) {
-  dd p = make(hi[n - 1], lo[n - 1]);
-  for (int i = n - 2; i >= 0; --i) p = dd_add(dd_mul(p, y), make(hi[i], lo[i]));
+// Checked: with the operators' short circuits, for any argument.  Decaying:
+// every partial sum exceeds the term added to it in magnitude and nothing
+// overflows (the callers test the argument for that).
+struct Checked {
+  static __device__ __forceinline__ dd mul(dd a, dd b) { return dd_mul(a, b); }
+  static __device__ __forceinline__ dd add(dd a, dd b) { return dd_add(a, b); }      // any order
+  static __device__ __forceinline__ dd add_ord(dd a, dd b) { return dd_add(a, b); }  // |a| >= |b|
+};
+struct Decaying {
+  static __device__ __forceinline__ dd mul(dd a, dd b) { return dd_mul_gen(a, b); }
+  static __device__ __forceinline__ dd add(dd a, dd b) { return dd_add_gen(a, b); }
+  static __device__ __forceinline__ dd add_ord(dd a, dd b) { return dd_add_ord(a, b); }
+};
+#define MF_C(i) make(hi[i], lo[i])
+// horner: n = coefficient count (poly.inc:9-16): p * y + c, the sum written c + p * y.
+template <class Op, int N>
+__device__ __forceinline__ dd horner(dd y, const double* hi, const double* lo) {
+  dd p = MF_C(N - 1);
+#pragma unroll
+  for (int i = N - 2; i >= 0; --i) p = Op::add_ord(MF_C(i), Op::mul(p, y));
   return p;
 }
 // neval (Estrin), degree 10 and 12 cases (poly.inc:33-102).  C++ `a + b * c`
 // is a + (b*c); chains of `+` associate left.
+template <class Op>
 __device__ __forceinline__ dd neval10(dd x, const double* hi, const double* lo) {
-#define MF_C(i) make(hi[i], lo[i])
-  dd x2 = dd_mul(x, x);
-  dd x4 = dd_mul(x2, x2);
-  dd x8 = dd_mul(x4, x4);
-  dd p01 = dd_add(MF_C(0), dd_mul(MF_C(1), x));
-  dd p23 = dd_add(MF_C(2), dd_mul(MF_C(3), x));
-  dd p45 = dd_add(MF_C(4), dd_mul(MF_C(5), x));
-  dd p67 = dd_add(MF_C(6), dd_mul(MF_C(7), x));
-  dd p89 = dd_add(MF_C(8), dd_mul(MF_C(9), x));
-  dd p03 = dd_add(p01, dd_mul(p23, x2));
-  dd p47 = dd_add(p45, dd_mul(p67, x2));
-  dd p810 = dd_add(p89, dd_mul(MF_C(10), x2));
-  return dd_add(dd_add(p03, dd_mul(p47, x4)), dd_mul(p810, x8));
+  dd x2 = Op::mul(x, x);
+  dd x4 = Op::mul(x2, x2);
+  dd x8 = Op::mul(x4, x4);
+  dd p01 = Op::add_ord(MF_C(0), Op::mul(MF_C(1), x));
+  dd p23 = Op::add_ord(MF_C(2), Op::mul(MF_C(3), x));
+  dd p45 = Op::add_ord(MF_C(4), Op::mul(MF_C(5), x));
+  dd p67 = Op::add_ord(MF_C(6), Op::mul(MF_C(7), x));
+  dd p89 = Op::add_ord(MF_C(8), Op::mul(MF_C(9), x));
+  dd p03 = Op::add_ord(p01, Op::mul(p23, x2));
+  dd p47 = Op::add_ord(p45, Op::mul(p67, x2));
+  dd p810 = Op::add_ord(p89, Op::mul(MF_C(10), x2));
+  return Op::add_ord(Op::add_ord(p03, Op::mul(p47, x4)), Op::mul(p810, x8));
 }
-__device__ __forceinline__ dd neval12(dd x, const double* hi, const double* lo) {
-  dd x2 = dd_mul(x, x);
-  dd x4 = dd_mul(x2, x2);
-  dd x8 = dd_mul(x4, x4);
-  dd p01 = dd_add(MF_C(0), dd_mul(MF_C(1), x));
-  dd p23 = dd_add(MF_C(2), dd_mul(MF_C(3), x));
-  dd p45 = dd_add(MF_C(4), dd_mul(MF_C(5), x));
-  dd p67 = dd_add(MF_C(6), dd_mul(MF_C(7), x));
-  dd p89 = dd_add(MF_C(8), dd_mul(MF_C(9), x));
-  dd p1011 = dd_add(MF_C(10), dd_mul(MF_C(11), x));
-  dd p03 = dd_add(p01, dd_mul(p23, x2));
-  dd p47 = dd_add(p45, dd_mul(p67, x2));
-  dd p811 = dd_add(p89, dd_mul(p1011, x2));
-  return dd_add(dd_add(p03, dd_mul(p47, x4)), dd_mul(dd_add(p811, dd_mul(MF_C(12), x4)), x8));
+// Degree 12 given the powers y2 = y*y, y4 = y2*y2, y8 = y4*y4 of its argument
+// y, so the sin and cos polynomials of the same argument can share them.
+template <class Op>
+__device__ __forceinline__ dd neval12_pow(dd y, dd y2, dd y4, dd y8, const double* hi,
+                                          const double* lo) {
+  dd p01 = Op::add_ord(MF_C(0), Op::mul(MF_C(1), y));
+  dd p23 = Op::add_ord(MF_C(2), Op::mul(MF_C(3), y));
+  dd p45 = Op::add_ord(MF_C(4), Op::mul(MF_C(5), y));
+  dd p67 = Op::add_ord(MF_C(6), Op::mul(MF_C(7), y));
+  dd p89 = Op::add_ord(MF_C(8), Op::mul(MF_C(9), y));
+  dd p1011 = Op::add_ord(MF_C(10), Op::mul(MF_C(11), y));
+  dd p03 = Op::add_ord(p01, Op::mul(p23, y2));
+  dd p47 = Op::add_ord(p45, Op::mul(p67, y2));
+  dd p811 = Op::add_ord(p89, Op::mul(p1011, y2));
+  return Op::add_ord(Op::add_ord(p03, Op::mul(p47, y4)),
+                     Op::mul(Op::add_ord(p811, Op::mul(MF_C(12), y4)), y8));
+}
 #undef MF_C
-}
 
 // ---- exp (src/float64x2/exp_log.inc:26-72, :237-277) -----------------------
-__device__ __forceinline__ dd exp2_from_reduced(double n_d, double rh, double rl) {
+// 2^n_d (T 2^s) with k = rint(256 rh) clamped to +-128, s = (rh, rl) - k/256 and
+// the table value T = 2^(k/256).
+template <class Op>
+__device__ __forceinline__ dd exp2_poly(dd s) {
+  dd q = make(mf_exp2_coefs_hi[9], mf_exp2_coefs_lo[9]);
+#pragma unroll
+  for (int j = 8; j >= 1; --j) {
+    q = Op::mul(q, s);
+    q = Op::add_ord(make(mf_exp2_coefs_hi[j], mf_exp2_coefs_lo[j]), q);
+  }
+  return Op::add_ord(make(1.0, 0.0), Op::mul(s, q));
+}
+// Any reduced argument (out of range where the low limb was not one).
+static __device__ __noinline__ dd exp2_from_reduced_any(double n_d, double rh, double rl) {
   if (n_d > 1100.0) return make(CUDART_INF, 0.0);
   if (n_d < -1100.0) return make(0.0, 0.0);
   double k_d = rint(mul(rh, 256.0));
   int k = (int)k_d;
   if (k > 128) k = 128;
   if (k < -128) k = -128;
-  double sh = sub(rh, div_((double)k, 256.0));
+  double sh = sub(rh, mul((double)k, 0.00390625));
   double sl = rl;
   fast_two_sum(sh, sl, sh, sl);
-  dd s = make(sh, sl);
-  dd q = make(mf_exp2_coefs_hi[9], mf_exp2_coefs_lo[9]);
-#pragma unroll
-  for (int j = 8; j >= 1; --j) {
-    q = dd_mul(q, s);
-    q = dd_add(q, make(mf_exp2_coefs_hi[j], mf_exp2_coefs_lo[j]));
-  }
-  dd pow2s = dd_add(make(1.0, 0.0), dd_mul(s, q));
+  dd pow2s = exp2_poly<Checked>(make(sh, sl));
   dd T = make(gload(&mf_exp2_table_hi[k + 128]), gload(&mf_exp2_table_lo[k + 128]));
   dd m = dd_mul(T, pow2s);
   int n = (int)n_d;
   return make(ldexp(m.hi, n), ldexp(m.lo, n));
+}
+// |s| <= 1/128 keeps the polynomial decaying: |q s| <= |c_j| / 128.
+__device__ __forceinline__ dd exp2_from_reduced(double n_d, double rh, double rl) {
+  const double k_d = rint(mul(rh, 256.0));
+  double sh = sub(rh, mul(k_d, 0.00390625));
+  double sl = rl;
+  fast_two_sum(sh, sl, sh, sl);
+  if (!(fabs(rh) <= 0.5 && fabs(sh) <= 0.0078125 && fabs(n_d) <= 1100.0)) return exp2_from_reduced_any(n_d, rh, rl);
+  const int k = (int)k_d, n = (int)n_d;
+  const dd T = make(gload(&mf_exp2_table_hi[k + 128]), gload(&mf_exp2_table_lo[k + 128]));
+  const dd m = dd_mul_gen(T, exp2_poly<Decaying>(make(sh, sl)));
+  return make(scale2(m.hi, n), scale2(m.lo, n));
 }
 
 __device__ __forceinline__ dd dd_exp(dd x) {
@@ -307,6 +401,23 @@ __device__ __forceinline__ dd dd_exp(dd x) {
 }
 
 // ---- log (exp_log.inc:280-341) ---------------------------------------------
+// The polynomials in t2 = t^2, decaying for |t2| <= 1/64 (t2 is below 1/900 for
+// a normalised argument).
+struct Log2Wide {
+  template <class Op>
+  static __device__ __forceinline__ dd eval(dd t2) { return neval10<Op>(t2, mf_log2_wide_hi, mf_log2_wide_lo); }
+};
+struct Log2Narrow {
+  template <class Op>
+  static __device__ __forceinline__ dd eval(dd t2) { return horner<Op, 7>(t2, mf_log2_narrow_hi, mf_log2_narrow_lo); }
+};
+template <class P>
+static __device__ __noinline__ dd log2_poly_any(dd t2) { return P::template eval<Checked>(t2); }
+template <class P>
+__device__ __forceinline__ dd log2_poly(dd t2) {
+  if (!(fabs(t2.hi) <= 0.015625)) return log2_poly_any<P>(t2);
+  return P::template eval<Decaying>(t2);
+}
 __device__ __forceinline__ dd log2_kernel(dd x) {
   double hi = x.hi;
   if (hi > 15.0 / 16.0 && hi < 17.0 / 16.0) {
@@ -314,7 +425,7 @@ __device__ __forceinline__ dd log2_kernel(dd x) {
     dd den = dd_add(x, make(1.0, 0.0));
     dd t = dd_div(num, den);
     dd t2 = dd_mul(t, t);
-    dd p = neval10(t2, mf_log2_wide_hi, mf_log2_wide_lo);
+    dd p = log2_poly<Log2Wide>(t2);
     return dd_mul(t, p);
   }
   int e = ilogb(hi);
@@ -328,7 +439,7 @@ __device__ __forceinline__ dd log2_kernel(dd x) {
   dd den = dd_add(m, c);
   dd t = dd_div(num, den);
   dd t2 = dd_mul(t, t);
-  dd p = horner(t2, mf_log2_narrow_hi, mf_log2_narrow_lo, 7);
+  dd p = log2_poly<Log2Narrow>(t2);
   return dd_add(dd_add(make((double)e, 0.0), v), dd_mul(t, p));
 }
 __device__ __forceinline__ dd dd_log2(dd x) {
@@ -365,67 +476,75 @@ __device__ __forceinline__ dd reduce_pi_half(dd x, int& n_mod4) {
   dd_sub_step(rh, rl, ph, pl);
   ph = mul(n_float, mf_pi_half_cw[2]);
   dd_sub_step(rh, rl, ph, 0.0);
-  long long nn = (long long)fabs(n_float) & 3LL;
-  if (n_float < 0.0) nn = (4 - nn) & 3;
-  n_mod4 = (int)nn;
+  // |n| mod 4, negated for negative n: two's complement
+  if (fabs(n_float) < 0x1p31) {
+    n_mod4 = (int)n_float & 3;
+  } else {
+    n_mod4 = (int)((long long)n_float & 3LL);
+  }
   return make(rh, rl);
 }
-__device__ __forceinline__ dd sin_kernel(dd x) {
-  dd x2 = dd_mul(x, x);
-  return dd_mul(neval12(x2, mf_sin_taylor_hi, mf_sin_taylor_lo), x);
-}
-__device__ __forceinline__ dd cos_kernel(dd x) {
-  dd x2 = dd_mul(x, x);
-  return neval12(x2, mf_cos_taylor_hi, mf_cos_taylor_lo);
-}
-// Estrin degree-12 evaluation (poly.inc:91-102) given the powers y2 = y*y,
-// y4 = y2*y2, y8 = y4*y4 of its argument y, so the sin and cos polynomials of
-// the same argument can share them.
-__device__ __forceinline__ dd neval12_pow(dd y, dd y2, dd y4, dd y8, const double* hi,
-                                          const double* lo) {
-#define MF_C(i) make(hi[i], lo[i])
-  dd p01 = dd_add(MF_C(0), dd_mul(MF_C(1), y));
-  dd p23 = dd_add(MF_C(2), dd_mul(MF_C(3), y));
-  dd p45 = dd_add(MF_C(4), dd_mul(MF_C(5), y));
-  dd p67 = dd_add(MF_C(6), dd_mul(MF_C(7), y));
-  dd p89 = dd_add(MF_C(8), dd_mul(MF_C(9), y));
-  dd p1011 = dd_add(MF_C(10), dd_mul(MF_C(11), y));
-  dd p03 = dd_add(p01, dd_mul(p23, y2));
-  dd p47 = dd_add(p45, dd_mul(p67, y2));
-  dd p811 = dd_add(p89, dd_mul(p1011, y2));
-  return dd_add(dd_add(p03, dd_mul(p47, y4)), dd_mul(dd_add(p811, dd_mul(MF_C(12), y4)), y8));
-#undef MF_C
+// The sin and cos Taylor kernels of the same argument, powers of x*x shared.
+template <class Op>
+__device__ __forceinline__ void sincos_kernels(dd x, dd &sk, dd &ck) {
+  dd y = Op::mul(x, x);
+  dd y2 = Op::mul(y, y);
+  dd y4 = Op::mul(y2, y2);
+  dd y8 = Op::mul(y4, y4);
+  sk = Op::mul(neval12_pow<Op>(y, y2, y4, y8, mf_sin_taylor_hi, mf_sin_taylor_lo), x);
+  ck = neval12_pow<Op>(y, y2, y4, y8, mf_cos_taylor_hi, mf_cos_taylor_lo);
 }
 
-// sin_eval / cos_eval of trig.inc:165-187 without warp divergence.  The
-// reference evaluates sin_kernel(r) or cos_kernel(r) when |r| <= pi/8, and
-// both kernels at r -/+ pi/4 otherwise.  Here every thread evaluates both
-// kernels at its own argument (r, or r -/+ pi/4) with the powers of x*x
-// shared, then selects; each value is produced by exactly the reference's
-// sequence of operations, so results are bit-identical.
-__device__ __forceinline__ dd sincos_eval_one(dd r, bool want_sin) {
+// sincos_eval of trig.inc:165-236 without warp divergence.  The reference
+// evaluates sin_kernel(r) or cos_kernel(r) when |r| <= pi/8, and both kernels
+// at r -/+ pi/4 otherwise.  Here every thread evaluates both kernels at its own
+// argument (r, or r -/+ pi/4) and selects; each value is produced by exactly
+// the reference's sequence of operations, so results are bit-identical.
+// both: sin in s and cos in c; else the wanted one in s.
+template <class Op>
+__device__ __forceinline__ void sincos_finish(dd arg, bool small, bool pos, bool both, bool want_sin, dd &s, dd &c) {
+  dd sk, ck;
+  sincos_kernels<Op>(arg, sk, ck);
+  const dd is2 = make(mf_inv_sqrt2_hi[0], mf_inv_sqrt2_lo[0]);
+  if (both) {
+    s = sk;
+    c = ck;
+    if (!small) {
+      s = Op::mul(Op::add(sk, pos ? ck : neg(ck)), is2);  // pos: sk + ck, neg: sk - ck
+      c = Op::mul(Op::add(ck, pos ? neg(sk) : sk), is2);  // pos: ck - sk, neg: ck + sk
+    }
+    return;
+  }
+  const dd u = want_sin ? sk : ck;
+  s = u;
+  if (!small) {
+    const dd v = want_sin ? ck : neg(sk);
+    s = Op::mul(Op::add(u, pos ? v : neg(v)), is2);
+  }
+}
+static __device__ __noinline__ void sincos_finish_any(dd arg, bool small, bool pos, bool both, bool want_sin, dd &s,
+                                                      dd &c) {
+  sincos_finish<Checked>(arg, small, pos, both, want_sin, s, c);
+}
+__device__ __forceinline__ void sincos_eval(dd r, bool both, bool want_sin, dd &s, dd &c) {
   const double pi8 = 0.392699081698724;
   const bool small = fabs(r.hi) <= pi8;
   const bool pos = r.hi > 0.0;
-  dd pi4 = make(mf_pi_quarter_hi[0], mf_pi_quarter_lo[0]);
-  dd arg = small ? r : (pos ? dd_sub(r, pi4) : dd_add(r, pi4));
-  dd x2 = dd_mul(arg, arg);
-  dd y2 = dd_mul(x2, x2);
-  dd y4 = dd_mul(y2, y2);
-  dd y8 = dd_mul(y4, y4);
-  dd sk = dd_mul(neval12_pow(x2, y2, y4, y8, mf_sin_taylor_hi, mf_sin_taylor_lo), arg);
-  dd ck = neval12_pow(x2, y2, y4, y8, mf_cos_taylor_hi, mf_cos_taylor_lo);
-  if (small) return want_sin ? sk : ck;
-  dd is2 = make(mf_inv_sqrt2_hi[0], mf_inv_sqrt2_lo[0]);
-  dd u, v;
-  if (want_sin) {
-    u = sk;
-    v = ck;  // pos: (sk + ck), neg: (sk - ck)
-  } else {
-    u = ck;
-    v = neg(sk);  // pos: (ck - sk), neg: (ck + sk)
+  const dd pi4 = make(mf_pi_quarter_hi[0], mf_pi_quarter_lo[0]);
+  dd arg = r;
+  if (!small) arg = dd_add(r, pos ? neg(pi4) : pi4);
+  // |arg| <= 1/2 keeps both Taylor series decaying; only a reduction that lost
+  // its quadrant (|x| near 2^55) or an unnormalised operand is outside
+  if (!(fabs(arg.hi) <= 0.5)) {
+    sincos_finish_any(arg, small, pos, both, want_sin, s, c);
+    return;
   }
-  return pos ? dd_mul(dd_add(u, v), is2) : dd_mul(dd_sub(u, v), is2);
+  sincos_finish<Decaying>(arg, small, pos, both, want_sin, s, c);
+}
+__device__ __forceinline__ dd sincos_eval_one(dd r, bool want_sin) {
+  dd s, c;
+  sincos_eval(r, false, want_sin, s, c);
+  return s;
 }
 __device__ __forceinline__ bool trig_arg_too_large(double a) { return !(fabs(a) < 0x1p55); }
 
@@ -448,29 +567,6 @@ __device__ __forceinline__ dd dd_cos(dd x) {
 }
 
 // ---- fused sin / cos (trig.inc:189-236): one reduction, both evaluations ----
-// sincos_eval: the same two Taylor kernels and pi/4 shift as sin_eval and
-// cos_eval, so each output equals the separate call bit for bit.
-__device__ __forceinline__ void sincos_eval_both(dd r, dd &s, dd &c) {
-  const double pi8 = 0.392699081698724;
-  const bool small = fabs(r.hi) <= pi8;
-  const bool pos = r.hi > 0.0;
-  dd pi4 = make(mf_pi_quarter_hi[0], mf_pi_quarter_lo[0]);
-  dd arg = small ? r : (pos ? dd_sub(r, pi4) : dd_add(r, pi4));
-  dd x2 = dd_mul(arg, arg);
-  dd y2 = dd_mul(x2, x2);
-  dd y4 = dd_mul(y2, y2);
-  dd y8 = dd_mul(y4, y4);
-  dd sk = dd_mul(neval12_pow(x2, y2, y4, y8, mf_sin_taylor_hi, mf_sin_taylor_lo), arg);
-  dd ck = neval12_pow(x2, y2, y4, y8, mf_cos_taylor_hi, mf_cos_taylor_lo);
-  if (small) {
-    s = sk;
-    c = ck;
-    return;
-  }
-  dd is2 = make(mf_inv_sqrt2_hi[0], mf_inv_sqrt2_lo[0]);
-  s = pos ? dd_mul(dd_add(sk, ck), is2) : dd_mul(dd_sub(sk, ck), is2);
-  c = pos ? dd_mul(dd_sub(ck, sk), is2) : dd_mul(dd_add(ck, sk), is2);
-}
 // sincos(x, s, c) (trig.inc:216-236)
 __device__ __forceinline__ void dd_sincos(dd x, dd &s, dd &c) {
   if (!isfinite(x.hi) || trig_arg_too_large(x.hi)) {
@@ -485,7 +581,7 @@ __device__ __forceinline__ void dd_sincos(dd x, dd &s, dd &c) {
   int q;
   dd r = reduce_pi_half(x, q);
   dd ss, cc;
-  sincos_eval_both(r, ss, cc);
+  sincos_eval(r, true, false, ss, cc);
   switch (q) {
     case 0: s = ss; c = cc; break;
     case 1: s = cc; c = neg(ss); break;

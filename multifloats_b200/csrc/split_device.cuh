@@ -146,13 +146,8 @@ __device__ __forceinline__ int floor_log2(double v) {
 __device__ __forceinline__ int binade_above(double v) { return floor_log2(v) + 1; }
 __device__ __forceinline__ int binade_below(double v) { return floor_log2(v); }
 
-// Exact power of two 2^e for -1022 <= e <= 1023.
-__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
-// x 2^e, correctly rounded like ldexp: a multiplication by an exact power of
-// two when 2^e is a normal double, ldexp otherwise.
-__device__ __forceinline__ double scale2(double x, int e) {
-  return (e >= -1022 && e <= 1023) ? x * pow2(e) : ldexp(x, e);
-}
+using mfdev::pow2;
+using mfdev::scale2;
 
 // The entry rounded to the fixed-point grid of its row / column
 // (grid_round.cuh: X = rint(H) + rint((H - rint(H)) + L), H = hi 2^(W - sigma),
