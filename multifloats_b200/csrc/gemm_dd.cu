@@ -172,20 +172,39 @@ __global__ void __launch_bounds__(kThreads, 4)
 // p = 0..k-1, so there is one dependency chain per output and only a few
 // thousand of them; a CTA owns 32 outputs and splits each MAC
 // (matmul.inc:6-19) in two:
-//   * three producer warps stream the matrix through a 4-stage cp.async ring
-//     (32 outputs x 32 k per stage) and compute the accumulator-independent
-//     part of every MAC, p = ah*bh and q = fma(ah,bh,-p) + fma(ah,bl,al*bh),
-//     into a double-buffered shared array;
+//   * eight producer warps stream the matrix through an S-stage cp.async ring
+//     (a stage is 32 outputs x 32 k, four columns of it per warp) and compute
+//     the accumulator-independent part of every MAC, p = ah*bh and
+//     q = fma(ah,bh,-p) + fma(ah,bl,al*bh), into a double-buffered array;
 //   * one warp runs the accumulator chain (two_sum of s_hi with p, then
 //     s_lo += q + (aerr + berr)) and the renorm cadence, lane = output.
 // The operations and their order per output are the reference's, so results
-// are bit-identical; the producers and the chain hand over through
-// __syncthreads once per stage.
+// are bit-identical; the warps hand over through one named barrier per stage.
+//
+// Bound: the chain, 15 dependent additions of 8 cycles per eight steps and 62
+// FP64 instructions; as compiled it takes 32 cycles a step, where HBM at one
+// CTA per SM would take 19.  So the chain warp has a scheduler to itself (the
+// producers use the other three; the roles rotate with the wave of CTAs, so
+// that the chains of the CTAs of one SM land on different schedulers) and, in
+// the default cadence, no test between its steps.  S = 8 stages (one CTA per
+// SM) when the outputs are one wave, 4 (two CTAs) otherwise.
+// 4099 x 3001: 143 -> 62 us (y = A x), 143 -> 60 (y = x A); 16384 x 8192: 908 ->
+// 445, 862 -> 402 (HBM alone 328).
 // ---------------------------------------------------------------------------
-constexpr int kGvN = 32, kGvK = 32, kGvStages = 4, kGvPitch = 33, kGvProd = 3;
-constexpr int kGvThreads = 32 * (1 + kGvProd);
-constexpr size_t kGvRingBytes = sizeof(double2) * kGvStages * kGvN * kGvPitch;
-constexpr size_t kGvSmem = kGvRingBytes + sizeof(double2) * 2 * kGvK * kGvPitch;
+constexpr int kGvN = 32, kGvK = 32;
+constexpr int kGvWarps = 12, kGvThreads = 32 * kGvWarps;  // chain, eight producers, three without work
+constexpr int kGvProd = 8, kGvActive = 32 * (1 + kGvProd);
+// Row of the term array: the producers of y = x B write it transposed.
+__host__ __device__ constexpr int gv_pitch(bool vm) { return vm ? 33 : 32; }
+// Where the vector's entries of a stage come from: with S = 8 the first
+// producer copies them into the ring for all (one stage of the prefetch is then
+// spent on the hand-over); with S = 4 that stage is worth more than the ring, and
+// every producer loads its own a stage ahead (4800 x 3000: 108 -> 84 us; with
+// S = 8, 4099 x 3001: 75 instead of 62).
+__host__ __device__ constexpr bool gv_x_ring(int stages) { return stages > 4; }
+constexpr size_t gv_smem(bool vm, int stages) {
+  return sizeof(double2) * ((size_t)stages * (kGvN * kGvK + (gv_x_ring(stages) ? kGvK : 0)) + 2 * (size_t)kGvK * gv_pitch(vm));
+}
 
 template <int N>
 __device__ __forceinline__ void cp_async_wait_n() {
@@ -210,198 +229,169 @@ __device__ __forceinline__ double2 mac_terms(double ah, double al, double bh, do
   return make_double2(p, mfdev::add(e, cross));
 }
 
-// Runs the chain over stage st's terms (lane = output), renorm cadence as in
-// the reference: after each full chunk of ri steps when more remain.  The
-// MACs between two renorm points run as one branch-free loop, so the
-// compiler can start a MAC's t = s_hi + p while the previous MAC's error
-// terms are still in flight (same operations, same order).
-__device__ __forceinline__ void chain_stage(const double2 *__restrict__ pq, int cmax, int64_t p0, int64_t K,
-                                            int64_t ri, int lane, double &sh, double &sl, int64_t &cnt) {
+// Runs the chain over cmax terms of a stage that starts at step p0 (v: this
+// lane's column of the term array), renorm cadence as in the reference: after
+// each full chunk of ri steps when more remain.
+template <int PITCH>
+__device__ __forceinline__ void chain_stage(const double2 *__restrict__ v, int cmax, int64_t p0, int64_t K,
+                                            gtile::Cadence &cad, double &sh, double &sl) {
+  constexpr int G = gtile::kGroup;
+  auto group = [&](int c) {
+    double2 u[G];
+#pragma unroll
+    for (int r = 0; r < G; ++r) u[r] = v[(c + r) * PITCH];
+#pragma unroll
+    for (int r = 0; r < G; ++r) mac_chain(u[r].x, u[r].y, sh, sl);
+    if (cad.ends(G) && p0 + c + G < K) mfdev::renorm(sh, sl);
+  };
   int c = 0;
-  while (c < cmax) {
-    const int run = ri > 0 ? (int)min((int64_t)(cmax - c), ri - cnt) : cmax - c;
-    const double2 *v = pq + (size_t)c * kGvPitch + lane;
-#pragma unroll 8
-    for (int r = 0; r < run; ++r) mac_chain(v[r * kGvPitch].x, v[r * kGvPitch].y, sh, sl);
-    c += run;
-    if (ri > 0) {
-      cnt += run;
-      if (cnt == ri) {
-        cnt = 0;
-        if (p0 + c < K) mfdev::renorm(sh, sl);
+  if (cad.grouped) {
+    if (cad.ri == G && p0 + kGvK < K) {  // a renormalisation after every group: no tests
+#pragma unroll
+      for (int g = 0; g < kGvK / G; ++g) {
+        double2 u[G];
+#pragma unroll
+        for (int r = 0; r < G; ++r) u[r] = v[(g * G + r) * PITCH];
+#pragma unroll
+        for (int r = 0; r < G; ++r) mac_chain(u[r].x, u[r].y, sh, sl);
+        mfdev::renorm(sh, sl);
       }
+      return;
     }
+#pragma unroll 1
+    for (; c + G <= cmax; c += G) group(c);
+  }
+  while (c < cmax) {  // the steps up to the next chunk's end
+    const int run = cad.run(cmax - c);
+    const double2 *w = v + c * PITCH;
+#pragma unroll 4
+    for (int r = 0; r < run; ++r) mac_chain(w[r * PITCH].x, w[r * PITCH].y, sh, sl);
+    c += run;
+    if (cad.ends(run) && p0 + c < K) mfdev::renorm(sh, sl);
   }
 }
 
-// y(m) = A(m,k) x(k) (gaxpy_mv_panel, matmul.inc:47-88; A is the MAC's first
-// operand).  Producer warp w copies and evaluates the stage columns c with
-// c % 3 == w - 1, lane l = row i0 + l (each copy instruction moves one
-// 512-byte segment of column-major A; a thread reads only what it copied).
-template <bool ALIGNED>
+// VM false: y(M) = A(M,K) x(K) (gaxpy_mv_panel, matmul.inc:47-88; A is the
+// MAC's first operand); a stage is 32 columns of A, 32 rows (512 contiguous
+// bytes) each.  VM true: y(M) = x(K) A(K,M) (vm_impl, matmul.inc:213-239; x is
+// the MAC's first operand); a stage is 32 columns (outputs), 32 k each.
+template <bool VM, int S, bool ALIGNED>
 __global__ void __launch_bounds__(kGvThreads) gemv_dd_kernel(const double *__restrict__ A,
                                                              const double *__restrict__ x,
                                                              double *__restrict__ y, int64_t M,
-                                                             int64_t K, int64_t ri) {
+                                                             int64_t K, int64_t ri, int sms) {
+  constexpr int PITCH = gv_pitch(VM);
   extern __shared__ double2 smem_gv[];
-  double2 *ring = smem_gv;                                   // [stage][k][row pitch]
-  double2 *pq = smem_gv + (size_t)kGvStages * kGvK * kGvPitch;  // [2][k][row pitch]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t i = (int64_t)blockIdx.x * kGvN + lane;
-  const bool row_ok = i < M;
+  double2 *ring = smem_gv;                                 // [stage][column][32]
+  double2 *pq = ring + (size_t)S * kGvN * kGvK;            // [2][k][output]
+  double2 *xs = pq + 2 * (size_t)kGvK * PITCH;             // [stage][k] of the vector
+  const int lane = threadIdx.x & 31;
+  // role 0: chain; 4 and 8, which share its scheduler, and 11: none; else a producer
+  const int rot = (int)(blockIdx.x / (unsigned)sms) & 3;
+  const int role = ((int)(threadIdx.x >> 5) + kGvWarps - rot) % kGvWarps;
+  if (role == 4 || role == 8 || role == 11) return;
+  auto sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kGvActive) : "memory"); };
+  const int64_t i0 = (int64_t)blockIdx.x * kGvN;
   const int64_t nst = (K + kGvK - 1) / kGvK;
-  const int w = warp - 1;  // producer index
+
+  if (role == 0) {  // ---- accumulator chain
+    double sh = 0.0, sl = 0.0;
+    gtile::Cadence cad(ri);
+    if (gv_x_ring(S)) sync();
+    sync();  // the terms of stage 0 are ready
+    for (int64_t st = 0; st < nst; ++st) {
+      const int64_t p0 = st * kGvK;
+      const int cmax = (K - p0) < kGvK ? (int)(K - p0) : kGvK;
+      chain_stage<PITCH>(pq + (size_t)(st & 1) * kGvK * PITCH + lane, cmax, p0, K, cad, sh, sl);
+      sync();
+    }
+    const int64_t i = i0 + lane;
+    if (i < M) {
+      mfdev::renorm(sh, sl);
+      y[2 * i] = sh;
+      y[2 * i + 1] = sl;
+    }
+    return;
+  }
+  // ---- producer w: copies and terms of the columns w, w + 8, w + 16, w + 24
+  constexpr int COLS = kGvN / kGvProd;
+  constexpr bool XR = gv_x_ring(S);
+  constexpr int PENDING = XR ? S - 3 : S - 2;  // copies that may be in flight when a stage's terms are due
+  const int w = role < 4 ? role - 1 : role < 8 ? role - 2 : role - 3;
   auto issue = [&](int64_t st) {
     if (st < nst) {
-      double2 *dst = ring + (size_t)(st % kGvStages) * kGvK * kGvPitch;
+      double2 *dst = ring + ((size_t)(st % S) * kGvN + w) * 32 + lane;
       const int64_t p0 = st * kGvK;
-      const double *src = A + 2 * ((p0 + w) * M + i);
+      const double *src = VM ? A + 2 * ((i0 + w) * K + p0 + lane) : A + 2 * ((p0 + w) * M + i0 + lane);
+      const int64_t step = 2 * kGvProd * (VM ? K : M);
+      const bool ok = VM ? p0 + lane < K : i0 + lane < M;
+      const int64_t left = (VM ? M - i0 : K - p0) - w;  // columns from this warp's first one on
 #pragma unroll
-      for (int c = w; c < kGvK; c += kGvProd, src += 2 * kGvProd * M)
-        load_dd<ALIGNED>(&dst[c * kGvPitch + lane], src, row_ok && p0 + c < K, A);
+      for (int u = 0; u < COLS; ++u)
+        load_dd<ALIGNED>(dst + u * kGvProd * 32, src + u * step, ok && u * kGvProd < left, A);
+      if (XR && w == 0)
+        load_dd<ALIGNED>(xs + (size_t)(st % S) * kGvK + lane, x + 2 * (p0 + lane), p0 + lane < K, x);
     }
     cp_async_commit();
   };
-  auto load_x = [&](int64_t st) {  // lane l: x[st * 32 + l] (zero past k), one stage ahead of use
-    double2 v = make_double2(0.0, 0.0);
-    const int64_t p = st * kGvK + lane;
-    if (st < nst && p < K) {
-      const double *xp = x + 2 * p;
-      v = ALIGNED ? *reinterpret_cast<const double2 *>(xp) : make_double2(xp[0], xp[1]);
-    }
-    return v;
-  };
-  auto produce = [&](int64_t st, double2 xv) {  // terms of stage st into pq[st % 2]
-    if (st >= nst) return;
-    const int64_t p0 = st * kGvK;
-    const int cmax = (K - p0) < kGvK ? (int)(K - p0) : kGvK;
-    const double2 *src = ring + (size_t)(st % kGvStages) * kGvK * kGvPitch;
-    double2 *out = pq + (size_t)(st & 1) * kGvK * kGvPitch;
+  // the vector's entries: this lane's k, or (uniform over the warp) those of
+  // the warp's columns
+  constexpr int NX = VM ? 1 : COLS;
+  auto load_x = [&](int64_t st, double2 (&v)[NX]) {
 #pragma unroll
-    for (int c0 = 0; c0 < kGvK; c0 += kGvProd) {
-      const int c = c0 + w;
-      const double xh = __shfl_sync(0xffffffffu, xv.x, c & 31), xl = __shfl_sync(0xffffffffu, xv.y, c & 31);
-      if (c < cmax) {
-        const double2 av = src[c * kGvPitch + lane];
-        out[c * kGvPitch + lane] = mac_terms(av.x, av.y, xh, xl);
+    for (int u = 0; u < NX; ++u) {
+      const int64_t p = st * kGvK + (VM ? lane : w + u * kGvProd);
+      v[u] = make_double2(0.0, 0.0);
+      if (p < K) {
+        const double *xp = x + 2 * p;
+        v[u] = ALIGNED ? *reinterpret_cast<const double2 *>(xp) : make_double2(xp[0], xp[1]);
       }
     }
   };
-  double2 xnext = make_double2(0.0, 0.0);
-  if (warp > 0) {
-    for (int s0 = 0; s0 < kGvStages - 1; ++s0) issue(s0);
-    const double2 x0 = load_x(0);
-    xnext = load_x(1);
-    cp_async_wait_n<kGvStages - 2>();  // stage 0 landed
-    produce(0, x0);
-  }
-  __syncthreads();
-  double sh = 0.0, sl = 0.0;
-  int64_t cnt = 0;
-  for (int64_t st = 0; st < nst; ++st) {
-    if (warp == 0) {
-      const int64_t p0 = st * kGvK;
-      const int cmax = (K - p0) < kGvK ? (int)(K - p0) : kGvK;
-      chain_stage(pq + (size_t)(st & 1) * kGvK * kGvPitch, cmax, p0, K, ri, lane, sh, sl, cnt);
-    } else {
-      issue(st + kGvStages - 1);        // into the slot of stage st - 1, consumed already
-      const double2 xcur = xnext;
-      xnext = load_x(st + 2);
-      cp_async_wait_n<kGvStages - 2>();  // stage st + 1 landed
-      produce(st + 1, xcur);
-    }
-    __syncthreads();
-  }
-  if (warp > 0) cp_async_wait_n<0>();
-  if (warp == 0 && row_ok) {
-    mfdev::renorm(sh, sl);
-    y[2 * i] = sh;
-    y[2 * i + 1] = sl;
-  }
-}
-
-// y(n) = x(k) B(k,n) (vm_impl, matmul.inc:213-239; x is the MAC's first
-// operand).  Producer warp w copies the stage's columns jj with
-// jj % 3 == w - 1, lane l taking k = p0 + l (one 512-byte segment of
-// column-major B per copy instruction), and evaluates exactly the entries it
-// copied; the chain warp's lane j owns column j0 + j.
-template <bool ALIGNED>
-__global__ void __launch_bounds__(kGvThreads) gevm_dd_kernel(const double *__restrict__ x,
-                                                             const double *__restrict__ B,
-                                                             double *__restrict__ y, int64_t K,
-                                                             int64_t N, int64_t ri) {
-  extern __shared__ double2 smem_gv[];
-  double2 *ring = smem_gv;                                   // [stage][column][k pitch]
-  double2 *pq = smem_gv + (size_t)kGvStages * kGvN * kGvPitch;  // [2][k][column pitch]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t j0 = (int64_t)blockIdx.x * kGvN;
-  const int64_t nst = (K + kGvK - 1) / kGvK;
-  const int w = warp - 1;
-  auto issue = [&](int64_t st) {
-    if (st < nst) {
-      double2 *dst = ring + (size_t)(st % kGvStages) * kGvN * kGvPitch;
-      const int64_t p = st * kGvK + lane;
-      const double *src = B + 2 * ((j0 + w) * K + p);
-#pragma unroll
-      for (int jj = w; jj < kGvN; jj += kGvProd, src += 2 * kGvProd * K)
-        load_dd<ALIGNED>(&dst[jj * kGvPitch + lane], src, j0 + jj < N && p < K, B);
-    }
-    cp_async_commit();
-  };
-  auto load_x = [&](int64_t st) {  // lane l: x[st * 32 + l] (zero past k), one stage ahead of use
-    double2 v = make_double2(0.0, 0.0);
-    const int64_t p = st * kGvK + lane;
-    if (st < nst && p < K) {
-      const double *xp = x + 2 * p;
-      v = ALIGNED ? *reinterpret_cast<const double2 *>(xp) : make_double2(xp[0], xp[1]);
-    }
-    return v;
-  };
-  auto produce = [&](int64_t st, double2 xv) {
+  auto produce = [&](int64_t st, double2 (&v)[NX]) {
     if (st >= nst) return;
-    const int64_t p0 = st * kGvK;
-    const int cmax = (K - p0) < kGvK ? (int)(K - p0) : kGvK;
-    if (lane >= cmax) return;  // k = p0 + lane past the end: never read
-    const double2 *src = ring + (size_t)(st % kGvStages) * kGvN * kGvPitch;
-    double2 *out = pq + (size_t)(st & 1) * kGvK * kGvPitch;
+    const double2 *src = ring + ((size_t)(st % S) * kGvN + w) * 32 + lane;
+    double2 *out = pq + (size_t)(st & 1) * kGvK * PITCH;
+    double2 a[COLS];
+    if (XR) {
+      const double2 *xp = xs + (size_t)(st % S) * kGvK;
 #pragma unroll
-    for (int jj = w; jj < kGvN; jj += kGvProd) {
-      const double2 bv = src[jj * kGvPitch + lane];
-      out[lane * kGvPitch + jj] = mac_terms(xv.x, xv.y, bv.x, bv.y);  // pitch 33: conflict-free
+      for (int u = 0; u < NX; ++u) v[u] = xp[VM ? lane : w + u * kGvProd];
+    }
+#pragma unroll
+    for (int u = 0; u < COLS; ++u) a[u] = src[u * kGvProd * 32];
+#pragma unroll
+    for (int u = 0; u < COLS; ++u) {
+      const int c = w + u * kGvProd;
+      if (VM)
+        out[lane * PITCH + c] = mac_terms(v[0].x, v[0].y, a[u].x, a[u].y);  // pitch 33: conflict-free
+      else
+        out[c * PITCH + lane] = mac_terms(a[u].x, a[u].y, v[u % NX].x, v[u % NX].y);
     }
   };
-  double2 xnext = make_double2(0.0, 0.0);
-  if (warp > 0) {
-    for (int s0 = 0; s0 < kGvStages - 1; ++s0) issue(s0);
-    const double2 x0 = load_x(0);
-    xnext = load_x(1);
-    cp_async_wait_n<kGvStages - 2>();
-    produce(0, x0);
+  double2 xa[NX], xb[NX];
+  for (int st = 0; st < S - 1; ++st) issue(st);
+  if (!XR) {
+    load_x(0, xa);
+    load_x(1, xb);
   }
-  __syncthreads();
-  double sh = 0.0, sl = 0.0;
-  int64_t cnt = 0;
+  cp_async_wait_n<S - 2>();  // stage 0 landed
+  if (XR) sync();            // the vector's part of it for every producer
+  produce(0, xa);
+  cp_async_wait_n<PENDING>();
+  sync();
   for (int64_t st = 0; st < nst; ++st) {
-    if (warp == 0) {
-      const int64_t p0 = st * kGvK;
-      const int cmax = (K - p0) < kGvK ? (int)(K - p0) : kGvK;
-      chain_stage(pq + (size_t)(st & 1) * kGvK * kGvPitch, cmax, p0, K, ri, lane, sh, sl, cnt);
-    } else {
-      issue(st + kGvStages - 1);
-      const double2 xcur = xnext;
-      xnext = load_x(st + 2);
-      cp_async_wait_n<kGvStages - 2>();
-      produce(st + 1, xcur);
+    issue(st + S - 1);  // into the slot of stage st - 1, read two iterations ago
+    if (!XR) {
+#pragma unroll
+      for (int u = 0; u < NX; ++u) xa[u] = xb[u];
+      load_x(st + 2, xb);
     }
-    __syncthreads();
+    cp_async_wait_n<PENDING>();  // stage st + 1 landed (XR: st + 2, for the other producers)
+    produce(st + 1, xa);
+    sync();
   }
-  if (warp > 0) cp_async_wait_n<0>();
-  const int64_t j = j0 + lane;
-  if (warp == 0 && j < N) {
-    mfdev::renorm(sh, sl);
-    y[2 * j] = sh;
-    y[2 * j + 1] = sl;
-  }
+  cp_async_wait_n<0>();
 }
 
 static bool aligned16(const void *a, const void *b, const void *c) {
@@ -493,53 +483,46 @@ int cgemm_dev(const complex64x2 *a, const complex64x2 *b, complex64x2 *c, int64_
   return MFCUDA_OK;
 }
 
-// dynamic shared memory above the 48 KB default, set once per process
-static void gv_attrs() {
-  static std::once_flag once;
+// y(m) = A(m,k) x(k), or with VM y(m) = x(k) A(k,m).
+template <bool VM, int S, bool ALIGNED>
+static int launch_gemv(const double *A, const double *x, double *y, int64_t m, int64_t k, int64_t ri, int sms,
+                       cudaStream_t s) {
+  static std::once_flag once;  // dynamic shared memory above the 48 KB default
   std::call_once(once, [] {
-    cudaFuncSetAttribute(gemv_dd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGvSmem);
-    cudaFuncSetAttribute(gemv_dd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGvSmem);
-    cudaFuncSetAttribute(gevm_dd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGvSmem);
-    cudaFuncSetAttribute(gevm_dd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGvSmem);
+    cudaFuncSetAttribute(gemv_dd_kernel<VM, S, ALIGNED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)gv_smem(VM, S));
   });
+  gemv_dd_kernel<VM, S, ALIGNED><<<(unsigned)((m + kGvN - 1) / kGvN), kGvThreads, gv_smem(VM, S), s>>>(A, x, y, m, k,
+                                                                                                  ri, sms);
+  MF_TRY_CUDA(cudaGetLastError());
+  return MFCUDA_OK;
 }
-
-int gemv_dev(const float64x2 *a, const float64x2 *x, float64x2 *y, int64_t m, int64_t k,
-             int64_t ri, cudaStream_t s) {
+template <bool VM>
+static int gemv_any(const float64x2 *a, const float64x2 *x, float64x2 *y, int64_t m, int64_t k, int64_t ri,
+                    cudaStream_t s) {
   if (!shape_ok(m, k, 1, sizeof(float64x2))) return MFCUDA_ERR_INVALID_ARG;
   if (m == 0) return MFCUDA_OK;
   if (!y || (k > 0 && (!a || !x))) return MFCUDA_ERR_INVALID_ARG;
   MF_TRY(require_device());
-  int64_t blocks = (m + kGvN - 1) / kGvN;
+  const int64_t blocks = (m + kGvN - 1) / kGvN;
   if (blocks > INT32_MAX) return MFCUDA_ERR_UNSUPPORTED;
-  gv_attrs();
   const double *A = reinterpret_cast<const double *>(a), *X = reinterpret_cast<const double *>(x);
   double *Y = reinterpret_cast<double *>(y);
+  const int sms = sm_count();
+  const bool one_wave = blocks <= sms;
   if (aligned16(a, x, y))
-    gemv_dd_kernel<true><<<(unsigned)blocks, kGvThreads, kGvSmem, s>>>(A, X, Y, m, k, ri);
-  else
-    gemv_dd_kernel<false><<<(unsigned)blocks, kGvThreads, kGvSmem, s>>>(A, X, Y, m, k, ri);
-  MF_TRY_CUDA(cudaGetLastError());
-  return MFCUDA_OK;
+    return one_wave ? launch_gemv<VM, 8, true>(A, X, Y, m, k, ri, sms, s)
+                    : launch_gemv<VM, 4, true>(A, X, Y, m, k, ri, sms, s);
+  return one_wave ? launch_gemv<VM, 8, false>(A, X, Y, m, k, ri, sms, s)
+                  : launch_gemv<VM, 4, false>(A, X, Y, m, k, ri, sms, s);
 }
-
+int gemv_dev(const float64x2 *a, const float64x2 *x, float64x2 *y, int64_t m, int64_t k,
+             int64_t ri, cudaStream_t s) {
+  return gemv_any<false>(a, x, y, m, k, ri, s);
+}
 int gevm_dev(const float64x2 *x, const float64x2 *b, float64x2 *y, int64_t k, int64_t n,
              int64_t ri, cudaStream_t s) {
-  if (!shape_ok(1, k, n, sizeof(float64x2))) return MFCUDA_ERR_INVALID_ARG;
-  if (n == 0) return MFCUDA_OK;
-  if (!y || (k > 0 && (!b || !x))) return MFCUDA_ERR_INVALID_ARG;
-  MF_TRY(require_device());
-  int64_t blocks = (n + kGvN - 1) / kGvN;
-  if (blocks > INT32_MAX) return MFCUDA_ERR_UNSUPPORTED;
-  gv_attrs();
-  const double *X = reinterpret_cast<const double *>(x), *Bm = reinterpret_cast<const double *>(b);
-  double *Y = reinterpret_cast<double *>(y);
-  if (aligned16(x, b, y))
-    gevm_dd_kernel<true><<<(unsigned)blocks, kGvThreads, kGvSmem, s>>>(X, Bm, Y, k, n, ri);
-  else
-    gevm_dd_kernel<false><<<(unsigned)blocks, kGvThreads, kGvSmem, s>>>(X, Bm, Y, k, n, ri);
-  MF_TRY_CUDA(cudaGetLastError());
-  return MFCUDA_OK;
+  return gemv_any<true>(b, x, y, n, k, ri, s);
 }
 
 // ---- host-pointer (drop-in) forms -----------------------------------------

@@ -164,10 +164,12 @@ __device__ __forceinline__ void gemm_tile(const double *__restrict__ A, const do
       }
     }
     while (kk < kmax) {  // the steps up to the next chunk's end
-      const int end = kk + cad.run(kmax - kk), from = kk;
+      const int run = cad.run(kmax - kk);
+      const double2 *ar = as + kk * BM, *br = bs + kk * PB;
 #pragma unroll(TM * TN >= 16 ? 1 : 4)
-      for (; kk < end; ++kk) step(as + kk * BM, bs + kk * PB);
-      if (cad.ends(kk - from) && k0 + kk < K) renorm_all();
+      for (int u = 0; u < run; ++u) step(ar + u * BM, br + u * PB);
+      kk += run;
+      if (cad.ends(run) && k0 + kk < K) renorm_all();
     }
     __syncthreads();
   }
@@ -295,10 +297,12 @@ __device__ __forceinline__ void cgemm_tile(const double *__restrict__ A, const d
       }
     }
     while (kk < kmax) {  // the steps up to the next chunk's end
-      const int end = kk + cad.run(kmax - kk), from = kk;
+      const int run = cad.run(kmax - kk);
+      const double2 *ar = as + 2 * kk * BM, *br = bs + 2 * kk * PB;
 #pragma unroll(TM * TN >= 4 ? 1 : 4)
-      for (; kk < end; ++kk) step(as + 2 * kk * BM, bs + 2 * kk * PB);
-      if (cad.ends(kk - from) && k0 + kk < K) renorm_all();
+      for (int u = 0; u < run; ++u) step(ar + 2 * u * BM, br + 2 * u * PB);
+      kk += run;
+      if (cad.ends(run) && k0 + kk < K) renorm_all();
     }
     __syncthreads();
   }

@@ -51,3 +51,17 @@ def test_real_tiles_unaligned(dev, shape):
     da, db = (to_dev(np.concatenate([[0.0], x]), dev)[1:] for x in (a, b))
     got = to_host(api.matmuldd_mm(da, db, m, k, n, 8))
     assert O.same_bits(got, O.matmul_mm(a, b, m, k, n, 8)).all()
+
+
+MATVEC = [(1, 1), (31, 7), (33, 32), (40, 33), (65, 64), (130, 259), (148 * 32, 65), (148 * 32 + 5, 97)]
+
+
+@pytest.mark.parametrize("shape", MATVEC)  # one wave of CTAs up to 148 * 32 outputs, two CTAs per SM beyond
+@pytest.mark.parametrize("ri", [8, 0, 5, 24])
+@pytest.mark.parametrize("off", [0, 1])
+def test_matvec_stages(dev, shape, ri, off):
+    m, k = shape
+    a, x = W.dd_uniform(m * k, seed=m), W.dd_uniform(k, seed=k + 3)
+    da, dx = (to_dev(np.concatenate([np.zeros(off), v]), dev)[off:] for v in (a, x))
+    assert O.same_bits(to_host(api.matmuldd_mv(da, dx, m, k, ri)), O.matmul_mv(a, x, m, k, ri)).all()
+    assert O.same_bits(to_host(api.matmuldd_vm(dx, da, k, m, ri)), O.matmul_vm(x, a, k, m, ri)).all()
