@@ -67,14 +67,10 @@ __host__ __device__ inline double crt_bound(int W, int ra, int rb, int64_t k) {
   return (ldexp(1.0, 104 + ra - W) + ldexp(1.0, 104 + rb - W) + ldexp(1.0, 104 + ra + rb - 2 * W) + 0.5) /
          (double)k;
 }
-// Moduli needed for W-bit operands and inner dimension k: M >= 4 k 2^(2W) > 4 |C'|,
-// so |C'| / M < 1/4 and the rounded quotient estimate has a margin of 1/4.
-__host__ __device__ inline int crt_moduli(int W, int64_t k, const int *lg) {
-  const int need = 2 * W + ceil_log2(k) + 2;
-  int n = 1;
-  while (n < CRT_NMAX && lg[n] < need) ++n;
-  return n;
-}
+// Bits the moduli's product must have for W-bit operands and inner dimension k:
+// M >= 4 k 2^(2W) > 4 |C'|, so |C'| / M < 1/4 and the rounded quotient estimate
+// has a margin of 1/4.
+__host__ __device__ inline int crt_need(int W, int64_t k) { return 2 * W + ceil_log2(k) + 2; }
 // Most moduli the CRT form can need for inner dimension k (W <= bits, or
 // W <= CRT_WMAX when bits is 0): workspace sizing on the host.
 inline int crt_slices_max(int64_t k, int bits) {
@@ -98,44 +94,14 @@ __host__ __device__ inline int crt_tc_cols(int nbe) { return (nbe + 4 + 15) / 16
 // count N and the reconstruction constants.  bits > 0 forces W.
 __device__ __forceinline__ void crt_plan_body(const StatSet &st, int bits, double target, int64_t k,
                                               Plan *plan, CrtConst *cc) {
-  __shared__ int red[2][32];
-  __shared__ int sh_n;
-  int r[2] = {0, 0};
-  for (int o = 0; o < st.n; ++o)
-    for (int64_t i = threadIdx.x; i < st.count[o]; i += blockDim.x)
-      if (st.sig[o][i] != SENT_LO) r[st.side[o]] = max(r[st.side[o]], st.sig[o][i] - st.mu[o][i]);
-  int ra = r[0], rb = r[1];
-  for (int off = 16; off >= 1; off >>= 1) {
-    ra = max(ra, __shfl_xor_sync(0xffffffffu, ra, off));
-    rb = max(rb, __shfl_xor_sync(0xffffffffu, rb, off));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = ra;
-    red[1][threadIdx.x >> 5] = rb;
-  }
-  __syncthreads();
+  int ra, rb;
+  plan_spreads(st, ra, rb);
+  int W = bits;
+  if (W <= 0)  // the smallest w in [8, CRT_WMAX] with crt_bound <= target (CRT_WMAX if none)
+    W = plan_first(8, CRT_WMAX, [&](int w) { return crt_bound(w, ra, rb, k) <= target; });
+  const int need = crt_need(W, k);
+  const int n = plan_first(1, CRT_NMAX, [&](int q) { return crt_lg[q] >= need; });
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-      ra = max(ra, red[0][w]);
-      rb = max(rb, red[1][w]);
-    }
-    int W = bits;
-    if (W <= 0) {
-      // the smallest w in [8, CRT_WMAX] with crt_bound <= target (CRT_WMAX if
-      // none); the bound falls strictly with w, so bisection finds it
-      int lo = 8, hi = CRT_WMAX;
-      if (crt_bound(hi, ra, rb, k) <= target) {
-        while (lo < hi) {
-          const int mid = (lo + hi) / 2;
-          if (crt_bound(mid, ra, rb, k) <= target)
-            hi = mid;
-          else
-            lo = mid + 1;
-        }
-      }
-      W = hi;
-    }
-    const int n = crt_moduli(W, k, crt_lg);
     plan->S = n;
     plan->G = n - 1;
     plan->W = W;
@@ -143,10 +109,7 @@ __device__ __forceinline__ void crt_plan_body(const StatSet &st, int bits, doubl
     plan->rho_b = rb;
     plan->crt = 1;
     plan->nl = crt_tc_bytes(W, k) / 4;
-    sh_n = n;
   }
-  __syncthreads();
-  const int n = sh_n;
   // the constants of the n-moduli set, from the tables: column t of E
   if (threadIdx.x < (unsigned)CRT_EB_BYTES) {
     const int t = threadIdx.x;
@@ -171,10 +134,7 @@ __device__ __forceinline__ void crt_plan_body(const StatSet &st, int bits, doubl
   } else if (threadIdx.x < (unsigned)(CRT_EB_BYTES + CRT_NL)) {
     cc->Mw[threadIdx.x - CRT_EB_BYTES] = crt_M_n[n - 1][threadIdx.x - CRT_EB_BYTES];
   }
-  __syncthreads();
-  for (int o = 0; o < st.n; ++o)
-    for (int64_t i = threadIdx.x; i < st.count[o]; i += blockDim.x)
-      if (st.sig[o][i] == SENT_LO) st.sig[o][i] = 0;
+  plan_zero_rows(st);
 }
 
 // ---- residue slicing ----------------------------------------------------------

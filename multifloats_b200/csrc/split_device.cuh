@@ -125,15 +125,6 @@ static inline int take_wait_sticky(bool clear) {
 
 constexpr int SENT_LO = -100000, SENT_HI = 100000;
 
-static __global__ void init_stats_kernel(int *sig, int *mu, int *flag, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    sig[i] = SENT_LO;
-    mu[i] = SENT_HI;
-    flag[i] = 0;
-  }
-}
-
 // floor(log2 v) for a finite v > 0, read from the IEEE-754 fields (subnormals
 // from the position of the leading fraction bit).
 __device__ __forceinline__ int floor_log2(double v) {
@@ -192,62 +183,69 @@ static_assert(SMAX == 14, "for_each_slice_word unrolls 14 digit positions");
 // double2 index e * stride from its base (stride 1 for a real matrix, 2 for the
 // real or imaginary part of a complex one).
 //
-// A column-major m x k: thread per row, a chunk of columns per blockIdx.y.
-__device__ __forceinline__ void scan_a_body(const double *__restrict__ A, int64_t M,
-                                                     int64_t K, int64_t stride, int kchunk, int *sig,
-                                                     int *mu, int *flag, int64_t bx, int64_t by) {
-  int64_t i = bx * blockDim.x + threadIdx.x;
-  if (i >= M) return;
-  int64_t p0 = by * kchunk, p1 = p0 + kchunk < K ? p0 + kchunk : K;
+// Running exponent statistics of some entries of a row or column.
+struct ScanAcc {
   int hi_e = SENT_LO, lo_e = SENT_HI, bad = 0;
-  for (int64_t p = p0; p < p1; ++p) {
-    double2 v = __ldg(reinterpret_cast<const double2 *>(A) + (p * M + i) * stride);
+  __device__ __forceinline__ void add(double2 v) {  // (0, 0) adds nothing
     if (!isfinite(v.x) || !isfinite(v.y)) {
       bad = 1;
-      continue;
+      return;
     }
-    double a = fabs(v.x) + fabs(v.y);
+    const double a = fabs(v.x) + fabs(v.y);
     if (a != 0.0) {
       hi_e = max(hi_e, binade_above(a));
       lo_e = min(lo_e, binade_below(a));
     }
   }
-  if (hi_e != SENT_LO) atomicMax(&sig[i], hi_e);
-  if (lo_e != SENT_HI) atomicMin(&mu[i], lo_e);
-  if (bad) atomicOr(&flag[i], 1);
+  __device__ __forceinline__ void merge_warp() {
+    for (int off = 16; off >= 1; off >>= 1) {
+      hi_e = max(hi_e, __shfl_xor_sync(0xffffffffu, hi_e, off));
+      lo_e = min(lo_e, __shfl_xor_sync(0xffffffffu, lo_e, off));
+      bad |= __shfl_xor_sync(0xffffffffu, bad, off);
+    }
+  }
+  __device__ __forceinline__ void publish(int *sig, int *mu, int *flag) const {
+    if (hi_e != SENT_LO) atomicMax(sig, hi_e);
+    if (lo_e != SENT_HI) atomicMin(mu, lo_e);
+    if (bad) atomicOr(flag, 1);
+  }
+};
+constexpr int SCAN_LOADS = 4;  // entries in flight per thread
+
+// A column-major m x k: thread per row, a chunk of columns per block row by.
+__device__ __forceinline__ void scan_a_body(const double *__restrict__ A, int64_t M, int64_t K, int64_t stride,
+                                            int kchunk, int *sig, int *mu, int *flag, int64_t bx, int64_t by) {
+  const int64_t i = bx * blockDim.x + threadIdx.x;
+  if (i >= M) return;
+  const int64_t p0 = by * kchunk, p1 = p0 + kchunk < K ? p0 + kchunk : K;
+  const double2 *src = reinterpret_cast<const double2 *>(A) + i * stride;
+  ScanAcc acc;
+  for (int64_t p = p0; p < p1; p += SCAN_LOADS) {
+    double2 v[SCAN_LOADS];
+#pragma unroll
+    for (int u = 0; u < SCAN_LOADS; ++u)
+      v[u] = p + u < p1 ? __ldg(src + (p + u) * M * stride) : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int u = 0; u < SCAN_LOADS; ++u) acc.add(v[u]);
+  }
+  acc.publish(&sig[i], &mu[i], &flag[i]);
 }
 
-// B column-major k x n: a block per (column j, chunk of 2048 rows).
-__device__ __forceinline__ void scan_b_body(const double *__restrict__ B, int64_t K,
-                                                     int64_t N, int64_t stride, int *sig, int *mu,
-                                                     int *flag, int64_t bx, int64_t by) {
-  int64_t j = by;
-  int64_t p0 = bx * 2048;
-  int hi_e = SENT_LO, lo_e = SENT_HI, bad = 0;
-  for (int r = 0; r < 8; ++r) {
-    int64_t p = p0 + threadIdx.x + 256 * r;
-    if (p >= K) break;
-    double2 v = __ldg(reinterpret_cast<const double2 *>(B) + (j * K + p) * stride);
-    if (!isfinite(v.x) || !isfinite(v.y)) {
-      bad = 1;
-      continue;
-    }
-    double a = fabs(v.x) + fabs(v.y);
-    if (a != 0.0) {
-      hi_e = max(hi_e, binade_above(a));
-      lo_e = min(lo_e, binade_below(a));
-    }
+// Rows [p0, p1) of column j of B (k x n column-major), by one warp.
+__device__ __forceinline__ ScanAcc scan_column(const double *__restrict__ B, int64_t K, int64_t stride, int64_t j,
+                                               int64_t p0, int64_t p1) {
+  const double2 *src = reinterpret_cast<const double2 *>(B) + j * K * stride;
+  ScanAcc acc;
+  for (int64_t p = p0 + (threadIdx.x & 31); p < p1; p += 32 * SCAN_LOADS) {
+    double2 v[SCAN_LOADS];
+#pragma unroll
+    for (int u = 0; u < SCAN_LOADS; ++u)
+      v[u] = p + 32 * u < p1 ? __ldg(src + (p + 32 * u) * stride) : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int u = 0; u < SCAN_LOADS; ++u) acc.add(v[u]);
   }
-  for (int off = 16; off >= 1; off >>= 1) {
-    hi_e = max(hi_e, __shfl_xor_sync(0xffffffffu, hi_e, off));
-    lo_e = min(lo_e, __shfl_xor_sync(0xffffffffu, lo_e, off));
-    bad |= __shfl_xor_sync(0xffffffffu, bad, off);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (hi_e != SENT_LO) atomicMax(&sig[j], hi_e);
-    if (lo_e != SENT_HI) atomicMin(&mu[j], lo_e);
-    if (bad) atomicOr(&flag[j], 1);
-  }
+  acc.merge_warp();
+  return acc;
 }
 
 // Exponent statistics of the operands of one call: A-side operands (rows of
@@ -260,39 +258,55 @@ struct StatSet {
   int n;
 };
 
-__device__ __forceinline__ void plan_body(const StatSet &st, int slices, double target, Plan *plan) {
-  __shared__ int red[2][32];
+// One block: the largest exponent spread of the A side and of the B side, the
+// same values in every thread.  Reads through L2: the statistics may come from
+// atomics of other blocks of the same launch.
+__device__ __forceinline__ void plan_spreads(const StatSet &st, int &ra, int &rb) {
+  __shared__ int red[2];
+  if (threadIdx.x < 2) red[threadIdx.x] = 0;
   int r[2] = {0, 0};
   for (int o = 0; o < st.n; ++o)
-    for (int64_t i = threadIdx.x; i < st.count[o]; i += blockDim.x)
-      if (st.sig[o][i] != SENT_LO) r[st.side[o]] = max(r[st.side[o]], st.sig[o][i] - st.mu[o][i]);
-  int ra = r[0], rb = r[1];
-  for (int off = 16; off >= 1; off >>= 1) {
-    ra = max(ra, __shfl_xor_sync(0xffffffffu, ra, off));
-    rb = max(rb, __shfl_xor_sync(0xffffffffu, rb, off));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = ra;
-    red[1][threadIdx.x >> 5] = rb;
+    for (int64_t i = threadIdx.x; i < st.count[o]; i += blockDim.x) {
+      const int sg = __ldcg(&st.sig[o][i]);
+      if (sg != SENT_LO) r[st.side[o]] = max(r[st.side[o]], sg - __ldcg(&st.mu[o][i]));
+    }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int v = __reduce_max_sync(0xffffffffu, r[q]);
+    if ((threadIdx.x & 31) == 0) atomicMax(&red[q], v);
   }
   __syncthreads();
+  ra = red[0];
+  rb = red[1];
+}
+// Zero rows / columns: any sigma works, the digits are all zero.
+__device__ __forceinline__ void plan_zero_rows(const StatSet &st) {
+  for (int o = 0; o < st.n; ++o)
+    for (int64_t i = threadIdx.x; i < st.count[o]; i += blockDim.x)
+      if (__ldcg(&st.sig[o][i]) == SENT_LO) st.sig[o][i] = 0;
+}
+// The smallest value of [first, last] whose predicate holds, `last` if none
+// does: one value per thread (at least last - first threads).
+template <class Pred>
+__device__ __forceinline__ int plan_first(int first, int last, Pred holds) {
+  __shared__ int best;
+  __syncthreads();
+  if (threadIdx.x == 0) best = last;
+  __syncthreads();
+  const int v = first + (int)threadIdx.x;
+  if (v < last && holds(v)) atomicMin(&best, v);
+  __syncthreads();
+  return best;
+}
+
+__device__ __forceinline__ void plan_body(const StatSet &st, int slices, double target, Plan *plan) {
+  int ra, rb;
+  plan_spreads(st, ra, rb);
+  int S = slices;
+  if (S <= 0)  // smallest S with (S+1) 2^(106 - 8S + rho_a + rho_b) <= target
+    S = plan_first(2, SMAX, [&](int q) { return (q + 1) * ldexp(1.0, 106 - 8 * q + ra + rb) <= target; });
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-      ra = max(ra, red[0][w]);
-      rb = max(rb, red[1][w]);
-    }
-    int S = slices;
-    if (S <= 0) {
-      // smallest S with (S+1) 2^(106 - 8S + rho_a + rho_b) <= target
-      S = SMAX;
-      for (int q = 2; q <= SMAX; ++q) {
-        double ratio = (q + 1) * ldexp(1.0, 106 - 8 * q + ra + rb);
-        if (ratio <= target) {
-          S = q;
-          break;
-        }
-      }
-    }
     plan->S = S;
     plan->G = S - 1;
     plan->W = 8 * S - 2;
@@ -301,11 +315,7 @@ __device__ __forceinline__ void plan_body(const StatSet &st, int slices, double 
     plan->crt = 0;
     plan->nl = 0;
   }
-  // zero rows / columns: any sigma works, the digits are all zero
-  __syncthreads();
-  for (int o = 0; o < st.n; ++o)
-    for (int64_t i = threadIdx.x; i < st.count[o]; i += blockDim.x)
-      if (st.sig[o][i] == SENT_LO) st.sig[o][i] = 0;
+  plan_zero_rows(st);
 }
 
 // A (m x k column-major) -> As[s][i][p]: a block covers 32 rows x 64
@@ -377,45 +387,15 @@ __device__ __forceinline__ void slice_b_one(const double *__restrict__ B, int64_
     *reinterpret_cast<uint64_t *>(Bs + (((int64_t)sl * N_pad + j) * K_pad + p8)) = word;
   });
 }
-// A block per (column by, range of K): thread t of block bx takes entries
-// (bx * blockDim.x + t) * 8 .. + 7.
-__device__ __forceinline__ void slice_b_body(const double *__restrict__ B, int64_t K,
-                                             int64_t N, int64_t stride, int64_t N_pad,
-                                             int64_t K_pad, const int *sig, const int *flag,
-                                             const Plan *plan, int8_t *__restrict__ Bs, int64_t bx, int64_t by) {
-  const int64_t p8 = (bx * blockDim.x + threadIdx.x) * 8;
-  if (p8 >= K_pad) return;
-  slice_b_one(B, K, N, stride, N_pad, K_pad, sig, flag, plan, Bs, by, p8);
-}
-
-// Column j of B (k x n column-major view) scanned by one warp: lane l reads
-// entries l, l+32, ...; the warp's max / min / or is written by lane 0 (no
-// other warp touches column j).
+// Column j of B (k x n column-major view) scanned by one warp (no other warp
+// touches column j).
 __device__ __forceinline__ void scan_b_warp(const double *__restrict__ B, int64_t K, int64_t stride, int *sig,
                                             int *mu, int *flag, int64_t j) {
-  const int lane = threadIdx.x & 31;
-  int hi_e = SENT_LO, lo_e = SENT_HI, bad = 0;
-  for (int64_t p = lane; p < K; p += 32) {
-    double2 v = __ldg(reinterpret_cast<const double2 *>(B) + (j * K + p) * stride);
-    if (!isfinite(v.x) || !isfinite(v.y)) {
-      bad = 1;
-      continue;
-    }
-    double a = fabs(v.x) + fabs(v.y);
-    if (a != 0.0) {
-      hi_e = max(hi_e, binade_above(a));
-      lo_e = min(lo_e, binade_below(a));
-    }
-  }
-  for (int off = 16; off >= 1; off >>= 1) {
-    hi_e = max(hi_e, __shfl_xor_sync(0xffffffffu, hi_e, off));
-    lo_e = min(lo_e, __shfl_xor_sync(0xffffffffu, lo_e, off));
-    bad |= __shfl_xor_sync(0xffffffffu, bad, off);
-  }
-  if (lane == 0) {
-    sig[j] = hi_e;
-    mu[j] = lo_e;
-    flag[j] = bad;
+  const ScanAcc acc = scan_column(B, K, stride, j, 0, K);
+  if ((threadIdx.x & 31) == 0) {
+    sig[j] = acc.hi_e;
+    mu[j] = acc.lo_e;
+    flag[j] = acc.bad;
   }
 }
 

@@ -62,39 +62,117 @@ namespace split {
 // 1. scan
 // ---------------------------------------------------------------------------
 // ---- kernels of the single-problem pipeline (bodies in split_device.cuh) ----
-__global__ void __launch_bounds__(256) scan_a_kernel(const double *__restrict__ A, int64_t M, int64_t K,
-                                                     int64_t stride, int kchunk, int *sig, int *mu,
-                                                     int *flag) {
-  scan_a_body(A, M, K, stride, kchunk, sig, mu, flag, blockIdx.x, blockIdx.y);
+// One operand of a call: a view of double-double elements (element e at double2
+// index e * stride), its statistics and its slices.  Every phase is one launch
+// over the blocks of all operands (two, or four for a complex product): as a
+// launch per operand the scan phase of a 256^3 call took 44 of its 99 us.
+struct Operand {
+  const double *p;
+  int64_t stride;
+  int64_t rows, rows_pad;  // rows of A or columns of B, and padded
+  int *sig, *mu, *flag;
+  int8_t *slices;
+  int b_side;
+  int chunk;        // scan: columns of A per block, or rows of B per warp
+  unsigned first;   // first block of this operand in the current launch
+};
+struct Operands {
+  Operand op[4];
+  int n;
+  int64_t k, k_pad;
+};
+__device__ __forceinline__ const Operand &operand_of(const Operands &ops, unsigned block) {
+  int o = 0;
+#pragma unroll
+  for (int q = 1; q < 4; ++q)
+    if (q < ops.n && ops.op[q].first <= block) o = q;
+  return ops.op[o];
 }
-__global__ void __launch_bounds__(256) scan_b_kernel(const double *__restrict__ B, int64_t K, int64_t N,
-                                                     int64_t stride, int *sig, int *mu, int *flag) {
-  scan_b_body(B, K, N, stride, sig, mu, flag, blockIdx.x, blockIdx.y);
-}
-// slices_dev (may be NULL): read the slice count there instead (ranks that
-// agreed on one through a collective).
-__global__ void plan_kernel(StatSet st, int slices, double target, Plan *plan, const int *slices_dev) {
-  plan_body(st, slices_dev ? *slices_dev : slices, target, plan);
-}
-__global__ void __launch_bounds__(256) slice_a_kernel(const double *__restrict__ A, int64_t M, int64_t K,
-                                                      int64_t stride, int64_t M_pad, int64_t K_pad,
-                                                      const int *sig, const int *flag, const Plan *plan,
-                                                      int8_t *__restrict__ As) {
-  slice_a_body(A, M, K, stride, M_pad, K_pad, sig, flag, plan, As, blockIdx.x, blockIdx.y);
-}
-__global__ void __launch_bounds__(256) slice_b_kernel(const double *__restrict__ B, int64_t K, int64_t N,
-                                                      int64_t stride, int64_t N_pad, int64_t K_pad,
-                                                      const int *sig, const int *flag, const Plan *plan,
-                                                      int8_t *__restrict__ Bs) {
-  slice_b_body(B, K, N, stride, N_pad, K_pad, sig, flag, plan, Bs, blockIdx.x, blockIdx.y);
+
+// Statistics of every operand to their start values; status[0] and [1] (the
+// scan's ticket) to zero.
+__global__ void __launch_bounds__(256) init_kernel(const __grid_constant__ Operands ops, int *status) {
+  const Operand &op = operand_of(ops, blockIdx.x);
+  const int64_t i = (int64_t)(blockIdx.x - op.first) * blockDim.x + threadIdx.x;
+  if (i < op.rows_pad) {
+    op.sig[i] = SENT_LO;
+    op.mu[i] = SENT_HI;
+    op.flag[i] = 0;
+  }
+  if (blockIdx.x == 0 && threadIdx.x < 2) status[threadIdx.x] = 0;
 }
 
 // ---------------------------------------------------------------------------
 // 2. plan (one block)
 // ---------------------------------------------------------------------------
+// What the plan is made from; arg: slices, or (CRT) operand bits, 0 = from the
+// target.
+struct PlanIn {
+  StatSet st;
+  int crt, arg;
+  double target;
+  int64_t k;
+};
+__device__ __forceinline__ void plan_any(const PlanIn &in, int arg, Plan *plan, CrtConst *cc) {
+  if (in.crt)
+    crt_plan_body(in.st, arg, in.target, in.k, plan, cc);
+  else
+    plan_body(in.st, arg, in.target, plan);
+}
+// Scan of every operand; the block that finishes last makes the plan.
+// A: block = 256 rows x chunk columns; B: warp = one column x chunk rows.
+__global__ void __launch_bounds__(256) scan_plan_kernel(const __grid_constant__ Operands ops,
+                                                        const __grid_constant__ PlanIn in, Plan *plan, CrtConst *cc,
+                                                        int *ticket) {
+  const Operand &op = operand_of(ops, blockIdx.x);
+  const int64_t l = blockIdx.x - op.first;
+  if (op.b_side) {
+    const int64_t w = l * 8 + (threadIdx.x >> 5), segs = (ops.k + op.chunk - 1) / op.chunk;
+    const int64_t j = w / segs, p0 = (w % segs) * op.chunk;
+    if (j < op.rows) {
+      const ScanAcc acc = scan_column(op.p, ops.k, op.stride, j, p0, min(ops.k, p0 + op.chunk));
+      if ((threadIdx.x & 31) == 0) acc.publish(&op.sig[j], &op.mu[j], &op.flag[j]);
+    }
+  } else {
+    const int64_t nbx = (op.rows + 255) / 256;
+    scan_a_body(op.p, op.rows, ops.k, op.stride, op.chunk, op.sig, op.mu, op.flag, l % nbx, l / nbx);
+  }
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  plan_any(in, in.arg, plan, cc);
+}
+// The plan again from a slice count or operand width that ranks agreed on
+// (read on the device).
+__global__ void __launch_bounds__(1024) replan_kernel(const __grid_constant__ PlanIn in, const int *agreed, Plan *plan,
+                                                      CrtConst *cc) {
+  plan_any(in, *agreed, plan, cc);
+}
+
 // ---------------------------------------------------------------------------
 // 3. slice
 // ---------------------------------------------------------------------------
+// Digits: A in blocks of 32 rows x 64 columns, B flat (a thread per 8 entries
+// of a column).
+__global__ void __launch_bounds__(256) slice_kernel(const __grid_constant__ Operands ops, const Plan *plan) {
+  const Operand &op = operand_of(ops, blockIdx.x);
+  const unsigned l = blockIdx.x - op.first;
+  if (op.b_side) {
+    const unsigned per_col = (unsigned)(ops.k_pad / 8), t = l * 256 + threadIdx.x, j = t / per_col;
+    if (j < op.rows_pad)
+      slice_b_one(op.p, ops.k, op.rows, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, plan, op.slices, j,
+                  (int64_t)(t % per_col) * 8);
+  } else {
+    const unsigned nbx = (unsigned)(op.rows_pad / 32);
+    slice_a_body(op.p, op.rows, ops.k, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, plan, op.slices, l % nbx,
+                 l / nbx);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // 4. tcgen05 INT8 MMA, persistent
 // ---------------------------------------------------------------------------
@@ -782,28 +860,24 @@ constexpr int COMBINE_THREADS = 128;
 // ---------------------------------------------------------------------------
 // CRT form (crt_device.cuh): plan, residue slicing, reconstruction
 // ---------------------------------------------------------------------------
-// bits_dev (may be NULL): read the operand width there instead (ranks that
-// agreed on one through a collective).
-__global__ void crt_plan_kernel(StatSet st, int bits, double target, int64_t k, Plan *plan, CrtConst *cc,
-                                const int *bits_dev) {
-  crt_plan_body(st, bits_dev ? *bits_dev : bits, target, k, plan, cc);
-}
-// Block (x, y): column x (a K index) of A, rows 2048 y ..; MN-major planes.
-__global__ void __launch_bounds__(256) crt_slice_a_kernel(const double *__restrict__ A, int64_t M, int64_t K,
-                                                          int64_t stride, int64_t M_pad, int64_t K_pad,
-                                                          const int *sig, const int *flag, const Plan *plan,
-                                                          int8_t *__restrict__ As) {
-  const int64_t i8 = ((int64_t)blockIdx.y * blockDim.x + threadIdx.x) * 8;
-  if (i8 >= M_pad) return;
-  crt_slice_a_mn_one(A, M, K, stride, M_pad, K_pad, sig, flag, plan, As, i8, blockIdx.x);
-}
-__global__ void __launch_bounds__(256) crt_slice_b_kernel(const double *__restrict__ B, int64_t K, int64_t N,
-                                                          int64_t stride, int64_t N_pad, int64_t K_pad,
-                                                          const int *sig, const int *flag, const Plan *plan,
-                                                          int8_t *__restrict__ Bs, int64_t j0) {
-  const int64_t p8 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
-  if (p8 >= K_pad) return;
-  crt_slice_b_one(B, K, N, stride, N_pad, K_pad, sig, flag, plan, Bs, j0 + blockIdx.y, p8);  // column j0 + y
+// Residues, flat over each operand's padded entries: a thread per 8
+// consecutive rows of a K index (A, MN-major planes) or per 8 consecutive K
+// indices of a column (B: columns j0 .. of it).
+__global__ void __launch_bounds__(256) crt_slice_kernel(const __grid_constant__ Operands ops, const Plan *plan,
+                                                        unsigned j0, unsigned j1) {
+  const Operand &op = operand_of(ops, blockIdx.x);
+  const unsigned t = (blockIdx.x - op.first) * 256 + threadIdx.x;
+  if (op.b_side) {
+    const unsigned per_col = (unsigned)(ops.k_pad / 8), j = j0 + t / per_col;
+    if (j < j1)
+      crt_slice_b_one(op.p, ops.k, op.rows, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, plan, op.slices, j,
+                      (int64_t)(t % per_col) * 8);
+  } else {
+    const unsigned per_k = (unsigned)(op.rows_pad / 8), kp = t / per_k;
+    if (kp < ops.k_pad)
+      crt_slice_a_mn_one(op.p, op.rows, ops.k, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, plan, op.slices,
+                         (int64_t)(t % per_k) * 8, kp);
+  }
 }
 // Reconstruction fed by TMA (crt_recon_body): persistent, one CTA per SM;
 // units of 32 rows x one column quad, rows below M, quads qbase .. (columns
@@ -837,7 +911,7 @@ struct Layout {
   int nA, nB;
   int nsl;    // slices per operand allocated (digit slices, or CRT moduli)
   bool pair;  // 256 x (256 nsub) tiles on CTA pairs (m > 128), else 128 x 256 tiles
-  int nsub;   // 256-column halves per pair tile: 2 when n > 256
+  int nsub;   // 256-column halves per pair tile (pair_nsub)
   size_t off_plan, off_crt, off_stats[4], off_slices[4], off_D, total;
 };
 
@@ -853,26 +927,41 @@ static bool use_pair(int64_t m) {
   return enabled && m > BM;
 }
 
-// Output columns per pair tile in 256-column halves (1 or 2; 2 halves the
-// operand bytes per tensor op).  MFCUDA_SPLIT_NSUB=1 or 2 overrides.
-static int pair_nsub() {
-  static const int v = [] {
+// Output columns per pair tile in 256-column halves: 2 reads 2/3 of the
+// operand bytes per tensor op, but has one accumulator, so an item's drain is
+// not hidden; 1 has two.  The cost of a product is rounds x item: the pairs
+// work through ceil(items / pairs) rounds, and an item of one half costs, of
+// half an item of two, 1.05 - 1.5 / kblocks in the CRT form (one product per
+// item: measured 0.87 / 0.94 / 1.01 at 8 / 16 / 32 K blocks) and 1.1 in the
+// digit-sliced form (fifteen products per item: 1.05 - 1.12).  B200, tensor-core
+// phase with always two -> by this rule: CRT 1024^3 52 -> 43 us, 2048^3 216 ->
+// 195, 1500 x 2500 x 700 116 -> 79 (n = 700 pads to 768, not 1024);
+// digit-sliced 1500 x 2500 x 700 378 -> 211.  MFCUDA_SPLIT_NSUB=1 or 2
+// overrides.
+static int pair_nsub(int64_t m, int64_t n, int64_t kblocks, int64_t nkc, int nsl, bool crt) {
+  static const int forced = [] {
     const char *e = getenv("MFCUDA_SPLIT_NSUB");
-    return (e && e[0] == '1') ? 1 : 2;
+    return e && (e[0] == '1' || e[0] == '2') ? e[0] - '0' : 0;
   }();
-  return v;
+  if (n <= BN) return 1;
+  if (forced) return forced;
+  const int64_t pairs = sm_count() / 2, per_tile = (crt ? nsl : (nsl + 1) / 2) * nkc;
+  const int64_t ntm = (m + BM_PAIR - 1) / BM_PAIR;
+  auto rounds = [&](int64_t cols) { return (per_tile * ntm * ((n + cols - 1) / cols) + pairs - 1) / pairs; };
+  const int64_t half = crt ? 1050 - 1500 / kblocks : 1100;  // thousandths
+  return rounds(BN) * half < rounds(2 * BN) * 2000 ? 1 : 2;
 }
 
 static Layout layout(int64_t m, int64_t k, int64_t n, int nA, int nB, int nsl = SMAX, bool crt = false) {
   Layout L;
   L.nsl = nsl;
   L.pair = use_pair(m);
-  L.nsub = L.pair && n > BN ? pair_nsub() : 1;
-  L.M_pad = round_up(m < 1 ? 1 : m, L.pair ? BM_PAIR : BM);
-  L.N_pad = round_up(n < 1 ? 1 : n, BN * L.nsub);
   L.K_pad = round_up(k < 1 ? 1 : k, BK);
   L.kblocks = L.K_pad / BK;
   L.nkc = (L.kblocks + KC_BLOCKS - 1) / KC_BLOCKS;
+  L.nsub = L.pair ? pair_nsub(m, n, L.kblocks, L.nkc, nsl, crt) : 1;
+  L.M_pad = round_up(m < 1 ? 1 : m, L.pair ? BM_PAIR : BM);
+  L.N_pad = round_up(n < 1 ? 1 : n, BN * L.nsub);
   L.nA = nA;
   L.nB = nB;
   size_t off = 0;
@@ -1007,6 +1096,12 @@ size_t crt_workspace_size(int64_t m, int64_t k, int64_t n, int bits, bool comple
   return layout(m, k, n, no, no, crt_slices_max(k, bits), true).total;
 }
 
+// Blocks of an operand in the scan.
+static int64_t scan_blocks(const Operand &op, int64_t k) {
+  const int64_t chunks = (k + op.chunk - 1) / op.chunk;
+  return op.b_side ? (op.rows * chunks + 7) / 8 : ((op.rows + 255) / 256) * chunks;
+}
+
 static std::once_flag g_attr_once;
 
 // Persistent grid of the pair kernel: two CTAs per co-resident cluster.
@@ -1080,7 +1175,7 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
   Plan *plan = reinterpret_cast<Plan *>(base + L.off_plan);
   CrtConst *cc = reinterpret_cast<CrtConst *>(base + L.off_crt);
   int32_t *D = reinterpret_cast<int32_t *>(base + L.off_D);
-  int *status = reinterpret_cast<int *>(base + L.total - 256);
+  int *status = reinterpret_cast<int *>(base + L.total - 256);  // abort codes, the scan's ticket
   const int nops = nA + nB;
   int *sig[4], *mu[4], *flag[4];
   int8_t *sl[4];
@@ -1102,29 +1197,54 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
     });
     prof_call_begin();
     mark(0, s);
-    cudaMemsetAsync(status, 0, sizeof(int), s);
-    const int kch = 64;
-    StatSet st;
-    st.n = nops;
+    Operands ops = {};
+    ops.n = nops;
+    ops.k = k;
+    ops.k_pad = L.K_pad;
+    PlanIn in = {};
+    in.crt = crt;
+    in.arg = slices;
+    in.target = target;
+    in.k = k;
+    in.st.n = nops;
     for (int o = 0; o < nops; ++o) {
       const bool aside = o < nA;
-      int64_t rows = aside ? L.M_pad : L.N_pad;
-      init_stats_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, s>>>(sig[o], mu[o], flag[o], rows);
-      if (aside)
-        scan_a_kernel<<<dim3((unsigned)((m + 255) / 256), (unsigned)((k + kch - 1) / kch)), 256, 0, s>>>(
-            aview[o], m, k, astride[o], kch, sig[o], mu[o], flag[o]);
-      else
-        scan_b_kernel<<<dim3((unsigned)((k + 2047) / 2048), (unsigned)n), 256, 0, s>>>(
-            bview[o - nA], k, n, bstride[o - nA], sig[o], mu[o], flag[o]);
-      st.sig[o] = sig[o];
-      st.mu[o] = mu[o];
-      st.count[o] = aside ? m : n;
-      st.side[o] = aside ? 0 : 1;
+      Operand &op = ops.op[o];
+      op.p = aside ? aview[o] : bview[o - nA];
+      op.stride = aside ? astride[o] : bstride[o - nA];
+      op.rows = aside ? m : n;
+      op.rows_pad = aside ? L.M_pad : L.N_pad;
+      op.sig = sig[o];
+      op.mu = mu[o];
+      op.flag = flag[o];
+      op.slices = sl[o];
+      op.b_side = aside ? 0 : 1;
+      in.st.sig[o] = sig[o];
+      in.st.mu[o] = mu[o];
+      in.st.count[o] = op.rows;
+      in.st.side[o] = op.b_side;
     }
-    if (crt)
-      crt_plan_kernel<<<1, 1024, 0, s>>>(st, slices, target, k, plan, cc, nullptr);
-    else
-      plan_kernel<<<1, 1024, 0, s>>>(st, slices, target, plan, nullptr);
+    // blocks of a phase: blocks_of(operand) per operand, in order
+    auto lay_out = [&](int o0, int o1, auto blocks_of) -> unsigned {
+      int64_t total = 0;
+      for (int o = 0; o < nops; ++o) {
+        ops.op[o].first = (unsigned)total;
+        if (o >= o0 && o < o1) total += blocks_of(ops.op[o]);
+      }
+      // operands before o0 have no blocks: operand_of takes the last one that starts at 0
+      return (unsigned)total;
+    };
+    const unsigned init_blocks = lay_out(0, nops, [](const Operand &op) { return (op.rows_pad + 255) / 256; });
+    init_kernel<<<init_blocks, 256, 0, s>>>(ops, status);
+    // enough blocks to fill the chip, long enough chunks to keep the atomics few
+    for (int o = 0; o < nops; ++o) {
+      Operand &op = ops.op[o];
+      op.chunk = op.b_side ? 1024 : 64;
+      const int64_t want = 8 * (int64_t)sm_count() / nops;
+      while (op.chunk > (op.b_side ? 256 : 16) && scan_blocks(op, k) < want) op.chunk /= 2;
+    }
+    const unsigned scan_total = lay_out(0, nops, [&](const Operand &op) { return scan_blocks(op, k); });
+    scan_plan_kernel<<<scan_total, 256, 0, s>>>(ops, in, plan, cc, status + 1);
     if (agree) {
       // ranks holding other column panels of the same product agree on the
       // largest slice count / operand width (the one the single call would
@@ -1132,35 +1252,26 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
       int *val = crt ? &plan->W : &plan->S;
       rc = agree->fn(agree->ctx, val, s);
       if (rc != MFCUDA_OK) break;
-      if (crt)
-        crt_plan_kernel<<<1, 1024, 0, s>>>(st, slices, target, k, plan, cc, val);
-      else
-        plan_kernel<<<1, 1024, 0, s>>>(st, slices, target, plan, val);
+      replan_kernel<<<1, 1024, 0, s>>>(in, val, plan, cc);
     }
     mark(1, s);
-    const dim3 ga((unsigned)(L.M_pad / 32), (unsigned)(L.K_pad / 64));
-    const dim3 gb((unsigned)((L.K_pad / 8 + 255) / 256), (unsigned)L.N_pad);
-    const dim3 gca((unsigned)L.K_pad, (unsigned)((L.M_pad / 8 + 255) / 256));
     // column panels (CRT form on CTA pairs, when a sink wants the output panel
     // by panel): B's residues, every product and the reconstruction of panel p,
     // then the sink, then panel p + 1
     const int tn_cols = BN * L.nsub;
     const int ntn_all = (int)(L.N_pad / tn_cols);
     const int npan = (sink && crt && L.pair) ? std::max(1, std::min(sink->panels, ntn_all)) : 1;
-    for (int o = 0; o < nops; ++o) {
-      if (o >= nA && npan > 1) continue;  // sliced panel by panel below
-      if (o < nA && crt)
-        crt_slice_a_kernel<<<gca, 256, 0, s>>>(aview[o], m, k, astride[o], L.M_pad, L.K_pad, sig[o], flag[o], plan,
-                                               sl[o]);
-      else if (o < nA)
-        slice_a_kernel<<<ga, 256, 0, s>>>(aview[o], m, k, astride[o], L.M_pad, L.K_pad, sig[o], flag[o], plan,
-                                          sl[o]);
-      else if (crt)
-        crt_slice_b_kernel<<<gb, 256, 0, s>>>(bview[o - nA], k, n, bstride[o - nA], L.N_pad, L.K_pad, sig[o],
-                                              flag[o], plan, sl[o], 0);
-      else
-        slice_b_kernel<<<gb, 256, 0, s>>>(bview[o - nA], k, n, bstride[o - nA], L.N_pad, L.K_pad, sig[o],
-                                          flag[o], plan, sl[o]);
+    auto slice_blocks = [&](const Operand &op) {  // flat: a thread per 8 entries
+      return (op.rows_pad * (L.K_pad / 8) + 255) / 256;
+    };
+    if (crt) {  // with column panels B's residues follow panel by panel
+      const unsigned blocks = lay_out(0, npan > 1 ? nA : nops, slice_blocks);
+      crt_slice_kernel<<<blocks, 256, 0, s>>>(ops, plan, 0, (unsigned)L.N_pad);
+    } else {
+      const unsigned blocks = lay_out(0, nops, [&](const Operand &op) {
+        return op.b_side ? slice_blocks(op) : (op.rows_pad / 32) * (L.K_pad / 64);
+      });
+      slice_kernel<<<blocks, 256, 0, s>>>(ops, plan);
     }
     const int tile_m = L.pair ? BM_PAIR : BM;
     int items_max = L.nsl * (int)L.nkc * (int)((L.M_pad / tile_m) * (L.N_pad / (BN * L.nsub)));
@@ -1187,11 +1298,12 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
       const int tn0 = (int)((int64_t)ntn_all * pp / npan), tn1 = (int)((int64_t)ntn_all * (pp + 1) / npan);
       const int64_t j0 = npan == 1 ? 0 : (int64_t)tn0 * tn_cols;
       const int64_t j1 = npan == 1 ? n : std::min<int64_t>(n, (int64_t)tn1 * tn_cols);
-      if (npan > 1)  // this panel's columns of B (padding columns included)
-        for (int o = nA; o < nops; ++o)
-          crt_slice_b_kernel<<<dim3(gb.x, (unsigned)((tn1 - tn0) * tn_cols)), 256, 0, s>>>(
-              bview[o - nA], k, n, bstride[o - nA], L.N_pad, L.K_pad, sig[o], flag[o], plan, sl[o],
-              (int64_t)tn0 * tn_cols);
+      if (npan > 1) {  // this panel's columns of B (padding columns included)
+        const unsigned c0 = (unsigned)(tn0 * tn_cols), c1 = (unsigned)(tn1 * tn_cols);
+        const unsigned blocks = lay_out(
+            nA, nops, [&](const Operand &) { return ((int64_t)(c1 - c0) * (L.K_pad / 8) + 255) / 256; });
+        crt_slice_kernel<<<blocks, 256, 0, s>>>(ops, plan, c0, c1);
+      }
       int pgrid = grid;
       if (L.pair && npan > 1) {
         const int supers = (crt ? L.nsl : (L.nsl + 1) / 2) * (int)L.nkc * (int)(L.M_pad / tile_m) * (tn1 - tn0);
