@@ -143,9 +143,39 @@ template <> struct KindInfo<3> { static constexpr int NV = 2, ELEM = 4; };
 template <> struct KindInfo<4> { static constexpr int NV = 4, ELEM = 4; };
 template <> struct KindInfo<5> { static constexpr int NV = 1, ELEM = 4; };
 
+// The final step of each kind, applied to the fully combined NV values.
+template <int KIND>
+__device__ __forceinline__ void finish_kind(const dd *v, dd *out) {
+  if constexpr (KIND == 0 || KIND == 1) {
+    out[0] = v[0];
+  } else if constexpr (KIND == 2 || KIND == 5) {
+    out[0] = mfdev::dd_sqrt(v[0]);
+  } else if constexpr (KIND == 3) {
+    out[0] = v[0];
+    out[1] = v[1];
+  } else {
+    out[0] = mfdev::dd_add(v[0], v[1]);  // re = rr + ii
+    out[1] = mfdev::dd_sub(v[2], v[3]);  // im = ri - ir
+  }
+}
+// The result from the combined values: the final step (FINAL), or the values
+// themselves (a partial for a later cross-device combine).
+template <int KIND, bool FINAL>
+__device__ __forceinline__ void store_result(const dd *v, dd *out) {
+  if constexpr (FINAL) {
+    finish_kind<KIND>(v, out);
+  } else {
+#pragma unroll
+    for (int q = 0; q < KindInfo<KIND>::NV; ++q) out[q] = v[q];
+  }
+}
+
 // Stage 1: per-thread serial update over the strided subsequence, block tree,
-// one partial (NV DD values) per block.
-template <int KIND, bool ALIGNED>
+// one partial (NV DD values) per block.  SINGLE: the only block, which stores
+// the result itself -- stage 2 would fold its partial with zeros, eight
+// additions of which the first decides (it normalises, and the rest change
+// nothing); 1000 elements: two launches and a workspace 17 us a call, one launch 8.3.
+template <int KIND, bool ALIGNED, bool SINGLE = false, bool FINAL = true>
 __global__ void __launch_bounds__(kRThreads) reduce_stage1(const double *__restrict__ x,
                                                            const double *__restrict__ y,
                                                            int64_t n, int64_t ri,
@@ -215,24 +245,15 @@ __global__ void __launch_bounds__(kRThreads) reduce_stage1(const double *__restr
     v[0] = s;
   }
   block_combine<NV>(v);
-  if (threadIdx.x == 0)
+  if (threadIdx.x == 0) {
+    if constexpr (SINGLE) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) partials[(int64_t)blockIdx.x * NV + q] = v[q];
-}
-
-// The final step of each kind, applied to the fully combined NV values.
-template <int KIND>
-__device__ __forceinline__ void finish_kind(const dd *v, dd *out) {
-  if constexpr (KIND == 0 || KIND == 1) {
-    out[0] = v[0];
-  } else if constexpr (KIND == 2 || KIND == 5) {
-    out[0] = mfdev::dd_sqrt(v[0]);
-  } else if constexpr (KIND == 3) {
-    out[0] = v[0];
-    out[1] = v[1];
-  } else {
-    out[0] = mfdev::dd_add(v[0], v[1]);  // re = rr + ii
-    out[1] = mfdev::dd_sub(v[2], v[3]);  // im = ri - ir
+      for (int q = 0; q < NV; ++q) v[q] = mfdev::dd_add(v[q], mfdev::make(0.0, 0.0));
+      store_result<KIND, FINAL>(v, partials);
+    } else {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) partials[(int64_t)blockIdx.x * NV + q] = v[q];
+    }
   }
 }
 
@@ -254,14 +275,7 @@ __global__ void __launch_bounds__(kRThreads) reduce_stage2(const dd *__restrict_
     }
   }
   block_combine<NV>(v);
-  if (threadIdx.x == 0) {
-    if constexpr (FINAL) {
-      finish_kind<KIND>(v, out);
-    } else {
-#pragma unroll
-      for (int q = 0; q < NV; ++q) out[q] = v[q];
-    }
-  }
+  if (threadIdx.x == 0) store_result<KIND, FINAL>(v, out);
 }
 
 // Cross-device combine: the partials of `count` devices (NV values each, in
@@ -294,14 +308,21 @@ static int reduce_dev(const double *x, const double *y, int64_t n, int64_t ri, v
   int64_t blocks, threads;
   reduce_geometry(n, &blocks, &threads);
   size_t need = reduce_ws_size(n);
+  bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  if (ws && ws_bytes < need) return MFCUDA_ERR_WORKSPACE;
+  if (blocks == 1) {
+    if (aligned)
+      reduce_stage1<KIND, true, true, FINAL><<<1, (unsigned)threads, 0, s>>>(x, y, n, ri, static_cast<dd *>(out));
+    else
+      reduce_stage1<KIND, false, true, FINAL><<<1, (unsigned)threads, 0, s>>>(x, y, n, ri, static_cast<dd *>(out));
+    MF_TRY_CUDA(cudaGetLastError());
+    return MFCUDA_OK;
+  }
   void *own = nullptr;
   if (!ws) {
     MF_TRY(ws_alloc(&own, need, s));
     ws = own;
-  } else if (ws_bytes < need) {
-    return MFCUDA_ERR_WORKSPACE;
   }
-  bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
   dd *part = static_cast<dd *>(ws);
   if (aligned)
     reduce_stage1<KIND, true><<<(unsigned)blocks, (unsigned)threads, 0, s>>>(x, y, n, ri, part);
