@@ -21,8 +21,18 @@ from ._lib import check, check_last, complex64x2, float64x2, lib
 OP = {"exp": 0, "log": 1, "sin": 2, "cos": 3, "sqrt": 4, "exp2": 5, "log2": 6, "log10": 7}
 
 
+_torch = None  # imported with the first CUDA tensor
+
+
 def _is_dev(x) -> bool:
-    return hasattr(x, "is_cuda") and bool(x.is_cuda)
+    global _torch
+    if not getattr(x, "is_cuda", False):
+        return False
+    if _torch is None:
+        import torch
+
+        _torch = torch
+    return True
 
 
 def _ptr(x) -> int:
@@ -33,10 +43,14 @@ def _ptr(x) -> int:
     return x.ctypes.data
 
 
-def _stream():
-    import torch
+def _stream() -> int:
+    """The current device's current torch stream (read without building a
+    Stream object, which costs a small call a microsecond)."""
+    if _torch is None:  # no CUDA tensor seen yet (an empty batch)
+        import torch
 
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return torch.cuda.current_stream().cuda_stream
+    return _torch._C._cuda_getCurrentRawStream(_torch._C._cuda_getDevice())
 
 
 def _host(x, n_doubles: int, name: str) -> np.ndarray:
@@ -50,9 +64,7 @@ def _dev_check(x, n_doubles: int, name: str):
     """A device call's operand must be a contiguous float64 CUDA tensor: a host
     pointer handed to a kernel would fault, so mixed host / device operands
     are refused here."""
-    import torch
-
-    if (not _is_dev(x) or x.dtype != torch.float64 or not x.is_contiguous() or x.numel() != n_doubles):
+    if not _is_dev(x) or x.dtype != _torch.float64 or not x.is_contiguous() or x.numel() != n_doubles:
         raise ValueError(f"{name}: expected a contiguous float64 CUDA tensor of {n_doubles} doubles")
     return x
 
@@ -67,9 +79,7 @@ def _host_out(x, n_doubles: int, name: str) -> np.ndarray:
 
 def _empty_like_kind(ref, n_doubles: int):
     if _is_dev(ref):
-        import torch
-
-        return torch.empty(n_doubles, dtype=torch.float64, device=ref.device)
+        return ref.new_empty(n_doubles, dtype=_torch.float64)
     return np.empty(n_doubles, dtype=np.float64)
 
 
@@ -250,12 +260,13 @@ def unary(op: str, x, out=None):
     """y[i] = op(x[i]) for op in exp, log, sin, cos, sqrt, exp2, log2, log10."""
     L = lib()
     code = OP[op]
-    n = (x.numel() if _is_dev(x) else np.asarray(x).size) // 2
     if _is_dev(x):
+        n = x.numel() // 2
         x = _dev_check(x, 2 * n, "x")
         y = _dev_check(out, 2 * n, "out") if out is not None else _empty_like_kind(x, 2 * n)
-        check(L.mfcuda_unary_dd(code, _ptr(x), _ptr(y), n, _stream()), "mfcuda_unary_dd")
+        check(L.mfcuda_unary_dd(code, x.data_ptr(), y.data_ptr(), n, _stream()), "mfcuda_unary_dd")
         return y
+    n = np.asarray(x).size // 2
     x = _host(x, 2 * n, "x")
     y = _host_out(out, 2 * n, "out") if out is not None else np.empty(2 * n)
     getattr(L, f"{op}dd_array")(_ptr(x), _ptr(y), n)
@@ -339,10 +350,8 @@ def _dd_tuple(r) -> tuple:
 
 
 def _reduce_dev(fn: str, args: list, out_doubles: int, ref):
-    import torch
-
     L = lib()
-    out = torch.empty(out_doubles, dtype=torch.float64, device=ref.device)
+    out = ref.new_empty(out_doubles, dtype=_torch.float64)
     check(getattr(L, fn)(*args, _ptr(out), None, 0, _stream()), fn)
     return out
 
@@ -451,9 +460,7 @@ def _need(x, doubles: int, name: str):
     if x is None:
         raise ValueError(f"{name}: operand missing")
     if _is_dev(x):
-        import torch
-
-        if x.dtype != torch.float64 or not x.is_contiguous() or x.numel() < doubles:
+        if x.dtype != _torch.float64 or not x.is_contiguous() or x.numel() < doubles:
             raise ValueError(f"{name}: expected a contiguous float64 CUDA tensor of >= {doubles} doubles")
     elif not (isinstance(x, np.ndarray) and x.dtype == np.float64 and x.flags.c_contiguous and x.size >= doubles):
         raise ValueError(f"{name}: expected a contiguous float64 array of >= {doubles} doubles")

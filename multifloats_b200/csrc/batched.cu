@@ -695,7 +695,7 @@ static int create_plain(const mfcuda_gemm_desc *d, int64_t count, int64_t ri, co
   size_t o_items = ar.take(sizeof(PItem) * std::max<size_t>(items.size(), 1));
   size_t o_ctr = ar.take(sizeof(int));
   b->mem_bytes = ar.off;
-  if (injected_alloc_failure() || cudaMalloc(&b->mem, b->mem_bytes) != cudaSuccess) {
+  if (injected_alloc_failure() || device_malloc(&b->mem, b->mem_bytes) != cudaSuccess) {
     (void)cudaGetLastError();
     destroy(b);
     return MFCUDA_ERR_ALLOC;
@@ -887,7 +887,7 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
   b->cfg = cfg;
   cudaGetDevice(&b->device);
   b->mem_bytes = ar.off;
-  if (injected_alloc_failure() || cudaMalloc(&b->mem, b->mem_bytes) != cudaSuccess) {
+  if (injected_alloc_failure() || device_malloc(&b->mem, b->mem_bytes) != cudaSuccess) {
     (void)cudaGetLastError();
     destroy(b);
     return MFCUDA_ERR_ALLOC;
@@ -1088,7 +1088,7 @@ static int create_unary(int op, const float64x2 *const *xs, float64x2 *const *ys
   b->work = total;
   cudaGetDevice(&b->device);
   b->mem_bytes = sizeof(RArr) * std::max<int64_t>(count, 1);
-  if (injected_alloc_failure() || cudaMalloc(&b->mem, b->mem_bytes) != cudaSuccess) {
+  if (injected_alloc_failure() || device_malloc(&b->mem, b->mem_bytes) != cudaSuccess) {
     (void)cudaGetLastError();
     destroy(b);
     return MFCUDA_ERR_ALLOC;
@@ -1163,7 +1163,7 @@ static int tune_bucket(int form, const Bucket &bk, int64_t ri) {
   }
   void *buf = nullptr;
   const int64_t per = 2 * (m * k + k * n + m * n);
-  if (cudaMalloc(&buf, sizeof(double) * per * copies) != cudaSuccess) {
+  if (device_malloc(&buf, sizeof(double) * per * copies) != cudaSuccess) {
     (void)cudaGetLastError();
     return form == 0 ? plain_heuristic(m, n) : 256;
   }

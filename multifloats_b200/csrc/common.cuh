@@ -76,8 +76,11 @@ bool injected_alloc_failure();
 // now on (mfcuda_set_wait_limit_ns; 2 s unless set).
 uint64_t wait_limit_ns();
 
-// Stream-ordered workspace allocation for device-pointer calls given no workspace.
+// Stream-ordered workspace allocation for device-pointer calls given no
+// workspace, from a pool that keeps a bounded amount of free memory.
 int ws_alloc(void **p, size_t bytes, cudaStream_t s);
 void ws_free(void *p, cudaStream_t s);
+// cudaMalloc that gives the pool's free memory back before it fails.
+cudaError_t device_malloc(void **p, size_t bytes);
 
 }  // namespace mfcuda

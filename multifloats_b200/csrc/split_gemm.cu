@@ -903,6 +903,13 @@ __global__ void __launch_bounds__(256) crt_fold_kernel(uint32_t *D, const Plan *
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+// The plan of a call, the abort codes of its kernels and the scan's ticket, read
+// back together.
+struct PlanStatus {
+  Plan plan;
+  int status[2];
+};
+
 // Workspace of one call with nA A-side operands (m x k) and nB B-side
 // operands (k x n): per operand its exponent statistics and SMAX slices, one
 // INT32 diagonal scratch shared by the products, the plan and a status word.
@@ -970,7 +977,7 @@ static Layout layout(int64_t m, int64_t k, int64_t n, int nA, int nB, int nsl = 
     off = (size_t)round_up((int64_t)(off + bytes), 1024);
     return o;
   };
-  L.off_plan = take(sizeof(Plan));
+  L.off_plan = take(sizeof(PlanStatus));
   L.off_crt = take(sizeof(CrtConst));
   for (int o = 0; o < nA + nB; ++o) {
     int64_t rows = o < nA ? L.M_pad : L.N_pad;
@@ -979,7 +986,7 @@ static Layout layout(int64_t m, int64_t k, int64_t n, int nA, int nB, int nsl = 
   }
   // INT32 diagonal sums, or (CRT) one residue byte per output, modulus and K chunk
   L.off_D = take((size_t)nsl * L.nkc * L.N_pad * L.M_pad * (crt ? 1 : sizeof(int32_t)));
-  L.total = off + 256 /* status word */;
+  L.total = off;
   return L;
 }
 
@@ -1172,10 +1179,11 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
     return MFCUDA_ERR_WORKSPACE;
   }
   uint8_t *base = static_cast<uint8_t *>(ws);
-  Plan *plan = reinterpret_cast<Plan *>(base + L.off_plan);
   CrtConst *cc = reinterpret_cast<CrtConst *>(base + L.off_crt);
   int32_t *D = reinterpret_cast<int32_t *>(base + L.off_D);
-  int *status = reinterpret_cast<int *>(base + L.total - 256);  // abort codes, the scan's ticket
+  PlanStatus *ps = reinterpret_cast<PlanStatus *>(base + L.off_plan);
+  Plan *plan = &ps->plan;
+  int *status = ps->status;
   const int nops = nA + nB;
   int *sig[4], *mu[4], *flag[4];
   int8_t *sl[4];
@@ -1340,14 +1348,13 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
     mark(4, s);
     if (rc == MFCUDA_OK && cudaGetLastError() != cudaSuccess) rc = MFCUDA_ERR_CUDA;
     if (info && rc == MFCUDA_OK) {
-      Plan hp;
-      if (cudaMemcpyAsync(&hp, plan, sizeof(Plan), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      PlanStatus h;
+      if (cudaMemcpyAsync(&h, ps, sizeof h, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
           cudaStreamSynchronize(s) != cudaSuccess) {
         rc = MFCUDA_ERR_CUDA;
       } else {
-        int stv = 0;
-        cudaMemcpy(&stv, status, sizeof(int), cudaMemcpyDeviceToHost);
-        if (stv) rc = MFCUDA_ERR_TIMEOUT;
+        const Plan &hp = h.plan;
+        if (h.status[0]) rc = MFCUDA_ERR_TIMEOUT;
         info[0] = hp.S;
         info[1] = hp.rho_a;
         info[2] = hp.rho_b;
