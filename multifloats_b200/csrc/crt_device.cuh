@@ -134,7 +134,6 @@ __device__ __forceinline__ void crt_plan_body(const StatSet &st, int bits, doubl
   } else if (threadIdx.x < (unsigned)(CRT_EB_BYTES + CRT_NL)) {
     cc->Mw[threadIdx.x - CRT_EB_BYTES] = crt_M_n[n - 1][threadIdx.x - CRT_EB_BYTES];
   }
-  plan_zero_rows(st);
 }
 
 // ---- residue slicing ----------------------------------------------------------

@@ -259,17 +259,44 @@ struct StatSet {
 };
 
 // One block: the largest exponent spread of the A side and of the B side, the
-// same values in every thread.  Reads through L2: the statistics may come from
-// atomics of other blocks of the same launch.
+// same values in every thread; rows / columns of zeros get sigma = 0 (any works,
+// their digits are all zero).  Reads through L2, as the statistics may come from
+// atomics of other blocks of the same launch, eight rows per thread in flight
+// (one block sits alone on the chip here: row by row the loads' latency made
+// the plan 15-20 us long).
+constexpr int PLAN_LOADS = 8;
 __device__ __forceinline__ void plan_spreads(const StatSet &st, int &ra, int &rb) {
   __shared__ int red[2];
   if (threadIdx.x < 2) red[threadIdx.x] = 0;
   int r[2] = {0, 0};
-  for (int o = 0; o < st.n; ++o)
-    for (int64_t i = threadIdx.x; i < st.count[o]; i += blockDim.x) {
-      const int sg = __ldcg(&st.sig[o][i]);
-      if (sg != SENT_LO) r[st.side[o]] = max(r[st.side[o]], sg - __ldcg(&st.mu[o][i]));
+#pragma unroll
+  for (int o = 0; o < 4; ++o) {
+    if (o >= st.n) break;
+    int *sig = st.sig[o];
+    const int *mu = st.mu[o];
+    int big = 0;
+    for (int64_t i0 = threadIdx.x; i0 < st.count[o]; i0 += PLAN_LOADS * blockDim.x) {
+      int sg[PLAN_LOADS], m[PLAN_LOADS];
+#pragma unroll
+      for (int u = 0; u < PLAN_LOADS; ++u) {
+        const int64_t i = i0 + (int64_t)u * blockDim.x;
+        const bool in = i < st.count[o];
+        sg[u] = in ? __ldcg(&sig[i]) : 0;
+        m[u] = in ? __ldcg(&mu[i]) : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < PLAN_LOADS; ++u) {
+        if (sg[u] == SENT_LO)
+          sig[i0 + (int64_t)u * blockDim.x] = 0;
+        else
+          big = max(big, sg[u] - m[u]);
+      }
     }
+    if (st.side[o])
+      r[1] = max(r[1], big);
+    else
+      r[0] = max(r[0], big);
+  }
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
@@ -279,12 +306,6 @@ __device__ __forceinline__ void plan_spreads(const StatSet &st, int &ra, int &rb
   __syncthreads();
   ra = red[0];
   rb = red[1];
-}
-// Zero rows / columns: any sigma works, the digits are all zero.
-__device__ __forceinline__ void plan_zero_rows(const StatSet &st) {
-  for (int o = 0; o < st.n; ++o)
-    for (int64_t i = threadIdx.x; i < st.count[o]; i += blockDim.x)
-      if (__ldcg(&st.sig[o][i]) == SENT_LO) st.sig[o][i] = 0;
 }
 // The smallest value of [first, last] whose predicate holds, `last` if none
 // does: one value per thread (at least last - first threads).
@@ -315,7 +336,6 @@ __device__ __forceinline__ void plan_body(const StatSet &st, int slices, double 
     plan->crt = 0;
     plan->nl = 0;
   }
-  plan_zero_rows(st);
 }
 
 // A (m x k column-major) -> As[s][i][p]: a block covers 32 rows x 64
