@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -187,34 +188,30 @@ struct SProb {
   int nsl;       // slice slots per operand: SMAX digits, or the most moduli the CRT plan can use
   CrtConst *cc;  // the plan's reconstruction constants (CRT form)
 };
-// phases with a per-problem block count (prefix sums in a table); the
+// phases with a per-problem block count (and the items, with their prefix sums); the
 // recombination runs in two launches: stores first, then the - / + updates
 enum { PH_SCAN_A, PH_SCAN_B, PH_SLICE_A, PH_SLICE_B, PH_COMBINE, PH_COMBINE2, PH_ITEMS, PH_COUNT };
 
-__device__ __forceinline__ int find_prob(const int64_t *prefix, int nprob, int64_t b) {
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (prefix[mid] <= b)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  return lo;
-}
+// A block's problem and its index among the problem's blocks of the phase, from
+// a table made with the plan: a bisection over the problems' block counts
+// was eleven dependent loads at the head of every block (2000 products, both
+// slicers, the scans and the recombination together 6.1 -> 5.6 ms).
+struct Owner {
+  int p, local;
+};
 
-__global__ void __launch_bounds__(256) g_scan_a(const SProb *probs, const int64_t *prefix, int nprob) {
-  const int p = find_prob(prefix, nprob, blockIdx.x);
-  const SProb &P = probs[p];
-  const int64_t l = blockIdx.x - prefix[p];
+__global__ void __launch_bounds__(256) g_scan_a(const SProb *probs, const Owner *owner) {
+  const Owner own = owner[blockIdx.x];
+  const SProb &P = probs[own.p];
+  const int64_t l = own.local;
   const int64_t nbx = (P.m + 255) / 256;
   scan_a_body(P.A, P.m, P.k, P.astride, 64, P.sigA, P.muA, P.flagA, l % nbx, l / nbx);
 }
 // a warp per column, 8 columns per block
-__global__ void __launch_bounds__(256) g_scan_b(const SProb *probs, const int64_t *prefix, int nprob) {
-  const int p = find_prob(prefix, nprob, blockIdx.x);
-  const SProb &P = probs[p];
-  const int64_t j = (int64_t)(blockIdx.x - prefix[p]) * 8 + (threadIdx.x >> 5);
+__global__ void __launch_bounds__(256) g_scan_b(const SProb *probs, const Owner *owner) {
+  const Owner own = owner[blockIdx.x];
+  const SProb &P = probs[own.p];
+  const int64_t j = (int64_t)own.local * 8 + (threadIdx.x >> 5);
   if (j < P.n) scan_b_warp(P.B, P.k, P.bstride, P.sigB, P.muB, P.flagB, j);
 }
 __global__ void __launch_bounds__(256) g_plan(const SProb *probs, int slices, double target) {
@@ -238,40 +235,40 @@ __global__ void __launch_bounds__(256) g_plan(const SProb *probs, int slices, do
   else
     plan_body(st, slices, target, P.plan);
 }
-__global__ void __launch_bounds__(256) g_slice_a(const SProb *probs, const int64_t *prefix, int nprob) {
-  const int p = find_prob(prefix, nprob, blockIdx.x);
-  const SProb &P = probs[p];
-  const int64_t l = blockIdx.x - prefix[p];
+__global__ void __launch_bounds__(256) g_slice_a(const SProb *probs, const Owner *owner) {
+  const Owner own = owner[blockIdx.x];
+  const SProb &P = probs[own.p];
+  const int64_t l = own.local;
   const int64_t nbx = P.M_pad / 32;
   slice_a_body(P.A, P.m, P.k, P.astride, P.M_pad, P.K_pad, P.sigA, P.flagA, P.plan, P.As, l % nbx, l / nbx);
 }
 // CRT form: residues instead of digits, in MN-major planes As[t][p][i] (the
 // rows of one K index contiguous); flat: thread t of the problem takes K
 // index t / (M_pad / 8), rows 8 (t % (M_pad / 8)) .. + 7
-__global__ void __launch_bounds__(256) g_crt_slice_a(const SProb *probs, const int64_t *prefix, int nprob) {
-  const int p = find_prob(prefix, nprob, blockIdx.x);
-  const SProb &P = probs[p];
-  const int64_t t = (int64_t)(blockIdx.x - prefix[p]) * 256 + threadIdx.x;
+__global__ void __launch_bounds__(256) g_crt_slice_a(const SProb *probs, const Owner *owner) {
+  const Owner own = owner[blockIdx.x];
+  const SProb &P = probs[own.p];
+  const int64_t t = (int64_t)own.local * 256 + threadIdx.x;
   const int64_t per_k = P.M_pad / 8;
   const int64_t kp = t / per_k;
   if (kp < P.K_pad)
     crt_slice_a_mn_one(P.A, P.m, P.k, P.astride, P.M_pad, P.K_pad, P.sigA, P.flagA, P.plan, P.As,
                        (t % per_k) * 8, kp);
 }
-__global__ void __launch_bounds__(256) g_crt_slice_b(const SProb *probs, const int64_t *prefix, int nprob) {
-  const int p = find_prob(prefix, nprob, blockIdx.x);
-  const SProb &P = probs[p];
-  const int64_t t = (int64_t)(blockIdx.x - prefix[p]) * 256 + threadIdx.x;
+__global__ void __launch_bounds__(256) g_crt_slice_b(const SProb *probs, const Owner *owner) {
+  const Owner own = owner[blockIdx.x];
+  const SProb &P = probs[own.p];
+  const int64_t t = (int64_t)own.local * 256 + threadIdx.x;
   const int64_t per_col = P.K_pad / 8;
   const int64_t j = t / per_col;
   if (j < P.N_pad)
     crt_slice_b_one(P.B, P.k, P.n, P.bstride, P.N_pad, P.K_pad, P.sigB, P.flagB, P.plan, P.Bs, j, (t % per_col) * 8);
 }
 // flat: thread t of the problem takes column t / (K_pad / 8), entries 8 (t % (K_pad / 8)) .. + 7
-__global__ void __launch_bounds__(256) g_slice_b(const SProb *probs, const int64_t *prefix, int nprob) {
-  const int p = find_prob(prefix, nprob, blockIdx.x);
-  const SProb &P = probs[p];
-  const int64_t t = (int64_t)(blockIdx.x - prefix[p]) * 256 + threadIdx.x;
+__global__ void __launch_bounds__(256) g_slice_b(const SProb *probs, const Owner *owner) {
+  const Owner own = owner[blockIdx.x];
+  const SProb &P = probs[own.p];
+  const int64_t t = (int64_t)own.local * 256 + threadIdx.x;
   const int64_t per_col = P.K_pad / 8;
   const int64_t j = t / per_col;
   if (j < P.N_pad)
@@ -283,10 +280,10 @@ constexpr int kCombineThreads = 128;
 static int64_t combine_blocks(int64_t m, int64_t n) {
   return (((m + 3) / 4) * n + kCombineThreads - 1) / kCombineThreads;
 }
-__global__ void __launch_bounds__(kCombineThreads) g_combine(const SProb *probs, const int64_t *prefix, int nprob) {
-  const int p = find_prob(prefix, nprob, blockIdx.x);
-  const SProb &P = probs[p];
-  const int64_t t = (int64_t)(blockIdx.x - prefix[p]) * kCombineThreads + threadIdx.x;
+__global__ void __launch_bounds__(kCombineThreads) g_combine(const SProb *probs, const Owner *owner) {
+  const Owner own = owner[blockIdx.x];
+  const SProb &P = probs[own.p];
+  const int64_t t = (int64_t)own.local * kCombineThreads + threadIdx.x;
   const int64_t q = (P.m + 3) / 4;
   combine4_body(P.D, P.plan, P.sigA, P.flagA, P.sigB, P.flagB, P.m, P.n, P.M_pad, P.N_pad, P.nkc, P.C,
                 P.cstride, P.mode, t % q, t / q);
@@ -297,45 +294,96 @@ __global__ void __launch_bounds__(kCombineThreads) g_combine(const SProb *probs,
 static int64_t crt_combine_blocks(int64_t m, int64_t n) {
   return ((m + CTC_THREADS - 1) / CTC_THREADS) * (((n + 3) / 4 + CTC_QUADS - 1) / CTC_QUADS);
 }
-__global__ void __launch_bounds__(CTC_THREADS, 4) g_crt_combine(const SProb *probs, const int64_t *prefix, int nprob,
+__global__ void __launch_bounds__(CTC_THREADS, 4) g_crt_combine(const SProb *probs, const Owner *owner,
                                                              int *status, uint64_t wait_ns) {
   extern __shared__ uint8_t ctc_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(ctc_raw) + 1023) & ~uintptr_t(1023));
-  const int p = find_prob(prefix, nprob, blockIdx.x);
-  const SProb &P = probs[p];
-  const int64_t l = blockIdx.x - prefix[p], nbx = (P.m + CTC_THREADS - 1) / CTC_THREADS;
+  const Owner own = owner[blockIdx.x];
+  const SProb &P = probs[own.p];
+  const int64_t l = own.local, nbx = (P.m + CTC_THREADS - 1) / CTC_THREADS;
   crt_combine_tc_body(reinterpret_cast<const uint8_t *>(P.D), P.plan, P.cc, P.sigA, P.flagA, P.sigB, P.flagB, P.m,
                       P.n, P.M_pad, P.N_pad, P.nkc, P.k, P.C, P.cstride, P.mode, (l % nbx) * CTC_THREADS,
                       (l / nbx) * CTC_QUADS, smem, status, wait_ns);
 }
 
-struct GItem {
-  int g, kc, tm, tn;
+// Work item of the tensor-core kernels, with all they need to know of its
+// problem.  The list is written on the device once the plans are known
+// (g_items) and every role reads its next entry while it works on the current
+// one: finding an item's problem by bisection and walking to its plan was a
+// dozen dependent loads per role and item, about 10 of the 13 us an item took.
+struct __align__(16) GItem {
+  int p;           // problem (tensor maps 2 p, 2 p + 1)
+  int g, nd;       // digits: diagonals g, g - 1, ... (nd of them); CRT: modulus g, nd = 1; nd = 0: beyond the plan
+  int kb0, kb1;    // K blocks
+  int a_row, b_row;  // first row of A and column of B
+  int bn;
+  int M_pad, pad[3];
+  int32_t *dst;    // D of diagonal / modulus g, K chunk and tile
+  int64_t gstride;  // INT32 sums between diagonals
 };
-__device__ __forceinline__ GItem decode_item(const SProb &P, int64_t local) {
+static_assert(sizeof(GItem) == 64 && offsetof(GItem, M_pad) == 32 && offsetof(GItem, dst) == 48, "read by load_item");
+// Field by field: a struct filled through a pointer would live in local memory
+// and be read again after every barrier wait.
+__device__ __forceinline__ GItem load_item(const GItem *items, int64_t w, int64_t n) {
   GItem it;
-  const int ntiles = P.ntm * P.ntn;
-  const int64_t per_g = (int64_t)P.nkc * ntiles;
-  it.g = P.nsl - 1 - (int)(local / per_g);
-  const int64_t r = local % per_g;
-  it.kc = (int)(r / ntiles);
-  const int tile = (int)(r % ntiles);
-  it.tm = tile % P.ntm;
-  it.tn = tile / P.ntm;
+  it.nd = 0;
+  if (w < n) {
+    const int4 *src = reinterpret_cast<const int4 *>(items + w);
+    const int4 a = __ldg(src), b = __ldg(src + 1);
+    const int2 c = __ldg(reinterpret_cast<const int2 *>(src + 2));
+    const longlong2 e = __ldg(reinterpret_cast<const longlong2 *>(src + 3));
+    it.p = a.x;
+    it.g = a.y;
+    it.nd = a.z;
+    it.kb0 = a.w;
+    it.kb1 = b.x;
+    it.a_row = b.y;
+    it.b_row = b.z;
+    it.bn = b.w;
+    it.M_pad = c.x;
+    it.dst = reinterpret_cast<int32_t *>(e.x);
+    it.gstride = e.y;
+  }
   return it;
 }
+// Diagonals of an item of the digit-sliced form.
+constexpr int GD_DIAGS = 2;
+__host__ __device__ constexpr int g_groups(int nsl, bool crt) { return crt ? nsl : (nsl + GD_DIAGS - 1) / GD_DIAGS; }
+// A block per problem: its items, the longest first.
+__global__ void __launch_bounds__(128) g_items(const SProb *probs, const int64_t *prefix, GItem *items) {
+  const SProb &P = probs[blockIdx.x];
+  const int G = P.plan->G, ntiles = P.ntm * P.ntn, per_g = P.nkc * ntiles, groups = g_groups(P.nsl, P.crt != 0);
+  for (int64_t l = threadIdx.x; l < (int64_t)groups * per_g; l += blockDim.x) {
+    GItem it;
+    const int q = (int)(l / per_g), r = (int)(l % per_g), kc = r / ntiles, tile = r % ntiles;
+    it.p = (int)blockIdx.x;
+    it.g = P.crt ? P.nsl - 1 - q : G - GD_DIAGS * q;
+    it.nd = P.crt ? (it.g <= G ? 1 : 0) : max(0, min(GD_DIAGS, it.g + 1));
+    it.kb0 = kc * P.kcb;
+    it.kb1 = min(P.kblocks, it.kb0 + P.kcb);
+    it.a_row = tile % P.ntm * BM;
+    it.b_row = tile / P.ntm * P.bn;
+    it.bn = P.bn;
+    it.M_pad = (int)P.M_pad;
+    it.pad[0] = it.pad[1] = it.pad[2] = 0;
+    it.gstride = (int64_t)P.nkc * P.N_pad * P.M_pad;
+    const int64_t off = (int64_t)max(it.g, 0) * it.gstride + ((int64_t)kc * P.N_pad + it.b_row) * P.M_pad + it.a_row;
+    // CRT: one byte per output, four columns per 32-bit word (crt_device.cuh)
+    it.dst = P.crt ? P.D + crt_word_index(off, P.M_pad) : P.D + off;
+    items[prefix[blockIdx.x] + l] = it;
+  }
+}
 
-// Persistent tensor-core kernel over every problem's items (static
-// round-robin).  The warp roles and barriers of split_mma_kernel, with eight
-// epilogue warps (two per TMEM lane quadrant, each draining half of the
-// accumulator's columns); per item it looks up the problem, skips diagonals
-// beyond the problem's plan, and uses the problem's tensor maps (global
-// memory) and tile width.
+// Persistent tensor-core kernel of the CRT form over every problem's items,
+// one product of a modulus, K chunk and tile each (static round-robin).  The
+// warp roles and barriers of split_mma_kernel, with eight epilogue warps (two
+// per TMEM lane quadrant, each draining half of the accumulator's columns); per
+// item it uses the problem's tensor maps (global memory) and tile width.
 constexpr int G_EPI_WARPS = 8;
 constexpr int G_THREADS = 64 + 32 * G_EPI_WARPS;  // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 __global__ void __launch_bounds__(G_THREADS, 1)
-    g_mma(const SProb *__restrict__ probs, const CUtensorMap *__restrict__ maps,
-          const int64_t *__restrict__ prefix, int nprob, int64_t items, int *status, uint64_t wait_ns) {
+    g_crt_mma(const GItem *__restrict__ items, int64_t nitems, const CUtensorMap *__restrict__ maps, int *status,
+              uint64_t wait_ns) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t *sA = smem;
@@ -376,45 +424,31 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   };
   ArmedStages<NSTAGE> arm;  // the producer's armed stages
   arm.clear();
-  // item -> (problem, decoded item, active?)
-  auto lookup = [&](int64_t w, int &p, GItem &it) -> bool {
-    p = find_prob(prefix, nprob, w);
-    const SProb &P = probs[p];
-    it = decode_item(P, w - prefix[p]);
-    return it.g <= P.plan->G;
-  };
-
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int64_t w = blockIdx.x; w < items && ok; w += gridDim.x) {
-        int p;
-        GItem it;
-        if (!lookup(w, p, it)) continue;
-        const SProb &P = probs[p];
-        const int kb0 = it.kc * P.kcb, kb1 = min(P.kblocks, kb0 + P.kcb);
-        const uint32_t bytes = (uint32_t)(A_STAGE + P.bn * BK);
-        for (int s = P.crt ? it.g : 0; s <= it.g && ok; ++s) {  // CRT: the single product A_g B_g
-          for (int kb = kb0; kb < kb1; ++kb) {
-            if (!wait_bar(&empty[stage], phase ^ 1, abort_flag, wait_ns)) {
-              fail(1);
-              ok = false;
-              break;
-            }
-            mftc::mbar_arrive_expect_tx(&full[stage], bytes);
-            if (P.crt)  // MN-major residue planes: (row, K index, modulus)
-              mftc::tma_load_3d(sA + stage * A_STAGE, &maps[2 * p], &full[stage], it.tm * BM, kb * BK, s);
-            else
-              mftc::tma_load_3d(sA + stage * A_STAGE, &maps[2 * p], &full[stage], kb * BK, it.tm * BM, s);
-            mftc::tma_load_3d(sB + stage * B_STAGE, &maps[2 * p + 1], &full[stage], kb * BK, it.tn * P.bn,
-                              P.crt ? s : it.g - s);
-            arm.arm(stage, phase);
-            if (++stage == NSTAGE) {
-              stage = 0;
-              phase ^= 1;
-            }
+      GItem next = load_item(items, blockIdx.x, nitems);
+      for (int64_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+        const GItem it = next;
+        next = load_item(items, w + gridDim.x, nitems);
+        if (!it.nd) continue;
+        const uint32_t bytes = (uint32_t)(A_STAGE + it.bn * BK);
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
+          if (!wait_bar(&empty[stage], phase ^ 1, abort_flag, wait_ns)) {
+            fail(1);
+            ok = false;
+            break;
+          }
+          mftc::mbar_arrive_expect_tx(&full[stage], bytes);
+          // A: MN-major residue planes (row, K index, modulus)
+          mftc::tma_load_3d(sA + stage * A_STAGE, &maps[2 * it.p], &full[stage], it.a_row, kb * BK, it.g);
+          mftc::tma_load_3d(sB + stage * B_STAGE, &maps[2 * it.p + 1], &full[stage], kb * BK, it.b_row, it.g);
+          arm.arm(stage, phase);
+          if (++stage == NSTAGE) {
+            stage = 0;
+            phase ^= 1;
           }
         }
       }
@@ -426,15 +460,13 @@ __global__ void __launch_bounds__(G_THREADS, 1)
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int64_t w = blockIdx.x; w < items && ok; w += gridDim.x) {
-        int p;
-        GItem it;
-        if (!lookup(w, p, it)) continue;
-        const SProb &P = probs[p];
-        const int kb0 = it.kc * P.kcb, kb1 = min(P.kblocks, kb0 + P.kcb);
-        // CRT residues are unsigned, and A's planes MN-major (a K step of 32 rows is 4096 bytes)
-        const uint32_t idesc = P.crt ? mftc::idesc_u8(BM, P.bn) | mftc::IDESC_A_MN : mftc::idesc_i8(BM, P.bn);
-        const uint32_t a_kstep = P.crt ? 32 * 128 : UMMA_K;
+      GItem next = load_item(items, blockIdx.x, nitems);
+      for (int64_t w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+        const GItem it = next;
+        next = load_item(items, w + gridDim.x, nitems);
+        if (!it.nd) continue;
+        const uint32_t idesc = mftc::idesc_u8(BM, it.bn) | mftc::IDESC_A_MN;
+        const uint32_t a_kstep = 32 * 128;  // a K step of 32 rows of the MN-major A tile
         if (!wait_bar(&tempty[acc], acc_phase ^ 1, abort_flag, wait_ns)) {
           fail(2);
           break;
@@ -442,27 +474,25 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         mftc::tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
         uint32_t accumulate = 0;
-        for (int s = P.crt ? it.g : 0; s <= it.g && ok; ++s) {
-          for (int kb = kb0; kb < kb1; ++kb) {
-            if (!wait_bar(&full[stage], phase, abort_flag, wait_ns)) {
-              fail(4);
-              ok = false;
-              break;
-            }
-            mftc::tc_fence_after();
-            const uint32_t a0 = mftc::smem_u32(sA + stage * A_STAGE);
-            const uint32_t b0 = mftc::smem_u32(sB + stage * B_STAGE);
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
+          if (!wait_bar(&full[stage], phase, abort_flag, wait_ns)) {
+            fail(4);
+            ok = false;
+            break;
+          }
+          mftc::tc_fence_after();
+          const uint32_t a0 = mftc::smem_u32(sA + stage * A_STAGE);
+          const uint32_t b0 = mftc::smem_u32(sB + stage * B_STAGE);
 #pragma unroll
-            for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-              mftc::umma_i8(d_tmem, mftc::smem_desc_k_sw128(a0 + kk * a_kstep),
-                            mftc::smem_desc_k_sw128(b0 + kk * UMMA_K), idesc, accumulate);
-              accumulate = 1;
-            }
-            mftc::umma_commit(&empty[stage]);
-            if (++stage == NSTAGE) {
-              stage = 0;
-              phase ^= 1;
-            }
+          for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+            mftc::umma_i8(d_tmem, mftc::smem_desc_k_sw128(a0 + kk * a_kstep),
+                          mftc::smem_desc_k_sw128(b0 + kk * UMMA_K), idesc, accumulate);
+            accumulate = 1;
+          }
+          mftc::umma_commit(&empty[stage]);
+          if (++stage == NSTAGE) {
+            stage = 0;
+            phase ^= 1;
           }
         }
         if (!ok) break;
@@ -483,41 +513,28 @@ __global__ void __launch_bounds__(G_THREADS, 1)
     const int row = quad * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
-    for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
-      int p;
-      GItem it;
-      if (!lookup(w, p, it)) continue;
-      const SProb &P = probs[p];
+    GItem next = load_item(items, blockIdx.x, nitems);
+    for (int64_t w = blockIdx.x; w < nitems; w += gridDim.x) {
+      const GItem it = next;
+      next = load_item(items, w + gridDim.x, nitems);
+      if (!it.nd) continue;
       bool got = wait_bar(&tfull[acc], acc_phase, abort_flag, wait_ns);
       if (!__all_sync(0xffffffffu, got)) {
         if (lane == 0) fail(8);
         break;
       }
       mftc::tc_fence_after();
-      const int64_t off = ((int64_t)(it.g * P.nkc + it.kc) * P.N_pad + (int64_t)it.tn * P.bn) * P.M_pad +
-                          (int64_t)it.tm * BM + row;
-      const int nch = P.bn / 64, ch0 = half * nch;  // this warp's 32-column chunks
-      if (P.crt) {  // residues modulo m_g, four columns per 32-bit word (crt_device.cuh)
-        uint32_t *dst = reinterpret_cast<uint32_t *>(P.D) + crt_word_index(off, P.M_pad) + (int64_t)ch0 * 8 * P.M_pad;
-        for (int chunk = ch0; chunk < ch0 + nch; ++chunk) {
-          uint32_t r[32];
-          mftc::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN + chunk * 32), r);
-          mftc::tmem_wait_ld();
+      const int nch = it.bn / 64, ch0 = half * nch;  // this warp's 32-column chunks
+      // residues modulo m_g, four columns per 32-bit word (crt_device.cuh)
+      uint32_t *dst = reinterpret_cast<uint32_t *>(it.dst) + row + (int64_t)ch0 * 8 * it.M_pad;
+      for (int chunk = ch0; chunk < ch0 + nch; ++chunk) {
+        uint32_t r[32];
+        mftc::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN + chunk * 32), r);
+        mftc::tmem_wait_ld();
 #pragma unroll
-          for (int g = 0; g < 8; ++g) {
-            __stcs(dst, crt_pack4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3], it.g));
-            dst += P.M_pad;
-          }
-        }
-      } else {
-        int32_t *dst_base = P.D + off;
-        for (int chunk = ch0; chunk < ch0 + nch; ++chunk) {
-          uint32_t r[32];
-          mftc::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN + chunk * 32), r);
-          mftc::tmem_wait_ld();
-          int32_t *dst = dst_base + (int64_t)chunk * 32 * P.M_pad;
-#pragma unroll
-          for (int q = 0; q < 32; ++q) __stcs(dst + (int64_t)q * P.M_pad, (int32_t)r[q]);  // evict-first: keep L2 for the slices
+        for (int g = 0; g < 8; ++g) {
+          __stcs(dst, crt_pack4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3], it.g));
+          dst += it.M_pad;
         }
       }
       mftc::tc_fence_before();
@@ -535,6 +552,288 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   if (*abort_flag) {  // read after the barrier: the same value in every thread
     // copies in flight that no MMA consumed land before shared memory is released
     if (warp == 0 && lane == 0) arm.drain(full, NSTAGE);
+    __syncthreads();
+  }
+  if (warp == 1) {
+    __syncwarp();
+    mftc::tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+}
+
+// Persistent tensor-core kernel of the digit-sliced form.  An item is two
+// consecutive diagonals g, g - 1 of one tile (128 rows x bn <= 256 columns) and
+// K chunk, accumulated side by side in tensor memory.  Per K block the slices
+// come in the order A_0, B_g, B_{g-1}, A_1, B_{g-2}, ...: step s multiplies A_s
+// with B_{g-s} and B_{g-s-1}, one product per diagonal, and then lets A_s and
+// B_{g-s} go, so each slice is loaded once for both diagonals.  A and B have
+// rings of their own because a step holds two B tiles but one A tile.
+//
+// CTAs take items from a counter (the producer does, one item ahead, and hands
+// each to the other roles through a small ring in shared memory): dealt round
+// robin the busiest CTA had 16 % more work than the mean.
+//
+// Bound: the tensor pipe while an item runs (two thirds of the issuing
+// thread's time goes into MMAs waiting for it), then the drain, hidden only
+// behind the next item's loads (the accumulators fill tensor memory; they are
+// handed back one by one in the order the next item needs them).  Four
+// diagonals on 128 x 128 tiles load less, but a 128-column MMA takes 102 cycles
+// instead of its 64 (shared-memory reads).  2000 products of sizes up to 1024:
+// 9.0 ms with one diagonal at a time and items found by bisection, 7.8 four by
+// 128 columns, 6.0 two by 256.
+constexpr int GD_BN = BN, GD_NA = 4, GD_NB = 5, GD_NW = 4;
+constexpr int GD_TILE_A = A_STAGE, GD_TILE_B = B_STAGE;  // bytes of a slot
+constexpr int GD_SMEM = GD_NA * GD_TILE_A + GD_NB * GD_TILE_B + 1024 /*align*/ + 512 /*barriers, items*/;
+static_assert(GD_DIAGS * GD_BN == TMEM_COLS && GD_NB > GD_DIAGS, "accumulators fill tensor memory");
+
+// Position in a ring of N slots and the parity of its current pass.
+template <int N>
+struct RingPos {
+  int slot = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void advance() {
+    if (++slot == N) {
+      slot = 0;
+      phase ^= 1;
+    }
+  }
+  __device__ __forceinline__ int at(int d) const { return slot + d < N ? slot + d : slot + d - N; }
+  __device__ __forceinline__ uint32_t phase_at(int d) const { return slot + d < N ? phase : phase ^ 1; }
+};
+
+__global__ void __launch_bounds__(G_THREADS, 1)
+    g_digit_mma(const GItem *__restrict__ items, int64_t nitems, int *counter, const CUtensorMap *__restrict__ maps,
+                int *status, uint64_t wait_ns) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *sA = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t *sB = sA + GD_NA * GD_TILE_A;
+  uint64_t *fullA = reinterpret_cast<uint64_t *>(sB + GD_NB * GD_TILE_B);
+  uint64_t *emptyA = fullA + GD_NA;
+  uint64_t *fullB = emptyA + GD_NA;
+  uint64_t *emptyB = fullB + GD_NB;
+  uint64_t *tempty = emptyB + GD_NB;    // per accumulator
+  uint64_t *tfull = tempty + GD_DIAGS;  // the item's accumulators
+  uint64_t *wfull = tfull + 1;  // the ring of items
+  uint64_t *wempty = wfull + GD_NW;
+  uint64_t *drain = wempty + GD_NW;
+  GItem *work = reinterpret_cast<GItem *>((reinterpret_cast<uintptr_t>(drain + 2) + 15) & ~uintptr_t(15));
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < GD_NA; ++s) {
+      mftc::mbar_init(&fullA[s], 1);
+      mftc::mbar_init(&emptyA[s], 1);
+    }
+    for (int s = 0; s < GD_NB; ++s) {
+      mftc::mbar_init(&fullB[s], 1);
+      mftc::mbar_init(&emptyB[s], 1);
+    }
+    for (int d = 0; d < GD_DIAGS; ++d) mftc::mbar_init(&tempty[d], G_EPI_WARPS);
+    mftc::mbar_init(tfull, 1);
+    for (int s = 0; s < GD_NW; ++s) {
+      mftc::mbar_init(&wfull[s], 1);
+      mftc::mbar_init(&wempty[s], 1 + G_EPI_WARPS);  // the issuer and every epilogue warp
+    }
+    mftc::mbar_init(drain, 1);
+    *abort_flag = 0;
+    mftc::fence_mbar_init();
+  }
+  if (warp == 1) {
+    mftc::tmem_alloc(tmem_slot, TMEM_COLS);
+    mftc::tmem_relinquish();
+  }
+  mftc::tc_fence_before();
+  __syncthreads();
+  mftc::tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  auto fail = [&](int code) {
+    *abort_flag = 1;
+    record_abort(status, code);
+  };
+  ArmedStages<GD_NA> armA;  // the producer's armed slots
+  ArmedStages<GD_NB> armB;
+  armA.clear();
+  armB.clear();
+
+  if (warp == 0) {
+    if (lane == 0) {  // ---- TMA producer
+      RingPos<GD_NA> ra;
+      RingPos<GD_NB> rb;
+      RingPos<GD_NW> rw;
+      bool ok = true;
+      int64_t w = (unsigned)atomicAdd(counter, 1);
+      GItem next = load_item(items, w, nitems);
+      while (ok) {
+        const GItem it = next;
+        const bool end = w >= nitems;
+        if (!end) {
+          w = (unsigned)atomicAdd(counter, 1);
+          next = load_item(items, w, nitems);
+        }
+        if (!end && !it.nd) continue;
+        if (!wait_bar(&wempty[rw.slot], rw.phase ^ 1, abort_flag, wait_ns)) {
+          fail(1);
+          break;
+        }
+        work[rw.slot] = it;  // nd = 0: no more items
+        mftc::mbar_arrive(&wfull[rw.slot]);
+        rw.advance();
+        if (end) break;
+        const CUtensorMap *ma = &maps[2 * it.p], *mb = ma + 1;
+        const uint32_t b_bytes = (uint32_t)(it.bn * BK);
+        for (int kb = it.kb0; kb < it.kb1 && ok; ++kb) {
+          int t = it.g;  // next slice of B
+          for (int s = 0; s <= it.g && ok; ++s) {
+            if (!wait_bar(&emptyA[ra.slot], ra.phase ^ 1, abort_flag, wait_ns)) {
+              fail(1);
+              ok = false;
+              break;
+            }
+            mftc::mbar_arrive_expect_tx(&fullA[ra.slot], GD_TILE_A);
+            mftc::tma_load_3d(sA + ra.slot * GD_TILE_A, ma, &fullA[ra.slot], kb * BK, it.a_row, s);
+            armA.arm(ra.slot, ra.phase);
+            ra.advance();
+            for (; t >= 0 && t > it.g - s - it.nd; --t) {  // up to what step s multiplies
+              if (!wait_bar(&emptyB[rb.slot], rb.phase ^ 1, abort_flag, wait_ns)) {
+                fail(1);
+                ok = false;
+                break;
+              }
+              mftc::mbar_arrive_expect_tx(&fullB[rb.slot], b_bytes);
+              mftc::tma_load_3d(sB + rb.slot * GD_TILE_B, mb, &fullB[rb.slot], kb * BK, it.b_row, t);
+              armB.arm(rb.slot, rb.phase);
+              rb.advance();
+            }
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {  // ---- MMA issuer
+      const uint64_t descA = mftc::smem_desc_k_sw128(mftc::smem_u32(sA));
+      const uint64_t descB = mftc::smem_desc_k_sw128(mftc::smem_u32(sB));
+      RingPos<GD_NA> ra;
+      RingPos<GD_NB> rb;
+      uint32_t acc_phase = 0;  // bit d: parity of tempty[d]
+      bool ok = true;
+      RingPos<GD_NW> rw;
+      while (ok) {
+        if (!wait_bar(&wfull[rw.slot], rw.phase, abort_flag, wait_ns)) {
+          fail(4);
+          break;
+        }
+        const int g = work[rw.slot].g, it_nd = work[rw.slot].nd, kb0 = work[rw.slot].kb0, kb1 = work[rw.slot].kb1,
+                  bn = work[rw.slot].bn;
+        mftc::mbar_arrive(&wempty[rw.slot]);
+        rw.advance();
+        if (!it_nd) break;
+        const uint32_t idesc = mftc::idesc_i8(BM, bn);
+        uint32_t accumulate = 0;
+        for (int kb = kb0; kb < kb1 && ok; ++kb) {
+          int landed = 0;  // B tiles from rb on known to have landed
+          for (int s = 0; s <= g; ++s) {
+            const int nd = min(it_nd, g - s + 1);
+            ok = wait_bar(&fullA[ra.slot], ra.phase, abort_flag, wait_ns);
+            for (; ok && landed < nd; ++landed)
+              ok = wait_bar(&fullB[rb.at(landed)], rb.phase_at(landed), abort_flag, wait_ns);
+            if (!ok) {
+              fail(4);
+              break;
+            }
+            mftc::tc_fence_after();
+            const uint64_t ad = descA + (uint64_t)(ra.slot * (GD_TILE_A / 16));
+#pragma unroll
+            for (int d = 0; d < GD_DIAGS; ++d) {
+              if (d >= nd) break;
+              if (!accumulate) {  // first step: the previous item's drain handed this accumulator back
+                if (!wait_bar(&tempty[d], ((acc_phase >> d) & 1u) ^ 1u, abort_flag, wait_ns)) {
+                  fail(2);
+                  ok = false;
+                  break;
+                }
+                acc_phase ^= 1u << d;
+                mftc::tc_fence_after();
+              }
+              const uint64_t bd = descB + (uint64_t)(rb.at(d) * (GD_TILE_B / 16));
+              const uint32_t acc = tmem_base + (uint32_t)(d * GD_BN);
+#pragma unroll
+              for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                mftc::umma_i8(acc, ad + (uint64_t)(kk * UMMA_K / 16), bd + (uint64_t)(kk * UMMA_K / 16), idesc,
+                              kk == 0 ? accumulate : 1u);
+            }
+            if (!ok) break;
+            accumulate = 1;
+            mftc::umma_commit(&emptyA[ra.slot]);
+            mftc::umma_commit(&emptyB[rb.slot]);
+            ra.advance();
+            rb.advance();
+            --landed;
+          }
+        }
+        if (!ok) break;
+        mftc::umma_commit(tfull);
+      }
+      mftc::umma_commit(drain);
+      uint64_t t0 = globaltimer();
+      while (!mftc::mbar_try_wait(drain, 0) && globaltimer() - t0 < WAIT_NS) {
+      }
+    }
+  } else {  // ---- epilogue
+    const int quad = warp & 3;        // TMEM lanes this warp may read
+    const int half = (warp - 2) / 4;  // which half of an accumulator's columns
+    const int row = quad * 32 + lane;
+    uint32_t item_phase = 0;
+    RingPos<GD_NW> rw;
+    while (true) {
+      bool got = wait_bar(&wfull[rw.slot], rw.phase, abort_flag, wait_ns);
+      if (!__all_sync(0xffffffffu, got)) {
+        if (lane == 0) fail(8);
+        break;
+      }
+      int32_t *const it_dst = work[rw.slot].dst;
+      const int64_t gstride = work[rw.slot].gstride;
+      const int nd = work[rw.slot].nd, bn = work[rw.slot].bn, M_pad = work[rw.slot].M_pad;
+      __syncwarp();
+      if (lane == 0) mftc::mbar_arrive(&wempty[rw.slot]);
+      rw.advance();
+      if (!nd) break;
+      got = wait_bar(tfull, item_phase, abort_flag, wait_ns);
+      if (!__all_sync(0xffffffffu, got)) {
+        if (lane == 0) fail(8);
+        break;
+      }
+      item_phase ^= 1;
+      mftc::tc_fence_after();
+      const int nch = bn / 64, ch0 = half * nch;  // this warp's 32-column chunks
+      for (int d = 0; d < nd; ++d) {
+        int32_t *dst = it_dst - d * gstride + (int64_t)ch0 * 32 * M_pad + row;
+        for (int chunk = ch0; chunk < ch0 + nch; ++chunk) {
+          uint32_t r[32];
+          mftc::tmem_ld_32x32b_x32(
+              tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(d * GD_BN + chunk * 32), r);
+          mftc::tmem_wait_ld();
+#pragma unroll
+          for (int q = 0; q < 32; ++q) {
+            __stcs(dst, (int32_t)r[q]);  // evict-first: keep L2 for the slices
+            dst += M_pad;
+          }
+        }
+        mftc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mftc::mbar_arrive(&tempty[d]);
+      }
+    }
+  }
+  mftc::tc_fence_before();
+  __syncthreads();
+  mftc::tc_fence_after();
+  if (*abort_flag) {  // read after the barrier: the same value in every thread
+    // copies in flight that no MMA consumed land before shared memory is released
+    if (warp == 0 && lane == 0) {
+      armA.drain(fullA, GD_NA);
+      armB.drain(fullB, GD_NB);
+    }
     __syncthreads();
   }
   if (warp == 1) {
@@ -807,13 +1106,14 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
   std::vector<SProb> probs(np);
   Arena ar;
   size_t o_probs = ar.take(sizeof(SProb) * std::max(np, 1));
-  size_t o_prefix = ar.take(sizeof(int64_t) * PH_COUNT * std::max(np, 1));
+  size_t o_prefix = ar.take(sizeof(int64_t) * std::max(np, 1));
   size_t o_maps = ar.take(sizeof(CUtensorMap) * 2 * std::max(np, 1), 128);
-  size_t o_status = ar.take(sizeof(int));
+  size_t o_status = ar.take(2 * sizeof(int));  // abort codes, the digit kernel's item counter
   std::vector<size_t> o_plan(np, 0), o_cc(np, 0), o_as(np, 0), o_bs(np, 0), o_d(np);
   std::vector<int64_t> rowA(np, -1), rowB(np, -1);  // statistics rows of owned operands
   int64_t rows_total = 0;
-  std::vector<int64_t> prefix(PH_COUNT * (size_t)std::max(np, 1), 0);
+  std::vector<int64_t> prefix((size_t)std::max(np, 1), 0);  // of the items
+  std::vector<Owner> owner[PH_ITEMS];                         // of the blocks of the other phases
   int64_t total[PH_COUNT] = {0, 0, 0, 0, 0, 0, 0};
   for (int q = 0; q < np; ++q) {
     const Spec &g = sp[q];
@@ -867,14 +1167,18 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
         P.own_b ? (P.N_pad * (P.K_pad / 8) + 255) / 256 : 0,
         P.mode == 0 ? comb : 0,
         P.mode != 0 ? comb : 0,
-        (int64_t)P.nsl * P.nkc * P.ntm * P.ntn};
+        (int64_t)g_groups(P.nsl, crt) * P.nkc * P.ntm * P.ntn};
+    prefix[q] = total[PH_ITEMS];
     for (int ph = 0; ph < PH_COUNT; ++ph) {
-      prefix[(size_t)ph * np + q] = total[ph];
       total[ph] += blocks[ph];
+      if (total[ph] > INT32_MAX) return MFCUDA_ERR_UNSUPPORTED;
+      if (ph != PH_ITEMS)
+        for (int64_t l = 0; l < blocks[ph]; ++l) owner[ph].push_back({q, (int)l});
     }
   }
-  for (int ph = 0; ph < PH_COUNT; ++ph)
-    if (total[ph] > INT32_MAX) return MFCUDA_ERR_UNSUPPORTED;
+  size_t o_owner[PH_ITEMS];
+  for (int ph = 0; ph < PH_ITEMS; ++ph) o_owner[ph] = ar.take(sizeof(Owner) * std::max<int64_t>(total[ph], 1));
+  const size_t o_items = ar.take(sizeof(GItem) * std::max<int64_t>(total[PH_ITEMS], 1));
   // exponent statistics of all owned operands in three contiguous arrays
   const size_t o_sig = ar.take(sizeof(int) * std::max<int64_t>(rows_total, 1));
   const size_t o_mu = ar.take(sizeof(int) * std::max<int64_t>(rows_total, 1));
@@ -951,18 +1255,28 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
   }
   SProb *dp = reinterpret_cast<SProb *>(base + o_probs);
   int64_t *dprefix = reinterpret_cast<int64_t *>(base + o_prefix);
+  Owner *downer[PH_ITEMS];
+  bool copied = true;
+  for (int ph = 0; ph < PH_ITEMS; ++ph) {
+    downer[ph] = reinterpret_cast<Owner *>(base + o_owner[ph]);
+    if (!owner[ph].empty() && cudaMemcpy(downer[ph], owner[ph].data(), sizeof(Owner) * owner[ph].size(),
+                                         cudaMemcpyHostToDevice) != cudaSuccess)
+      copied = false;
+  }
   CUtensorMap *dmaps = reinterpret_cast<CUtensorMap *>(base + o_maps);
+  GItem *ditems = reinterpret_cast<GItem *>(base + o_items);
   b->status = reinterpret_cast<int *>(base + o_status);
   if (np > 0 && (cudaMemcpy(dp, probs.data(), sizeof(SProb) * np, cudaMemcpyHostToDevice) != cudaSuccess ||
-                 cudaMemcpy(dprefix, prefix.data(), sizeof(int64_t) * PH_COUNT * np, cudaMemcpyHostToDevice) !=
-                     cudaSuccess ||
+                 cudaMemcpy(dprefix, prefix.data(), sizeof(int64_t) * np, cudaMemcpyHostToDevice) != cudaSuccess ||
+                 !copied ||
                  cudaMemcpy(dmaps, maps.data(), sizeof(CUtensorMap) * 2 * np, cudaMemcpyHostToDevice) !=
                      cudaSuccess)) {
     destroy(b);
     return MFCUDA_ERR_CUDA;
   }
   std::call_once(g_gmma_attr, [] {
-    cudaFuncSetAttribute(g_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+    cudaFuncSetAttribute(g_crt_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, MMA_SMEM);
+    cudaFuncSetAttribute(g_digit_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, GD_SMEM);
     cudaFuncSetAttribute(g_crt_combine, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          crt_tc_smem((CRT_NMAX + 31) / 32));
   });
@@ -973,32 +1287,36 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
   if (mma_grid > total[PH_ITEMS]) mma_grid = (int)std::max<int64_t>(total[PH_ITEMS], 1);
   const uint64_t wait_ns = wait_limit_ns();  // captured into the graph with the plan
   int rc = capture(b, [&](cudaStream_t cs) {
-    cudaMemsetAsync(b->status, 0, sizeof(int), cs);
+    cudaMemsetAsync(b->status, 0, 2 * sizeof(int), cs);
     if (np == 0) return;
     const unsigned fb = (unsigned)((rows_total + 255) / 256);
     fill_kernel<<<fb, 256, 0, cs>>>(sig0, rows_total, SENT_LO);
     fill_kernel<<<fb, 256, 0, cs>>>(mu0, rows_total, SENT_HI);
     fill_kernel<<<fb, 256, 0, cs>>>(flag0, rows_total, 0);
-    if (total[PH_SCAN_A]) g_scan_a<<<(unsigned)total[PH_SCAN_A], 256, 0, cs>>>(dp, dprefix + PH_SCAN_A * np, np);
-    if (total[PH_SCAN_B]) g_scan_b<<<(unsigned)total[PH_SCAN_B], 256, 0, cs>>>(dp, dprefix + PH_SCAN_B * np, np);
+    if (total[PH_SCAN_A]) g_scan_a<<<(unsigned)total[PH_SCAN_A], 256, 0, cs>>>(dp, downer[PH_SCAN_A]);
+    if (total[PH_SCAN_B]) g_scan_b<<<(unsigned)total[PH_SCAN_B], 256, 0, cs>>>(dp, downer[PH_SCAN_B]);
     g_plan<<<np, 256, 0, cs>>>(dp, slices, target);
     if (total[PH_SLICE_A] && crt)
-      g_crt_slice_a<<<(unsigned)total[PH_SLICE_A], 256, 0, cs>>>(dp, dprefix + PH_SLICE_A * np, np);
+      g_crt_slice_a<<<(unsigned)total[PH_SLICE_A], 256, 0, cs>>>(dp, downer[PH_SLICE_A]);
     else if (total[PH_SLICE_A])
-      g_slice_a<<<(unsigned)total[PH_SLICE_A], 256, 0, cs>>>(dp, dprefix + PH_SLICE_A * np, np);
+      g_slice_a<<<(unsigned)total[PH_SLICE_A], 256, 0, cs>>>(dp, downer[PH_SLICE_A]);
     if (total[PH_SLICE_B] && crt)
-      g_crt_slice_b<<<(unsigned)total[PH_SLICE_B], 256, 0, cs>>>(dp, dprefix + PH_SLICE_B * np, np);
+      g_crt_slice_b<<<(unsigned)total[PH_SLICE_B], 256, 0, cs>>>(dp, downer[PH_SLICE_B]);
     else if (total[PH_SLICE_B])
-      g_slice_b<<<(unsigned)total[PH_SLICE_B], 256, 0, cs>>>(dp, dprefix + PH_SLICE_B * np, np);
-    g_mma<<<mma_grid, G_THREADS, MMA_SMEM, cs>>>(dp, dmaps, dprefix + PH_ITEMS * np, np, total[PH_ITEMS],
-                                                   b->status, wait_ns);
+      g_slice_b<<<(unsigned)total[PH_SLICE_B], 256, 0, cs>>>(dp, downer[PH_SLICE_B]);
+    g_items<<<np, 128, 0, cs>>>(dp, dprefix, ditems);
+    if (crt)
+      g_crt_mma<<<mma_grid, G_THREADS, MMA_SMEM, cs>>>(ditems, total[PH_ITEMS], dmaps, b->status, wait_ns);
+    else
+      g_digit_mma<<<mma_grid, G_THREADS, GD_SMEM, cs>>>(ditems, total[PH_ITEMS], b->status + 1, dmaps, b->status,
+                                                        wait_ns);
     for (int ph : {PH_COMBINE, PH_COMBINE2}) {
       if (!total[ph]) continue;
       if (crt)
         g_crt_combine<<<(unsigned)total[ph], CTC_THREADS, crt_tc_smem((nsl_max + 31) / 32), cs>>>(
-            dp, dprefix + ph * np, np, b->status, wait_ns);
+            dp, downer[ph], b->status, wait_ns);
       else
-        g_combine<<<(unsigned)total[ph], kCombineThreads, 0, cs>>>(dp, dprefix + ph * np, np);
+        g_combine<<<(unsigned)total[ph], kCombineThreads, 0, cs>>>(dp, downer[ph]);
     }
   });
   if (rc != MFCUDA_OK) {
