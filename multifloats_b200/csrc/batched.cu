@@ -239,17 +239,17 @@ __global__ void __launch_bounds__(256) g_slice_a(const SProb *probs, const Owner
   const Owner own = owner[blockIdx.x];
   const SProb &P = probs[own.p];
   const int64_t l = own.local;
-  const int64_t nbx = P.M_pad / 32;
+  const int64_t nbx = (P.m + 31) / 32;
   slice_a_body(P.A, P.m, P.k, P.astride, P.M_pad, P.K_pad, P.sigA, P.flagA, P.plan, P.As, l % nbx, l / nbx);
 }
 // CRT form: residues instead of digits, in MN-major planes As[t][p][i] (the
 // rows of one K index contiguous); flat: thread t of the problem takes K
-// index t / (M_pad / 8), rows 8 (t % (M_pad / 8)) .. + 7
+// index t / ceil(m / 8), rows 8 (t % ceil(m / 8)) .. + 7
 __global__ void __launch_bounds__(256) g_crt_slice_a(const SProb *probs, const Owner *owner) {
   const Owner own = owner[blockIdx.x];
   const SProb &P = probs[own.p];
   const int64_t t = (int64_t)own.local * 256 + threadIdx.x;
-  const int64_t per_k = P.M_pad / 8;
+  const int64_t per_k = (P.m + 7) / 8;
   const int64_t kp = t / per_k;
   if (kp < P.K_pad)
     crt_slice_a_mn_one(P.A, P.m, P.k, P.astride, P.M_pad, P.K_pad, P.sigA, P.flagA, P.plan, P.As,
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(256) g_crt_slice_b(const SProb *probs, const O
   const int64_t t = (int64_t)own.local * 256 + threadIdx.x;
   const int64_t per_col = P.K_pad / 8;
   const int64_t j = t / per_col;
-  if (j < P.N_pad)
+  if (j < P.n)
     crt_slice_b_one(P.B, P.k, P.n, P.bstride, P.N_pad, P.K_pad, P.sigB, P.flagB, P.plan, P.Bs, j, (t % per_col) * 8);
 }
 // flat: thread t of the problem takes column t / (K_pad / 8), entries 8 (t % (K_pad / 8)) .. + 7
@@ -271,16 +271,16 @@ __global__ void __launch_bounds__(256) g_slice_b(const SProb *probs, const Owner
   const int64_t t = (int64_t)own.local * 256 + threadIdx.x;
   const int64_t per_col = P.K_pad / 8;
   const int64_t j = t / per_col;
-  if (j < P.N_pad)
+  if (j < P.n)
     slice_b_one(P.B, P.k, P.n, P.bstride, P.N_pad, P.K_pad, P.sigB, P.flagB, P.plan, P.Bs, j, (t % per_col) * 8);
 }
 // flat: thread t of the problem owns rows 4 (t % q) .. + 3 of column t / q,
 // q = ceil(m / 4) (combine4_body)
-constexpr int kCombineThreads = 128;
+constexpr int kCombineThreads = COMBINE_THREADS;
 static int64_t combine_blocks(int64_t m, int64_t n) {
   return (((m + 3) / 4) * n + kCombineThreads - 1) / kCombineThreads;
 }
-__global__ void __launch_bounds__(kCombineThreads) g_combine(const SProb *probs, const Owner *owner) {
+__global__ void __launch_bounds__(kCombineThreads, COMBINE_BLOCKS) g_combine(const SProb *probs, const Owner *owner) {
   const Owner own = owner[blockIdx.x];
   const SProb &P = probs[own.p];
   const int64_t t = (int64_t)own.local * kCombineThreads + threadIdx.x;
@@ -1163,8 +1163,8 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
     const int64_t blocks[PH_COUNT] = {
         P.own_a ? ((P.m + 255) / 256) * ((P.k + 63) / 64) : 0,
         P.own_b && P.k > 0 ? (P.n + 7) / 8 : 0,
-        P.own_a ? (crt ? (P.K_pad * (P.M_pad / 8) + 255) / 256 : (P.M_pad / 32) * (P.K_pad / 64)) : 0,
-        P.own_b ? (P.N_pad * (P.K_pad / 8) + 255) / 256 : 0,
+        P.own_a ? (crt ? (P.K_pad * ((P.m + 7) / 8) + 255) / 256 : ((P.m + 31) / 32) * (P.K_pad / 64)) : 0,
+        P.own_b ? (P.n * (P.K_pad / 8) + 255) / 256 : 0,
         P.mode == 0 ? comb : 0,
         P.mode != 0 ? comb : 0,
         (int64_t)g_groups(P.nsl, crt) * P.nkc * P.ntm * P.ntn};

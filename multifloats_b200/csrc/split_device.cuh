@@ -351,7 +351,7 @@ __device__ __forceinline__ void slice_a_body(const double *__restrict__ A, int64
                                                       const Plan *plan, int8_t *__restrict__ As, int64_t bx, int64_t by) {
   __shared__ __align__(16) uint8_t tile[SMAX][SA_ROWS * SA_STRIDE];
   const int S = plan->S, W = plan->W;
-  const int64_t i0 = bx * SA_ROWS, p0 = by * SA_COLS;
+  const int64_t i0 = bx * SA_ROWS, p0 = by * SA_COLS;  // rows past M are padding no output depends on
   const int t = threadIdx.x;
   const int ii = t % SA_ROWS, grp = t / SA_ROWS;
   const int64_t i = i0 + ii;
@@ -383,7 +383,7 @@ __device__ __forceinline__ void slice_a_body(const double *__restrict__ A, int64
 // B (k x n column-major) -> Bs[s][j][p]: each thread rounds and slices 8
 // consecutive entries of one column (128 contiguous bytes in, one 8-byte word
 // per slice out).
-// Entries p8 .. p8+7 of column j (0 <= j < N_pad, p8 a multiple of 8 below K_pad).
+// Entries p8 .. p8+7 of column j (0 <= j < N, p8 a multiple of 8 below K_pad).
 __device__ __forceinline__ void slice_b_one(const double *__restrict__ B, int64_t K, int64_t N,
                                             int64_t stride, int64_t N_pad, int64_t K_pad, const int *sig,
                                             const int *flag, const Plan *plan, int8_t *__restrict__ Bs,
@@ -419,78 +419,20 @@ __device__ __forceinline__ void scan_b_warp(const double *__restrict__ B, int64_
   }
 }
 
-// Thread per row i (consecutive threads -> consecutive rows: every load and
-// store is coalesced); the grid's y dimension strides over the columns.  The
+// C_ij = 2^(sigma_i + tau_j - 12) sum_kc sum_g D_g,kc 2^(-8g), summed in DD
+// chunk by chunk, each from the smallest diagonal up, then scaled exactly.  The
 // output is a strided view (C element (i,j) at double2 index (jM + i) cstride)
 // and `mode` stores the product P (0), or replaces C by the DD difference
 // C - P (1) or sum C + P (2), which assembles complex products.
-__device__ __forceinline__ void combine_body(const int32_t *__restrict__ D, const Plan *plan,
-                                                      const int *sigA, const int *flagA,
-                                                      const int *sigB, const int *flagB, int64_t M,
-                                                      int64_t N, int64_t M_pad, int64_t N_pad,
-                                                      int nkc, double *__restrict__ C, int64_t cstride,
-                                                      int mode, int64_t bx, int64_t by, int64_t ny) {
-  const int G = plan->G;
-  const int64_t i = bx * blockDim.x + threadIdx.x;
-  if (i >= M) return;
-  const int64_t gstride = (int64_t)nkc * N_pad * M_pad;  // distance between diagonals
-  const int sa = sigA[i], fa = flagA[i];
-  // two columns per pass: 2 x (G+1) independent loads in flight per thread
-  for (int64_t j0 = by; j0 < N; j0 += 2 * ny) {
-    const int64_t jj[2] = {j0, j0 + ny};
-    double hi[2] = {0.0, 0.0}, lo[2] = {0.0, 0.0};
-    for (int kc = 0; kc < nkc; ++kc) {
-      int32_t v[2][SMAX];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const int32_t *src = D + ((int64_t)kc * N_pad + (jj[c] < N ? jj[c] : j0)) * M_pad + i;
-#pragma unroll
-        for (int g = 0; g < SMAX; ++g) v[c][g] = g <= G ? __ldcs(src + g * gstride) : 0;
-      }
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int g = SMAX - 1; g >= 0; --g) {
-          if (g <= G) {
-            double tv = mfdev::mul((double)v[c][g], pow2(-8 * g));  // exact
-            double s_, err;
-            mfdev::two_sum(hi[c], tv, s_, err);
-            hi[c] = s_;
-            lo[c] = mfdev::add(lo[c], err);
-          }
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int64_t j = jj[c];
-      if (j >= N) break;
-      double h, l;
-      mfdev::two_sum(hi[c], lo[c], h, l);
-      double2 out;
-      if (fa | flagB[j]) {
-        out = make_double2(CUDART_NAN, 0.0);
-      } else {
-        int ex = sa + sigB[j] - 12;
-        out = make_double2(scale2(h, ex), scale2(l, ex));
-      }
-      double2 *dst = reinterpret_cast<double2 *>(C) + (j * M + i) * cstride;
-      if (mode != 0) {
-        double2 prev = *dst;
-        mfdev::dd p = mfdev::make(out.x, out.y), q = mfdev::make(prev.x, prev.y);
-        mfdev::dd r = mode == 1 ? mfdev::dd_sub(q, p) : mfdev::dd_add(q, p);
-        out = make_double2(r.hi, r.lo);
-      }
-      __stcs(dst, out);
-    }
-  }
-}
-
-// Same result as combine_body, element for element (same operations in the
-// same order), with a thread per 4 consecutive rows of one column: each
-// diagonal is one 16-byte load per thread (512 contiguous bytes per warp), all
-// G+1 of them in flight before the DD accumulation.  Requires M_pad % 4 == 0
-// and a 16-byte aligned D.  Thread (q = blockIdx.x * blockDim.x + t) owns rows
-// 4q..4q+3 of column j = column index given by the caller.
+//
+// A thread owns rows 4 quad .. + 3 of column j: each diagonal is one 16-byte
+// load per thread (512 contiguous bytes per warp).  Requires M_pad % 4 == 0 and
+// a 16-byte aligned D.  The bound is HBM (14 INT32 in, 16 bytes out), but a
+// block is little more than its loads' latency, so warps matter more than
+// loads per thread: seven diagonals at a time leave room for six blocks per
+// SM where all fourteen left four (2000 products 2.36 -> 1.70 ms; eight spill: 1.89).
+constexpr int COMBINE_THREADS = 128, COMBINE_BLOCKS = 6, COMBINE_LOADS = 7;
+static_assert(SMAX % COMBINE_LOADS == 0, "whole groups of diagonals");
 __device__ __forceinline__ void combine4_body(const int32_t *__restrict__ D, const Plan *plan,
                                               const int *sigA, const int *flagA, const int *sigB,
                                               const int *flagB, int64_t M, int64_t N, int64_t M_pad,
@@ -504,21 +446,27 @@ __device__ __forceinline__ void combine4_body(const int32_t *__restrict__ D, con
   for (int kc = 0; kc < nkc; ++kc) {
     const int4 *src = reinterpret_cast<const int4 *>(D + ((int64_t)kc * N_pad + j) * M_pad + i0);
     const int64_t gs4 = gstride / 4;
-    int4 v[SMAX];
 #pragma unroll
-    for (int g = 0; g < SMAX; ++g) v[g] = g <= G ? __ldcs(src + g * gs4) : make_int4(0, 0, 0, 0);
+    for (int top = SMAX - 1; top >= 0; top -= COMBINE_LOADS) {
+      if (top - COMBINE_LOADS + 1 > G) continue;
+      int4 v[COMBINE_LOADS];
 #pragma unroll
-    for (int g = SMAX - 1; g >= 0; --g) {
-      if (g <= G) {
-        const double sc = pow2(-8 * g);
-        const int d[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
+      for (int u = 0; u < COMBINE_LOADS; ++u)
+        v[u] = top - u <= G ? __ldcs(src + (top - u) * gs4) : make_int4(0, 0, 0, 0);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          double tv = mfdev::mul((double)d[r], sc);  // exact
-          double s_, err;
-          mfdev::two_sum(hi[r], tv, s_, err);
-          hi[r] = s_;
-          lo[r] = mfdev::add(lo[r], err);
+      for (int u = 0; u < COMBINE_LOADS; ++u) {
+        const int g = top - u;
+        if (g <= G) {
+          const double sc = pow2(-8 * g);
+          const int d[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            double tv = mfdev::mul((double)d[r], sc);  // exact
+            double s_, err;
+            mfdev::two_sum(hi[r], tv, s_, err);
+            hi[r] = s_;
+            lo[r] = mfdev::add(lo[r], err);
+          }
         }
       }
     }

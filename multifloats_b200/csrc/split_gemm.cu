@@ -163,11 +163,11 @@ __global__ void __launch_bounds__(256) slice_kernel(const __grid_constant__ Oper
   const unsigned l = blockIdx.x - op.first;
   if (op.b_side) {
     const unsigned per_col = (unsigned)(ops.k_pad / 8), t = l * 256 + threadIdx.x, j = t / per_col;
-    if (j < op.rows_pad)
+    if (j < op.rows)
       slice_b_one(op.p, ops.k, op.rows, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, plan, op.slices, j,
                   (int64_t)(t % per_col) * 8);
   } else {
-    const unsigned nbx = (unsigned)(op.rows_pad / 32);
+    const unsigned nbx = (unsigned)((op.rows + 31) / 32);
     slice_a_body(op.p, op.rows, ops.k, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, plan, op.slices, l % nbx,
                  l / nbx);
   }
@@ -847,7 +847,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 // ---------------------------------------------------------------------------
 // 5. combine
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) combine_kernel(const int32_t *__restrict__ D, const Plan *plan,
+__global__ void __launch_bounds__(COMBINE_THREADS, COMBINE_BLOCKS) combine_kernel(const int32_t *__restrict__ D, const Plan *plan,
                                                       const int *sigA, const int *flagA, const int *sigB,
                                                       const int *flagB, int64_t M, int64_t N,
                                                       int64_t M_pad, int64_t N_pad, int nkc,
@@ -855,12 +855,12 @@ __global__ void __launch_bounds__(128) combine_kernel(const int32_t *__restrict_
   combine4_body(D, plan, sigA, flagA, sigB, flagB, M, N, M_pad, N_pad, nkc, C, cstride, mode,
                 (int64_t)blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
 }
-constexpr int COMBINE_THREADS = 128;
 
 // ---------------------------------------------------------------------------
 // CRT form (crt_device.cuh): plan, residue slicing, reconstruction
 // ---------------------------------------------------------------------------
-// Residues, flat over each operand's padded entries: a thread per 8
+// Residues, flat over each operand's entries (K padded with zeros; rows and
+// columns past the operand are padding no output depends on): a thread per 8
 // consecutive rows of a K index (A, MN-major planes) or per 8 consecutive K
 // indices of a column (B: columns j0 .. of it).
 __global__ void __launch_bounds__(256) crt_slice_kernel(const __grid_constant__ Operands ops, const Plan *plan,
@@ -869,11 +869,11 @@ __global__ void __launch_bounds__(256) crt_slice_kernel(const __grid_constant__ 
   const unsigned t = (blockIdx.x - op.first) * 256 + threadIdx.x;
   if (op.b_side) {
     const unsigned per_col = (unsigned)(ops.k_pad / 8), j = j0 + t / per_col;
-    if (j < j1)
+    if (j < j1 && j < op.rows)
       crt_slice_b_one(op.p, ops.k, op.rows, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, plan, op.slices, j,
                       (int64_t)(t % per_col) * 8);
   } else {
-    const unsigned per_k = (unsigned)(op.rows_pad / 8), kp = t / per_k;
+    const unsigned per_k = (unsigned)((op.rows + 7) / 8), kp = t / per_k;
     if (kp < ops.k_pad)
       crt_slice_a_mn_one(op.p, op.rows, ops.k, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, plan, op.slices,
                          (int64_t)(t % per_k) * 8, kp);
@@ -1270,14 +1270,14 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
     const int ntn_all = (int)(L.N_pad / tn_cols);
     const int npan = (sink && crt && L.pair) ? std::max(1, std::min(sink->panels, ntn_all)) : 1;
     auto slice_blocks = [&](const Operand &op) {  // flat: a thread per 8 entries
-      return (op.rows_pad * (L.K_pad / 8) + 255) / 256;
+      return (op.b_side ? op.rows * (L.K_pad / 8) : (op.rows + 7) / 8 * L.K_pad) / 256 + 1;
     };
     if (crt) {  // with column panels B's residues follow panel by panel
       const unsigned blocks = lay_out(0, npan > 1 ? nA : nops, slice_blocks);
       crt_slice_kernel<<<blocks, 256, 0, s>>>(ops, plan, 0, (unsigned)L.N_pad);
     } else {
       const unsigned blocks = lay_out(0, nops, [&](const Operand &op) {
-        return op.b_side ? slice_blocks(op) : (op.rows_pad / 32) * (L.K_pad / 64);
+        return op.b_side ? slice_blocks(op) : (op.rows + 31) / 32 * (L.K_pad / 64);
       });
       slice_kernel<<<blocks, 256, 0, s>>>(ops, plan);
     }
