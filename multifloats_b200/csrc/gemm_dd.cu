@@ -18,8 +18,6 @@
 // (16-byte copies, zero-filled past the matrix edge) in a two-stage ring.
 // Bound: FP64 pipe, 13 FP64 instructions per MAC plus 6 per renormalisation.
 // Which tiles a product is cut into is decided by pick_tiles.
-#include <mutex>
-
 #include "common.cuh"
 #include "dd_device.cuh"
 #include "gemm_tile.cuh"
@@ -172,9 +170,9 @@ __global__ void __launch_bounds__(kThreads, 4)
 // p = 0..k-1, so there is one dependency chain per output and only a few
 // thousand of them; a CTA owns 32 outputs and splits each MAC
 // (matmul.inc:6-19) in two:
-//   * eight producer warps stream the matrix through an S-stage cp.async ring
-//     (a stage is 32 outputs x 32 k, four columns of it per warp) and compute
-//     the accumulator-independent part of every MAC, p = ah*bh and
+//   * eight producer warps stream the matrix (a stage is 32 outputs x 32 k, four
+//     columns of it per warp, P stages ahead in registers) and compute the
+//     accumulator-independent part of every MAC, p = ah*bh and
 //     q = fma(ah,bh,-p) + fma(ah,bl,al*bh), into a double-buffered array;
 //   * one warp runs the accumulator chain (two_sum of s_hi with p, then
 //     s_lo += q + (aerr + berr)) and the renorm cadence, lane = output.
@@ -182,29 +180,27 @@ __global__ void __launch_bounds__(kThreads, 4)
 // are bit-identical; the warps hand over through one named barrier per stage.
 //
 // Bound: the chain, 15 dependent additions of 8 cycles per eight steps and 62
-// FP64 instructions; as compiled it takes 32 cycles a step, where HBM at one
+// FP64 instructions; as compiled it takes 28-32 cycles a step, where HBM at one
 // CTA per SM would take 19.  So the chain warp has a scheduler to itself (the
 // producers use the other three; the roles rotate with the wave of CTAs, so
-// that the chains of the CTAs of one SM land on different schedulers) and, in
-// the default cadence, no test between its steps.  S = 8 stages (one CTA per
-// SM) when the outputs are one wave, 4 (two CTAs) otherwise.
-// 4099 x 3001: 143 -> 62 us (y = A x), 143 -> 60 (y = x A); 16384 x 8192: 908 ->
-// 445, 862 -> 402 (HBM alone 328).
+// that the chains of the CTAs of one SM land on different schedulers), no
+// test between its steps in the default cadence, and the shared memory nearly
+// to itself: with the matrix staged there too, its traffic cost the chain a
+// quarter of its time.  The matrix reaches the registers through L2, where each
+// producer prefetches its columns eight stages ahead (none: a third slower; 24
+// ahead of 16384 rows: likewise).  P = 4 stages (one CTA per SM) when the outputs are one wave, 2 (two
+// CTAs) otherwise.
+// Inputs not in L2: 4099 x 3001 144 -> 49 us (y = A x), 142 -> 48 (y = x A); 200
+// x 6000 278 -> 85; 16384 x 8192 904 -> 353, 866 -> 351 (HBM alone 328).
 // ---------------------------------------------------------------------------
 constexpr int kGvN = 32, kGvK = 32;
 constexpr int kGvWarps = 12, kGvThreads = 32 * kGvWarps;  // chain, eight producers, three without work
 constexpr int kGvProd = 8, kGvActive = 32 * (1 + kGvProd);
-// Row of the term array: the producers of y = x B write it transposed.
-__host__ __device__ constexpr int gv_pitch(bool vm) { return vm ? 33 : 32; }
-// Where the vector's entries of a stage come from: with S = 8 the first
-// producer copies them into the ring for all (one stage of the prefetch is then
-// spent on the hand-over); with S = 4 that stage is worth more than the ring, and
-// every producer loads its own a stage ahead (4800 x 3000: 108 -> 84 us; with
-// S = 8, 4099 x 3001: 75 instead of 62).
-__host__ __device__ constexpr bool gv_x_ring(int stages) { return stages > 4; }
-constexpr size_t gv_smem(bool vm, int stages) {
-  return sizeof(double2) * ((size_t)stages * (kGvN * kGvK + (gv_x_ring(stages) ? kGvK : 0)) + 2 * (size_t)kGvK * gv_pitch(vm));
-}
+// Row of the term array, padded for the producers of y = x B, which write it
+// transposed (and the same for both: the chain's code is then one).
+constexpr int kGvPitch = 33;
+constexpr int kGvAhead = 8;   // stages of the matrix ahead in L2
+constexpr int kGvXStages = 8;  // stages of the vector in flight
 
 template <int N>
 __device__ __forceinline__ void cp_async_wait_n() {
@@ -229,6 +225,21 @@ __device__ __forceinline__ double2 mac_terms(double ah, double al, double bh, do
   return make_double2(p, mfdev::add(e, cross));
 }
 
+// Runs the chain over a whole stage with a renormalisation after every group of
+// eight steps.
+template <int PITCH>
+__device__ __forceinline__ void chain_groups(const double2 *__restrict__ v, double &sh, double &sl) {
+  constexpr int G = gtile::kGroup;
+#pragma unroll
+  for (int g = 0; g < kGvK / G; ++g) {
+    double2 u[G];
+#pragma unroll
+    for (int r = 0; r < G; ++r) u[r] = v[(g * G + r) * PITCH];
+#pragma unroll
+    for (int r = 0; r < G; ++r) mac_chain(u[r].x, u[r].y, sh, sl);
+    mfdev::renorm(sh, sl);
+  }
+}
 // Runs the chain over cmax terms of a stage that starts at step p0 (v: this
 // lane's column of the term array), renorm cadence as in the reference: after
 // each full chunk of ri steps when more remain.
@@ -246,18 +257,6 @@ __device__ __forceinline__ void chain_stage(const double2 *__restrict__ v, int c
   };
   int c = 0;
   if (cad.grouped) {
-    if (cad.ri == G && p0 + kGvK < K) {  // a renormalisation after every group: no tests
-#pragma unroll
-      for (int g = 0; g < kGvK / G; ++g) {
-        double2 u[G];
-#pragma unroll
-        for (int r = 0; r < G; ++r) u[r] = v[(g * G + r) * PITCH];
-#pragma unroll
-        for (int r = 0; r < G; ++r) mac_chain(u[r].x, u[r].y, sh, sl);
-        mfdev::renorm(sh, sl);
-      }
-      return;
-    }
 #pragma unroll 1
     for (; c + G <= cmax; c += G) group(c);
   }
@@ -275,16 +274,14 @@ __device__ __forceinline__ void chain_stage(const double2 *__restrict__ v, int c
 // MAC's first operand); a stage is 32 columns of A, 32 rows (512 contiguous
 // bytes) each.  VM true: y(M) = x(K) A(K,M) (vm_impl, matmul.inc:213-239; x is
 // the MAC's first operand); a stage is 32 columns (outputs), 32 k each.
-template <bool VM, int S, bool ALIGNED>
-__global__ void __launch_bounds__(kGvThreads) gemv_dd_kernel(const double *__restrict__ A,
-                                                             const double *__restrict__ x,
-                                                             double *__restrict__ y, int64_t M,
-                                                             int64_t K, int64_t ri, int sms) {
-  constexpr int PITCH = gv_pitch(VM);
-  extern __shared__ double2 smem_gv[];
-  double2 *ring = smem_gv;                                 // [stage][column][32]
-  double2 *pq = ring + (size_t)S * kGvN * kGvK;            // [2][k][output]
-  double2 *xs = pq + 2 * (size_t)kGvK * PITCH;             // [stage][k] of the vector
+template <bool VM, int P, bool ALIGNED>
+__global__ void __launch_bounds__(kGvThreads, P > 2 ? 1 : 2) gemv_dd_kernel(const double *__restrict__ A,
+                                                                            const double *__restrict__ x,
+                                                                            double *__restrict__ y, int64_t M,
+                                                                            int64_t K, int64_t ri, int sms) {
+  constexpr int PITCH = kGvPitch, S = kGvXStages;
+  __shared__ __align__(16) double2 xs[S * kGvK];           // [stage][k] of the vector
+  __shared__ __align__(16) double2 pq[2 * kGvK * PITCH];   // [2][k][output]
   const int lane = threadIdx.x & 31;
   // role 0: chain; 4 and 8, which share its scheduler, and 11: none; else a producer
   const int rot = (int)(blockIdx.x / (unsigned)sms) & 3;
@@ -297,12 +294,20 @@ __global__ void __launch_bounds__(kGvThreads) gemv_dd_kernel(const double *__res
   if (role == 0) {  // ---- accumulator chain
     double sh = 0.0, sl = 0.0;
     gtile::Cadence cad(ri);
-    if (gv_x_ring(S)) sync();
+    sync();  // the vector's first stage landed
     sync();  // the terms of stage 0 are ready
-    for (int64_t st = 0; st < nst; ++st) {
+    // stages with more steps after them in the default cadence: no tests at all
+    const int64_t plain = cad.ri == gtile::kGroup ? (K - 1) / kGvK : 0;
+    const double2 *v = pq + lane;
+    int64_t st = 0;
+    for (; st < plain; ++st) {
+      chain_groups<PITCH>(v + (st & 1) * kGvK * PITCH, sh, sl);
+      sync();
+    }
+    for (; st < nst; ++st) {
       const int64_t p0 = st * kGvK;
       const int cmax = (K - p0) < kGvK ? (int)(K - p0) : kGvK;
-      chain_stage<PITCH>(pq + (size_t)(st & 1) * kGvK * PITCH + lane, cmax, p0, K, cad, sh, sl);
+      chain_stage<PITCH>(v + (st & 1) * kGvK * PITCH, cmax, p0, K, cad, sh, sl);
       sync();
     }
     const int64_t i = i0 + lane;
@@ -313,85 +318,87 @@ __global__ void __launch_bounds__(kGvThreads) gemv_dd_kernel(const double *__res
     }
     return;
   }
-  // ---- producer w: copies and terms of the columns w, w + 8, w + 16, w + 24
+  // ---- producer w: the columns w, w + 8, w + 16, w + 24 of every stage
   constexpr int COLS = kGvN / kGvProd;
-  constexpr bool XR = gv_x_ring(S);
-  constexpr int PENDING = XR ? S - 3 : S - 2;  // copies that may be in flight when a stage's terms are due
   const int w = role < 4 ? role - 1 : role < 8 ? role - 2 : role - 3;
-  auto issue = [&](int64_t st) {
-    if (st < nst) {
-      double2 *dst = ring + ((size_t)(st % S) * kGvN + w) * 32 + lane;
-      const int64_t p0 = st * kGvK;
-      const double *src = VM ? A + 2 * ((i0 + w) * K + p0 + lane) : A + 2 * ((p0 + w) * M + i0 + lane);
-      const int64_t step = 2 * kGvProd * (VM ? K : M);
-      const bool ok = VM ? p0 + lane < K : i0 + lane < M;
-      const int64_t left = (VM ? M - i0 : K - p0) - w;  // columns from this warp's first one on
+  // (not evict-first: a column of odd length starts inside a 128-byte line, and
+  // the CTA that shares it comes a little later -- 4099 x 3001 64 instead of 49 us)
+  auto load = [&](int64_t st, double2 (&a)[COLS]) {
+    const int64_t p0 = st * kGvK;
+    const double *src = VM ? A + 2 * ((i0 + w) * K + p0 + lane) : A + 2 * ((p0 + w) * M + i0 + lane);
+    const int64_t step = 2 * kGvProd * (VM ? K : M);
+    const bool ok = VM ? p0 + lane < K : i0 + lane < M;
+    const int64_t left = (VM ? M - i0 : K - p0) - w;  // columns from this warp's first one on
 #pragma unroll
-      for (int u = 0; u < COLS; ++u)
-        load_dd<ALIGNED>(dst + u * kGvProd * 32, src + u * step, ok && u * kGvProd < left, A);
-      if (XR && w == 0)
-        load_dd<ALIGNED>(xs + (size_t)(st % S) * kGvK + lane, x + 2 * (p0 + lane), p0 + lane < K, x);
-    }
-    cp_async_commit();
-  };
-  // the vector's entries: this lane's k, or (uniform over the warp) those of
-  // the warp's columns
-  constexpr int NX = VM ? 1 : COLS;
-  auto load_x = [&](int64_t st, double2 (&v)[NX]) {
-#pragma unroll
-    for (int u = 0; u < NX; ++u) {
-      const int64_t p = st * kGvK + (VM ? lane : w + u * kGvProd);
-      v[u] = make_double2(0.0, 0.0);
-      if (p < K) {
-        const double *xp = x + 2 * p;
-        v[u] = ALIGNED ? *reinterpret_cast<const double2 *>(xp) : make_double2(xp[0], xp[1]);
+    for (int u = 0; u < COLS; ++u) {
+      a[u] = make_double2(0.0, 0.0);
+      if (ok && u * kGvProd < left) {
+        const double *q = src + u * step;
+        a[u] = ALIGNED ? __ldg(reinterpret_cast<const double2 *>(q)) : make_double2(q[0], q[1]);
       }
     }
   };
-  auto produce = [&](int64_t st, double2 (&v)[NX]) {
-    if (st >= nst) return;
-    const double2 *src = ring + ((size_t)(st % S) * kGvN + w) * 32 + lane;
-    double2 *out = pq + (size_t)(st & 1) * kGvK * PITCH;
-    double2 a[COLS];
-    if (XR) {
-      const double2 *xp = xs + (size_t)(st % S) * kGvK;
+  // the same entries into L2, one 128-byte line per eight lanes
+  auto prefetch = [&](int64_t st) {
+    const int64_t p0 = st * kGvK;
+    const double *src = VM ? A + 2 * ((i0 + w) * K + p0 + lane) : A + 2 * ((p0 + w) * M + i0 + lane);
+    const int64_t step = 2 * kGvProd * (VM ? K : M);
+    const bool ok = (lane & 7) == 0 && (VM ? p0 + lane < K : i0 + lane < M);
+    const int64_t left = (VM ? M - i0 : K - p0) - w;
 #pragma unroll
-      for (int u = 0; u < NX; ++u) v[u] = xp[VM ? lane : w + u * kGvProd];
-    }
-#pragma unroll
-    for (int u = 0; u < COLS; ++u) a[u] = src[u * kGvProd * 32];
-#pragma unroll
-    for (int u = 0; u < COLS; ++u) {
-      const int c = w + u * kGvProd;
-      if (VM)
-        out[lane * PITCH + c] = mac_terms(v[0].x, v[0].y, a[u].x, a[u].y);  // pitch 33: conflict-free
-      else
-        out[c * PITCH + lane] = mac_terms(a[u].x, a[u].y, v[u % NX].x, v[u % NX].y);
-    }
+    for (int u = 0; u < COLS; ++u)
+      if (ok && u * kGvProd < left) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + u * step));
   };
-  double2 xa[NX], xb[NX];
-  for (int st = 0; st < S - 1; ++st) issue(st);
-  if (!XR) {
-    load_x(0, xa);
-    load_x(1, xb);
-  }
-  cp_async_wait_n<S - 2>();  // stage 0 landed
-  if (XR) sync();            // the vector's part of it for every producer
-  produce(0, xa);
-  cp_async_wait_n<PENDING>();
-  sync();
-  for (int64_t st = 0; st < nst; ++st) {
-    issue(st + S - 1);  // into the slot of stage st - 1, read two iterations ago
-    if (!XR) {
-#pragma unroll
-      for (int u = 0; u < NX; ++u) xa[u] = xb[u];
-      load_x(st + 2, xb);
+  auto load_x = [&](int64_t st) {  // by the first producer, for all
+    if (st < nst) {
+      const int64_t p = st * kGvK + lane;
+      load_dd<ALIGNED>(xs + (st % S) * kGvK + lane, x + 2 * p, p < K, x);
     }
-    cp_async_wait_n<PENDING>();  // stage st + 1 landed (XR: st + 2, for the other producers)
-    produce(st + 1, xa);
-    sync();
+    cp_async_commit();
+  };
+  double2 a[P][COLS];
+  if (w == 0) {
+    for (int st = 0; st < S - 1; ++st) load_x(st);
+    cp_async_wait_n<S - 2>();
   }
-  cp_async_wait_n<0>();
+#pragma unroll
+  for (int q = 0; q < P; ++q) load(q, a[q]);
+  for (int q = P; q < kGvAhead; ++q) prefetch(q);
+  sync();  // the vector's first stage landed
+  for (int64_t base = 0; base <= nst; base += P) {
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+      const int64_t st = base + q;
+      if (st > nst) break;
+      if (w == 0) {
+        load_x(st + S - 1);        // into the slot of stage st - 1, read an iteration ago
+        cp_async_wait_n<S - 2>();  // stage st + 1 landed, for everyone after this iteration's barrier
+      }
+      if (st < nst) {
+        const double2 *xp = xs + (st % S) * kGvK;
+        double2 *out = pq + (st & 1) * kGvK * PITCH;
+        double2 v[VM ? 1 : COLS];
+        if (VM) {
+          v[0] = xp[lane];
+        } else {
+#pragma unroll
+          for (int u = 0; u < COLS; ++u) v[VM ? 0 : u] = xp[w + u * kGvProd];
+        }
+#pragma unroll
+        for (int u = 0; u < COLS; ++u) {
+          const int c = w + u * kGvProd;
+          if (VM)
+            out[lane * PITCH + c] = mac_terms(v[0].x, v[0].y, a[q][u].x, a[q][u].y);  // pitch 33: conflict-free
+          else
+            out[c * PITCH + lane] = mac_terms(a[q][u].x, a[q][u].y, v[VM ? 0 : u].x, v[VM ? 0 : u].y);
+        }
+        load(st + P, a[q]);
+        prefetch(st + kGvAhead);
+      }
+      sync();
+    }
+  }
+  if (w == 0) cp_async_wait_n<0>();
 }
 
 static bool aligned16(const void *a, const void *b, const void *c) {
@@ -484,16 +491,10 @@ int cgemm_dev(const complex64x2 *a, const complex64x2 *b, complex64x2 *c, int64_
 }
 
 // y(m) = A(m,k) x(k), or with VM y(m) = x(k) A(k,m).
-template <bool VM, int S, bool ALIGNED>
+template <bool VM, int P, bool ALIGNED>
 static int launch_gemv(const double *A, const double *x, double *y, int64_t m, int64_t k, int64_t ri, int sms,
                        cudaStream_t s) {
-  static std::once_flag once;  // dynamic shared memory above the 48 KB default
-  std::call_once(once, [] {
-    cudaFuncSetAttribute(gemv_dd_kernel<VM, S, ALIGNED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)gv_smem(VM, S));
-  });
-  gemv_dd_kernel<VM, S, ALIGNED><<<(unsigned)((m + kGvN - 1) / kGvN), kGvThreads, gv_smem(VM, S), s>>>(A, x, y, m, k,
-                                                                                                  ri, sms);
+  gemv_dd_kernel<VM, P, ALIGNED><<<(unsigned)((m + kGvN - 1) / kGvN), kGvThreads, 0, s>>>(A, x, y, m, k, ri, sms);
   MF_TRY_CUDA(cudaGetLastError());
   return MFCUDA_OK;
 }
@@ -511,10 +512,10 @@ static int gemv_any(const float64x2 *a, const float64x2 *x, float64x2 *y, int64_
   const int sms = sm_count();
   const bool one_wave = blocks <= sms;
   if (aligned16(a, x, y))
-    return one_wave ? launch_gemv<VM, 8, true>(A, X, Y, m, k, ri, sms, s)
-                    : launch_gemv<VM, 4, true>(A, X, Y, m, k, ri, sms, s);
-  return one_wave ? launch_gemv<VM, 8, false>(A, X, Y, m, k, ri, sms, s)
-                  : launch_gemv<VM, 4, false>(A, X, Y, m, k, ri, sms, s);
+    return one_wave ? launch_gemv<VM, 4, true>(A, X, Y, m, k, ri, sms, s)
+                    : launch_gemv<VM, 2, true>(A, X, Y, m, k, ri, sms, s);
+  return one_wave ? launch_gemv<VM, 4, false>(A, X, Y, m, k, ri, sms, s)
+                  : launch_gemv<VM, 2, false>(A, X, Y, m, k, ri, sms, s);
 }
 int gemv_dev(const float64x2 *a, const float64x2 *x, float64x2 *y, int64_t m, int64_t k,
              int64_t ri, cudaStream_t s) {

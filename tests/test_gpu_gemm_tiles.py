@@ -53,7 +53,8 @@ def test_real_tiles_unaligned(dev, shape):
     assert O.same_bits(got, O.matmul_mm(a, b, m, k, n, 8)).all()
 
 
-MATVEC = [(1, 1), (31, 7), (33, 32), (40, 33), (65, 64), (130, 259), (148 * 32, 65), (148 * 32 + 5, 97)]
+MATVEC = [(1, 1), (31, 7), (33, 32), (40, 33), (65, 64), (130, 259), (148 * 32, 65), (148 * 32 + 5, 97),
+          (70, 8 * 32), (70, 16 * 32 + 1)]
 
 
 @pytest.mark.parametrize("shape", MATVEC)  # one wave of CTAs up to 148 * 32 outputs, two CTAs per SM beyond
