@@ -38,6 +38,14 @@ def _run(dev, shapes, form, slices, R=0):
     return host, out, kc
 
 
+@pytest.mark.parametrize("extra", [[], [(900, 5, 1000)] * 12])  # alone, and beside short-k work for every SM
+def test_plain_tiles(dev, extra):
+    shapes = SHAPES + [(40, 700, 30), (23, 9, 60)] + extra
+    host, out, _ = _run(dev, shapes, "plain", 0)
+    for (m, k, n), (a, b), got in zip(shapes, host, out):
+        assert O.same_bits(got, O.matmul_mm(a, b, m, k, n, 8)).all(), (m, k, n)
+
+
 @pytest.mark.parametrize("slices", [0, 2, 3, 13])
 def test_digit_tiles(dev, slices):
     host, out, kc = _run(dev, SHAPES, "split", slices)
