@@ -34,7 +34,7 @@ SOURCES = [
     "shard.cu",
 ]
 HEADERS = ["common.cuh", "dd_device.cuh", "dd_tables.h", "tcgen05.cuh", "split_device.cuh", "gemm_tile.cuh",
-           "crt_device.cuh", "crt_tables.h", "grid_round.cuh"]
+           "crt_device.cuh", "crt_tables.h", "grid_round.cuh", "log_queue.cuh"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = [

@@ -39,6 +39,7 @@
 #include "dd_device.cuh"
 #include "gemm_tile.cuh"
 #include "crt_device.cuh"
+#include "log_queue.cuh"
 #include "split_device.cuh"
 #include "tcgen05.cuh"
 
@@ -149,14 +150,27 @@ __device__ __forceinline__ int find_array(const RArr *arrs, int narr, int64_t e)
 template <int OP>
 __global__ void __launch_bounds__(256) ragged_unary_kernel(const RArr *__restrict__ arrs, int narr,
                                                            int64_t total) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
+  auto ld = [&](int64_t e, mfdev::dd &v, double *&y) {
     const RArr a = arrs[find_array(arrs, narr, e)];
     const int64_t i = e - a.off;
-    mfdev::dd v = mfdev::make(a.x[2 * i], a.x[2 * i + 1]);
-    mfdev::dd r = apply<OP>(v);
-    a.y[2 * i] = r.hi;
-    a.y[2 * i + 1] = r.lo;
+    v = mfdev::make(a.x[2 * i], a.x[2 * i + 1]);
+    y = a.y + 2 * i;
+  };
+  auto st = [](double *y, mfdev::dd r) {
+    y[0] = r.hi;
+    y[1] = r.lo;
+  };
+  if constexpr (log_op<OP>) {
+    __shared__ LogQueue q;
+    log_map(q, total, ld, [](mfdev::dd v) { return apply<OP>(v); }, st);
+  } else {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
+      mfdev::dd v;
+      double *y;
+      ld(e, v, y);
+      st(y, apply<OP>(v));
+    }
   }
 }
 

@@ -10,6 +10,7 @@
 // exception and is HBM-bound.
 #include "common.cuh"
 #include "dd_device.cuh"
+#include "log_queue.cuh"
 
 namespace mfcuda {
 
@@ -29,24 +30,29 @@ __device__ __forceinline__ mfdev::dd apply(mfdev::dd x) {
 template <int OP, bool ALIGNED>
 __global__ void __launch_bounds__(256) unary_kernel(const double *__restrict__ x,
                                                     double *__restrict__ y, int64_t n) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    mfdev::dd v;
+  auto ld = [&](int64_t i) {
     if constexpr (ALIGNED) {
       double2 t = __ldcs(reinterpret_cast<const double2 *>(x) + i);
-      v.hi = t.x;
-      v.lo = t.y;
-    } else {
-      v.hi = x[2 * i];
-      v.lo = x[2 * i + 1];
+      return mfdev::make(t.x, t.y);
     }
-    mfdev::dd r = apply<OP>(v);
+    return mfdev::make(x[2 * i], x[2 * i + 1]);
+  };
+  auto st = [](double *p, mfdev::dd r) {
     if constexpr (ALIGNED) {
-      __stcs(reinterpret_cast<double2 *>(y) + i, make_double2(r.hi, r.lo));
+      __stcs(reinterpret_cast<double2 *>(p), make_double2(r.hi, r.lo));
     } else {
-      y[2 * i] = r.hi;
-      y[2 * i + 1] = r.lo;
+      p[0] = r.hi;
+      p[1] = r.lo;
     }
+  };
+  if constexpr (log_op<OP>) {
+    __shared__ LogQueue q;
+    log_map(q, n, [&](int64_t i, mfdev::dd &v, double *&p) { v = ld(i), p = y + 2 * i; },
+            [](mfdev::dd v) { return apply<OP>(v); }, st);
+  } else {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+      st(y + 2 * i, apply<OP>(ld(i)));
   }
 }
 

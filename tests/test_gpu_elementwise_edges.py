@@ -75,3 +75,33 @@ def test_pair_edges(dev):
     s, c = api.sincos(to_dev(x, dev))
     assert O.same_bits(to_host(s), O.unary("sin", x)).all()
     assert O.same_bits(to_host(c), O.unary("cos", x)).all()
+
+
+# sizes around a warp, a block and one pass of the grid (148 SMs x 16 blocks of
+# 256); shares of arguments next to one from none to all, so that both queues of
+# a warp fill, overflow and are emptied with 1 to 31 arguments left
+@pytest.mark.parametrize("op", ["log", "log2", "log10"])
+@pytest.mark.parametrize("n, share", [(1, 1.0), (31, 0.5), (33, 0.5), (257, 0.03), (4099, 0.97), (1300001, 0.0),
+                                      (1300001, 0.1), (1300001, 0.6), (1300001, 1.0)])
+def test_log_mixed(cuda_lib, dev, op, n, share):
+    import ctypes as C
+
+    import torch
+
+    r = np.random.default_rng(n)
+    hi = np.where(r.uniform(size=n) < share, r.uniform(0.94, 1.06, n), np.exp2(r.uniform(-40, 40, n)))
+    x = _interleave(hi, hi * r.uniform(-1, 1, n) * 2.0 ** -53)
+    want = O.unary(op, x)
+    assert O.same_bits(to_host(api.unary(op, to_dev(x, dev))), want).all()
+    off = to_dev(np.concatenate([[0.0], x]), dev)[1:]  # 8-byte aligned
+    assert O.same_bits(to_host(api.unary(op, off)), want).all()
+    if op == "log":  # ragged: pieces of 0 to 1000 elements of the same array
+        d, y = to_dev(x, dev), torch.zeros(2 * n, dtype=torch.float64, device=dev)
+        cuts = np.unique(np.concatenate([[0, n], r.integers(0, n + 1, 1 + n // 500)]))
+        lens = np.diff(cuts).tolist()
+        cnt = len(lens)
+        X = (C.c_void_p * cnt)(*[d.data_ptr() + 16 * int(c) for c in cuts[:-1]])
+        Y = (C.c_void_p * cnt)(*[y.data_ptr() + 16 * int(c) for c in cuts[:-1]])
+        s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert cuda_lib.mfcuda_unary_dd_ragged(1, X, Y, (C.c_int64 * cnt)(*lens), cnt, s) == 0
+        assert O.same_bits(to_host(y), want).all()
