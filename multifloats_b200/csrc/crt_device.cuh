@@ -856,13 +856,20 @@ __host__ __device__ constexpr int cr_smem(int ktn) {
 // lane quadrant) takes units e, e + CR_SETS, ... of the CTA; per unit it
 // copies its slot to registers, hands the slot back, and forms and stores its
 // 128 outputs with NL-limb arithmetic.
+// Columns from `co` on (sigB, flagB and the residues run on) are the second
+// output's: column j - co of C[1], combined by mode[1].
+struct RecOut {
+  const int *sigA, *flagA, *sigB, *flagB;
+  int64_t M, N, co;
+  double *C[2];
+  int64_t cstride;
+  int mode[2];
+};
 struct RecEpi {
   const CrtConst *cc;
-  const int *sigA, *flagA, *sigB, *flagB;
-  int64_t M, N, qbase, nrb, units;
-  double *C;
-  int64_t cstride;
-  int mode, W, nbe, nb, slot_cols, nslots;
+  RecOut o;
+  int64_t qbase, nrb, units;
+  int W, nbe, nb, slot_cols, nslots;
   uint32_t tmem;
   uint64_t *tfull, *tempty;
   volatile int *abort_flag;
@@ -889,11 +896,13 @@ __device__ __forceinline__ void crt_recon_epilogue(const RecEpi &p) {
   for (UnitCursor c(blockIdx.x + (int64_t)set * gridDim.x, (int64_t)CR_SETS * gridDim.x, p.nrb); c.u < p.units;
        c.advance()) {
     const int64_t i = c.rb * 32 + (mrow >> 2), j = 4 * (p.qbase + c.qd) + (mrow & 3);
-    const bool live = i < p.M && j < p.N;
+    const int part = j >= p.o.co;
+    const int64_t jc = part ? j - p.o.co : j;  // column of its output
+    const bool live = i < p.o.M && jc < p.o.N;
     int shift = 0, bad = 0;
     if (live) {  // loaded before the wait, in flight meanwhile
-      shift = p.sigA[i] + p.sigB[j] - 2 * p.W;
-      bad = p.flagA[i] | p.flagB[j];
+      shift = p.o.sigA[i] + p.o.sigB[j] - 2 * p.W;
+      bad = p.o.flagA[i] | p.o.flagB[j];
     }
     const bool got = wait_bar(&p.tfull[slot / CR_SETS], tph, p.abort_flag, p.wait_ns);
     if (!__all_sync(0xffffffffu, got)) {
@@ -922,16 +931,16 @@ __device__ __forceinline__ void crt_recon_epilogue(const RecEpi &p) {
     if (live) {
       uint32_t limb[NL];
       crt_limbs_nl<NL>(S, Mn, p.nbe, limb);
-      crt_emit_nl<NL>(limb, bad != 0, shift, p.C + 2 * (j * p.M + i) * p.cstride, p.mode);
+      crt_emit_nl<NL>(limb, bad != 0, shift, p.o.C[part] + 2 * (jc * p.o.M + i) * p.o.cstride, p.o.mode[part]);
     }
   }
 }
 
+// Units of 32 rows x one column quad: rows 32 rb0 .. of the residue planes, quads
+// qbase .. of them.
 __device__ __forceinline__ void crt_recon_body(const CUtensorMap *tmD, const Plan *plan, const CrtConst *cc,
-                                               const int *sigA, const int *flagA, const int *sigB,
-                                               const int *flagB, int64_t M, int64_t N, int64_t qbase,
-                                               int64_t nrb, int64_t units, int64_t k, double *__restrict__ C,
-                                               int64_t cstride, int mode, uint8_t *smem, int *status,
+                                               const RecOut &out, int64_t rb0, int64_t qbase, int64_t nrb,
+                                               int64_t units, int64_t k, uint8_t *smem, int *status,
                                                uint64_t wait_ns) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = plan->S, W = plan->W;
@@ -1008,7 +1017,7 @@ __device__ __forceinline__ void crt_recon_body(const CUtensorMap *tmD, const Pla
         for (int e = 0; e < ne; ++e, c.advance())
           for (int kt = 0; kt < ktn; ++kt)  // boxes of 32 moduli
             mftc::tma_load_3d(ring + stage * stage_bytes + e * box_bytes + kt * CR_BOX_BYTES, tmD, &full[stage],
-                              (int32_t)(c.rb * 128), (int32_t)(qbase + c.qd), 32 * kt);
+                              (int32_t)((rb0 + c.rb) * 128), (int32_t)(qbase + c.qd), 32 * kt);
         arm.arm(stage, ph);
         if (++stage == nst) {
           stage = 0;
@@ -1055,8 +1064,8 @@ __device__ __forceinline__ void crt_recon_body(const CUtensorMap *tmD, const Pla
     }
   } else {  // ---- epilogue ----
     const int nl = nbe / 4;
-    const RecEpi ep{cc, sigA, flagA, sigB, flagB, M, N, qbase, nrb, units, C, cstride, mode, W, nbe, nb, slot_cols,
-                    nslots, tmem, tfull, tempty, abort_flag, status, wait_ns};
+    const RecEpi ep{cc, out, qbase, nrb, units, W, nbe, nb, slot_cols, nslots, tmem, tfull, tempty, abort_flag,
+                    status, wait_ns};
     if (nl <= 5)
       crt_recon_epilogue<5>(ep);
     else if (nl == 6)

@@ -69,7 +69,8 @@ namespace split {
 struct Operand {
   const double *p;
   int64_t stride;
-  int64_t rows, rows_pad;  // rows of A or columns of B, and padded
+  int64_t rows, rows_pad;  // rows of A or columns of B, and of the slice planes
+  int64_t stats;           // rows whose statistics belong to this operand
   int *sig, *mu, *flag;
   int8_t *slices;
   int b_side;
@@ -94,7 +95,7 @@ __device__ __forceinline__ const Operand &operand_of(const Operands &ops, unsign
 __global__ void __launch_bounds__(256) init_kernel(const __grid_constant__ Operands ops, int *status) {
   const Operand &op = operand_of(ops, blockIdx.x);
   const int64_t i = (int64_t)(blockIdx.x - op.first) * blockDim.x + threadIdx.x;
-  if (i < op.rows_pad) {
+  if (i < op.stats) {
     op.sig[i] = SENT_LO;
     op.mu[i] = SENT_HI;
     op.flag[i] = 0;
@@ -847,13 +848,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 // ---------------------------------------------------------------------------
 // 5. combine
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(COMBINE_THREADS, COMBINE_BLOCKS) combine_kernel(const int32_t *__restrict__ D, const Plan *plan,
-                                                      const int *sigA, const int *flagA, const int *sigB,
-                                                      const int *flagB, int64_t M, int64_t N,
-                                                      int64_t M_pad, int64_t N_pad, int nkc,
-                                                      double *__restrict__ C, int64_t cstride, int mode) {
-  combine4_body(D, plan, sigA, flagA, sigB, flagB, M, N, M_pad, N_pad, nkc, C, cstride, mode,
-                (int64_t)blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
+// Block rows from N on are the second output's: the columns from co on of D.
+__global__ void __launch_bounds__(COMBINE_THREADS, COMBINE_BLOCKS)
+    combine_kernel(const int32_t *__restrict__ D, const Plan *plan, const __grid_constant__ RecOut o, int64_t M_pad,
+                   int64_t N_pad, int nkc) {
+  const int part = blockIdx.y >= o.N;
+  const int64_t c0 = part ? o.co : 0;
+  combine4_body(D + c0 * M_pad, plan, o.sigA, o.flagA, o.sigB + c0, o.flagB + c0, o.M, o.N, M_pad, N_pad, nkc,
+                o.C[part], o.cstride, o.mode[part], (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+                part ? blockIdx.y - o.N : blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -880,16 +883,15 @@ __global__ void __launch_bounds__(256) crt_slice_kernel(const __grid_constant__ 
   }
 }
 // Reconstruction fed by TMA (crt_recon_body): persistent, one CTA per SM;
-// units of 32 rows x one column quad, rows below M, quads qbase .. (columns
-// below N).  Dynamic shared memory cr_smem(ceil(moduli / 32)).
-__global__ void __launch_bounds__(CR_THREADS, 1) crt_recon_kernel(
-    const __grid_constant__ CUtensorMap tmD, const Plan *plan, const CrtConst *cc, const int *sigA,
-    const int *flagA, const int *sigB, const int *flagB, int64_t M, int64_t N, int64_t qbase, int64_t nrb,
-    int64_t units, int64_t k, double *__restrict__ C, int64_t cstride, int mode, int *status, uint64_t wait_ns) {
+// units of 32 rows x one column quad (crt_recon_body).  Dynamic shared memory
+// cr_smem(ceil(moduli / 32)).
+__global__ void __launch_bounds__(CR_THREADS, 1)
+    crt_recon_kernel(const __grid_constant__ CUtensorMap tmD, const Plan *plan, const CrtConst *cc,
+                     const __grid_constant__ RecOut out, int64_t rb0, int64_t qbase, int64_t nrb, int64_t units,
+                     int64_t k, int *status, uint64_t wait_ns) {
   extern __shared__ uint8_t cr_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(cr_raw) + 1023) & ~uintptr_t(1023));
-  crt_recon_body(&tmD, plan, cc, sigA, flagA, sigB, flagB, M, N, qbase, nrb, units, k, C, cstride, mode, smem,
-                 status, wait_ns);
+  crt_recon_body(&tmD, plan, cc, out, rb0, qbase, nrb, units, k, smem, status, wait_ns);
 }
 // K chunks of the residue products folded into chunk 0 (block row y =
 // modulus), words w0 .. w1 - 1 of each plane (the column quads of a panel:
@@ -988,6 +990,37 @@ static Layout layout(int64_t m, int64_t k, int64_t n, int nA, int nB, int nsl = 
   L.off_D = take((size_t)nsl * L.nkc * L.N_pad * L.M_pad * (crt ? 1 : sizeof(int32_t)));
   L.total = off;
   return L;
+}
+
+// The four real products of a complex one as a single product of [Ar; Ai] with
+// [Br | Bi], the second parts starting at row `ro` and column `co`: one tensor-core
+// launch whose tiles fill the chip together (four launches of 1009 x 1100 x 907 in
+// the CRT form took 40.5 us each, 7 rounds of 256 x 256 tiles at the rate operands
+// come from L2; one takes 122 us with 256 x 512 tiles), and two recombinations
+// instead of four.  The scratch holds all four products at once: for scratches up
+// to JOINT_MAX; larger products take one after the other through one scratch and
+// lose nothing by it.  B200, one after the other -> joint, us: CRT 64^3 139 -> 97,
+// 300 x 400 x 500 184 -> 147, 1009 x 1100 x 907 463 -> 387, 2048^3 (0.5 GB) 1587 ->
+// 1554, 3000^3 (1 GB) 4224 -> 4185, 4096 x 512 x 4096 (2 GB) 3968 -> 4024; digits
+// 64^3 139 -> 84, 1024^3 545 -> 503, 2048^3 (0.9 GB) 3102 -> 2857, 3000^3 (2 GB)
+// 9126 -> 9198.
+constexpr size_t JOINT_MAX = (size_t)1 << 30;
+struct Joint {
+  int64_t ro, co;
+  Layout L;
+  bool ok;
+};
+static bool layout_ok(const Layout &L) {
+  return L.M_pad <= INT32_MAX / 2 && L.N_pad <= INT32_MAX / 2 && L.kblocks <= INT32_MAX / 2 && L.N_pad <= 65535 &&
+         L.K_pad / 64 <= 65535;
+}
+static Joint joint_layout(int64_t m, int64_t k, int64_t n, int nsl, bool crt) {
+  Joint J;
+  J.ro = round_up(m, 32);  // row blocks of the reconstruction and of A's slicers
+  J.co = round_up(n, 4);   // column quads
+  J.L = layout(J.ro + m, k, J.co + n, 1, 1, nsl, crt);
+  J.ok = layout_ok(J.L) && J.L.total - J.L.off_D <= JOINT_MAX;
+  return J;
 }
 
 static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -1094,13 +1127,20 @@ int profile_end(double *sums, int64_t *calls) {
   return MFCUDA_OK;
 }
 
+static size_t call_bytes(int64_t m, int64_t k, int64_t n, bool complex_operands, int nsl, bool crt) {
+  const int no = complex_operands ? 2 : 1;
+  size_t total = layout(m, k, n, no, no, nsl, crt).total;
+  if (complex_operands) {
+    const Joint J = joint_layout(m, k, n, nsl, crt);
+    if (J.ok) total = std::max(total, J.L.total);
+  }
+  return total;
+}
 size_t workspace_size(int64_t m, int64_t k, int64_t n, bool complex_operands) {
-  int no = complex_operands ? 2 : 1;
-  return layout(m, k, n, no, no).total;
+  return call_bytes(m, k, n, complex_operands, SMAX, false);
 }
 size_t crt_workspace_size(int64_t m, int64_t k, int64_t n, int bits, bool complex_operands) {
-  int no = complex_operands ? 2 : 1;
-  return layout(m, k, n, no, no, crt_slices_max(k, bits), true).total;
+  return call_bytes(m, k, n, complex_operands, crt_slices_max(k, bits), true);
 }
 
 // Blocks of an operand in the scan.
@@ -1167,13 +1207,25 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
                         const Product *prods, int nprod, int64_t m, int64_t k, int64_t n, int slices,
                         double target, void *ws, size_t ws_bytes, cudaStream_t s, int *info, int crt = 0,
                         const PanelSink *sink = nullptr, const Agree *agree = nullptr) {
-  Layout L = layout(m, k, n, nA, nB, crt ? crt_slices_max(k, slices) : SMAX, crt != 0);
-  if (L.M_pad > INT32_MAX / 2 || L.N_pad > INT32_MAX / 2 || L.kblocks > INT32_MAX / 2 ||
-      L.N_pad > 65535 || L.K_pad / 64 > 65535)
-    return MFCUDA_ERR_UNSUPPORTED;
+  const int nsl_max = crt ? crt_slices_max(k, slices) : SMAX;
+  Layout L = layout(m, k, n, nA, nB, nsl_max, crt != 0);
+  if (!layout_ok(L)) return MFCUDA_ERR_UNSUPPORTED;
+  // complex: the four products at once where the scratch for it is there (a
+  // workspace that is enough for one product at a time stays accepted)
+  Joint J = {};
+  bool joint = nprod == 4 && !sink;
+  if (joint) {
+    J = joint_layout(m, k, n, nsl_max, crt != 0);
+    joint = J.ok && (!ws || ws_bytes >= J.L.total);
+  }
   void *own = nullptr;
+  if (joint && !ws && ws_alloc(&own, J.L.total, s) != MFCUDA_OK) {
+    cudaGetLastError();  // no room for all four: one after the other
+    joint = false;
+  }
+  if (joint) L = J.L;
   if (!ws) {
-    MF_TRY(ws_alloc(&own, L.total, s));
+    if (!own) MF_TRY(ws_alloc(&own, L.total, s));
     ws = own;
   } else if (ws_bytes < L.total) {
     return MFCUDA_ERR_WORKSPACE;
@@ -1188,11 +1240,14 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
   int *sig[4], *mu[4], *flag[4];
   int8_t *sl[4];
   for (int o = 0; o < nops; ++o) {
-    int64_t rows = o < nA ? L.M_pad : L.N_pad;
-    sig[o] = reinterpret_cast<int *>(base + L.off_stats[o]);
+    const bool aside = o < nA;
+    const int64_t rows = aside ? L.M_pad : L.N_pad;
+    const int lo = joint ? (aside ? 0 : 1) : o;  // joint: the parts of a side share planes and statistics
+    const int64_t r0 = joint && o != (aside ? 0 : nA) ? (aside ? J.ro : J.co) : 0;
+    sig[o] = reinterpret_cast<int *>(base + L.off_stats[lo]) + r0;
     mu[o] = sig[o] + rows;
     flag[o] = mu[o] + rows;
-    sl[o] = reinterpret_cast<int8_t *>(base + L.off_slices[o]);
+    sl[o] = reinterpret_cast<int8_t *>(base + L.off_slices[lo]) + r0 * (aside && crt ? 1 : L.K_pad);
   }
   const uint64_t wait_ns = wait_limit_ns();
   int rc = MFCUDA_OK;
@@ -1222,6 +1277,7 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
       op.stride = aside ? astride[o] : bstride[o - nA];
       op.rows = aside ? m : n;
       op.rows_pad = aside ? L.M_pad : L.N_pad;
+      op.stats = !joint ? op.rows_pad : (o == 0 || o == nA) ? (aside ? J.ro : J.co) : op.rows;
       op.sig = sig[o];
       op.mu = mu[o];
       op.flag = flag[o];
@@ -1242,7 +1298,7 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
       // operands before o0 have no blocks: operand_of takes the last one that starts at 0
       return (unsigned)total;
     };
-    const unsigned init_blocks = lay_out(0, nops, [](const Operand &op) { return (op.rows_pad + 255) / 256; });
+    const unsigned init_blocks = lay_out(0, nops, [](const Operand &op) { return (op.stats + 255) / 256; });
     init_kernel<<<init_blocks, 256, 0, s>>>(ops, status);
     // enough blocks to fill the chip, long enough chunks to keep the atomics few
     for (int o = 0; o < nops; ++o) {
@@ -1297,7 +1353,8 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
     mark(2, s);
     CUtensorMap tmA[4], tmB[4], tmD;
     if (crt && !make_residue_map(&tmD, D, L.M_pad, L.N_pad, L.nkc, L.nsl)) rc = MFCUDA_ERR_CUDA;
-    for (int q = 0; q < nprod; ++q)
+    const int nmma = joint ? 1 : nprod;
+    for (int q = 0; q < nmma; ++q)
       if (!(crt ? make_map_mn(&tmA[q], sl[prods[q].a], L.M_pad, L.K_pad, L.nsl)
                 : make_map(&tmA[q], sl[prods[q].a], L.M_pad, L.K_pad, BM, L.nsl)) ||
           !make_map(&tmB[q], sl[nA + prods[q].b], L.N_pad, L.K_pad, L.pair ? 128 : BN, L.nsl))
@@ -1317,8 +1374,24 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
         const int supers = (crt ? L.nsl : (L.nsl + 1) / 2) * (int)L.nkc * (int)(L.M_pad / tile_m) * (tn1 - tn0);
         pgrid = std::min(pair_grid(), 2 * supers);
       }
-      for (int q = 0; q < nprod && rc == MFCUDA_OK; ++q) {
-        const int ia = prods[q].a, ib = nA + prods[q].b;
+      // outputs of the columns [j0, j1): of product p, or of products p and p2
+      // whose columns follow one another (joint)
+      auto recombine = [&](const Product &p, const Product *p2) {
+        const int ia = p.a, ib = nA;
+        const RecOut o = {sig[ia], flag[ia], sig[p2 ? ib : ib + p.b], flag[p2 ? ib : ib + p.b],
+                          m,       p2 ? n : j1, p2 ? J.co : INT64_MAX, {p.out, p2 ? p2->out : nullptr},
+                          p.ostride, {p.mode, p2 ? p2->mode : 0}};
+        const int64_t r0 = p2 && ia ? J.ro : 0;
+        if (crt) {
+          const int64_t q0 = j0 / 4, q1 = ((p2 ? J.co + n : j1) + 3) / 4, nrb = (m + 31) / 32, units = nrb * (q1 - q0);
+          crt_recon_kernel<<<(unsigned)std::min<int64_t>(units, sm_count()), CR_THREADS, cr_smem((L.nsl + 31) / 32),
+                             s>>>(tmD, plan, cc, o, r0 / 32, q0, nrb, units, k, status, wait_ns);
+        } else {
+          combine_kernel<<<dim3(cgx, (unsigned)(p2 ? 2 * n : n)), COMBINE_THREADS, 0, s>>>(D + r0, plan, o, L.M_pad,
+                                                                                          L.N_pad, (int)L.nkc);
+        }
+      };
+      for (int q = 0; q < nmma && rc == MFCUDA_OK; ++q) {
         if (L.pair)
           split_mma_pair_kernel<<<pgrid, PAIR_THREADS, PAIR_SMEM, s>>>(
               tmA[q], tmB[q], plan, D, (int)L.M_pad, (int)L.N_pad, (int)L.nkc, (int)L.kblocks, L.nsub, tn0,
@@ -1327,21 +1400,22 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
           split_mma_kernel<<<pgrid, MMA_THREADS, MMA_SMEM, s>>>(tmA[q], tmB[q], plan, D, (int)L.M_pad,
                                                                 (int)L.N_pad, (int)L.nkc, (int)L.kblocks,
                                                                 status, wait_ns);
-        if (q == nprod - 1 && pp == npan - 1) mark(3, s);
-        if (crt) {
-          const int64_t q0 = j0 / 4, q1 = (j1 + 3) / 4, nrb = (m + 31) / 32, units = nrb * (q1 - q0);
-          if (L.nkc > 1) {
-            const int64_t plane_words = L.N_pad * L.M_pad / 4, nw = (q1 - q0) * L.M_pad;
-            crt_fold_kernel<<<dim3((unsigned)((nw + 255) / 256), (unsigned)L.nsl), 256, 0, s>>>(
-                reinterpret_cast<uint32_t *>(D), plan, (int)L.nkc, plane_words, q0 * L.M_pad, q1 * L.M_pad);
+        if (q == nmma - 1 && pp == npan - 1) mark(3, s);
+        if (crt && L.nkc > 1) {
+          const int64_t q0 = j0 / 4, q1 = joint ? L.N_pad / 4 : (j1 + 3) / 4;
+          const int64_t plane_words = L.N_pad * L.M_pad / 4, nw = (q1 - q0) * L.M_pad;
+          crt_fold_kernel<<<dim3((unsigned)((nw + 255) / 256), (unsigned)L.nsl), 256, 0, s>>>(
+              reinterpret_cast<uint32_t *>(D), plan, (int)L.nkc, plane_words, q0 * L.M_pad, q1 * L.M_pad);
+        }
+        if (!joint)
+          recombine(prods[q], nullptr);
+        else  // Ar with both parts of B, then Ai: re = Ar Br, then - Ai Bi; im = Ar Bi, then + Ai Br
+          for (int part = 0; part < 2; ++part) {
+            const Product *pb[2] = {};
+            for (int t = 0; t < nprod; ++t)
+              if (prods[t].a == part) pb[prods[t].b] = &prods[t];
+            recombine(*pb[0], pb[1]);
           }
-          crt_recon_kernel<<<(unsigned)std::min<int64_t>(units, sm_count()), CR_THREADS, cr_smem((L.nsl + 31) / 32),
-                             s>>>(tmD, plan, cc, sig[ia], flag[ia], sig[ib], flag[ib], m, j1, q0, nrb, units, k,
-                                  prods[q].out, prods[q].ostride, prods[q].mode, status, wait_ns);
-        } else
-          combine_kernel<<<dim3(cgx, (unsigned)n), COMBINE_THREADS, 0, s>>>(
-              D, plan, sig[ia], flag[ia], sig[ib], flag[ib], m, n, L.M_pad, L.N_pad, (int)L.nkc, prods[q].out,
-              prods[q].ostride, prods[q].mode);
       }
       if (sink && rc == MFCUDA_OK) sink->done(sink->ctx, j0, j1, s);
     }
