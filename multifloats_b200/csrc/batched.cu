@@ -265,9 +265,9 @@ __global__ void __launch_bounds__(256) g_crt_slice_a(const SProb *probs, const O
   const int64_t t = (int64_t)own.local * 256 + threadIdx.x;
   const int64_t per_k = (P.m + 7) / 8;
   const int64_t kp = t / per_k;
-  if (kp < P.K_pad)
-    crt_slice_a_mn_one(P.A, P.m, P.k, P.astride, P.M_pad, P.K_pad, P.sigA, P.flagA, P.plan, P.As,
-                       (t % per_k) * 8, kp);
+  CrtSlice c;
+  c.a(P.A, P.m, P.k, P.astride, P.M_pad, P.K_pad, P.sigA, P.flagA, P.As, (t % per_k) * 8, kp);
+  c.run(P.plan);
 }
 __global__ void __launch_bounds__(256) g_crt_slice_b(const SProb *probs, const Owner *owner) {
   const Owner own = owner[blockIdx.x];
@@ -275,8 +275,9 @@ __global__ void __launch_bounds__(256) g_crt_slice_b(const SProb *probs, const O
   const int64_t t = (int64_t)own.local * 256 + threadIdx.x;
   const int64_t per_col = P.K_pad / 8;
   const int64_t j = t / per_col;
-  if (j < P.n)
-    crt_slice_b_one(P.B, P.k, P.n, P.bstride, P.N_pad, P.K_pad, P.sigB, P.flagB, P.plan, P.Bs, j, (t % per_col) * 8);
+  CrtSlice c;
+  c.b(P.B, P.k, P.n, P.bstride, P.N_pad, P.K_pad, P.sigB, P.flagB, P.Bs, j, (t % per_col) * 8);
+  c.run(P.plan);
 }
 // flat: thread t of the problem takes column t / (K_pad / 8), entries 8 (t % (K_pad / 8)) .. + 7
 __global__ void __launch_bounds__(256) g_slice_b(const SProb *probs, const Owner *owner) {

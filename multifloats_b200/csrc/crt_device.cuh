@@ -211,75 +211,73 @@ __device__ __forceinline__ void for_each_residue_word(const uint32_t (&dw)[8][4]
   else
     residue_words_nw<4>(dw, t0, t1, f);
 }
-// A (m x k column-major view) -> As[t][p][i]: the MN-major residue planes
-// of the tensor-core kernels (the rows of one K index
-// contiguous, so a thread's eight residues of consecutive rows are one
-// 64-bit store and a warp's stores are contiguous; no transposition).
-// Entries i8 .. i8+7 of column p.
-__device__ __forceinline__ void crt_slice_a_mn_one(const double *__restrict__ A, int64_t M, int64_t K,
-                                                   int64_t stride, int64_t M_pad, int64_t K_pad, const int *sig,
-                                                   const int *flag, const Plan *plan, int8_t *__restrict__ As,
-                                                   int64_t i8, int64_t p) {
-  const int n = plan->S, W = plan->W;
-  uint32_t y[8][4];
-  bool any = false;
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int64_t i = i8 + e;
-    if (p < K && i < M && !flag[i]) {
-      const double2 v = __ldg(reinterpret_cast<const double2 *>(A) + (p * M + i) * stride);
-      biased_bytes(v.x, v.y, sig[i], W, y[e]);
-      any = true;
-    } else {
-#pragma unroll
-      for (int w = 0; w < 4; ++w) y[e][w] = bias_word(w);  // X = 0: every residue zero
-    }
+// Residues of eight entries that follow one another in memory, by one thread.
+// a: entries i8 .. i8 + 7 of column p of A (m x k column-major view), to
+// As[t][p][i], the MN-major planes of the tensor-core kernels (the rows of one K
+// index contiguous, so no transposition).  b: entries p8 .. p8 + 7 of column j of
+// B (k x n), to Bs[t][j][p].  Either way one 8-byte word per modulus, contiguous
+// over a warp.  One code for both sides: the unrolled rounding and modulus loop are
+// some 45 KB of instructions, and with a copy per side 20 % of the stalls were
+// waits for instructions (the rest: the pipe of dp4a and the multiplications, 58 %
+// busy, and the loads).  B200, both operands: 1024^2 60 -> 52 us, 2048^2 170 -> 153,
+// 4096^2 (W = 105) 618 -> 582; a barrier before the moduli, so that a block's warps
+// fetch them together: no change; blocks of 128, 512, 1024 threads: 603, 645, 690.
+constexpr int CRT_SLICE_THREADS = 256;
+struct CrtSlice {
+  const double2 *src;
+  int64_t stride;
+  const int *sig, *flag;  // of the first entry
+  int each;               // 1: every entry has its own, 0: one for all
+  int valid;              // entries of the operand; -1: nothing to write
+  int8_t *out;
+  int64_t plane;
+  __device__ __forceinline__ void a(const double *A, int64_t M, int64_t K, int64_t stride_, int64_t M_pad, int64_t K_pad,
+                                    const int *sig_, const int *flag_, int8_t *As, int64_t i8, int64_t p) {
+    src = reinterpret_cast<const double2 *>(A) + (p * M + i8) * stride_;
+    stride = stride_;
+    sig = sig_ + i8;
+    flag = flag_ + i8;
+    each = 1;
+    valid = p >= K_pad ? -1 : p < K ? (int)min((int64_t)8, M - i8) : 0;
+    out = As + p * M_pad + i8;
+    plane = K_pad * M_pad;
   }
-  auto put = [&](int sl, uint64_t word) {
-    *reinterpret_cast<uint64_t *>(As + (((int64_t)sl * K_pad + p) * M_pad + i8)) = word;
-  };
-  if (any) {
+  __device__ __forceinline__ void b(const double *B, int64_t K, int64_t N, int64_t stride_, int64_t N_pad, int64_t K_pad,
+                                    const int *sig_, const int *flag_, int8_t *Bs, int64_t j, int64_t p8) {
+    src = reinterpret_cast<const double2 *>(B) + (j * K + p8) * stride_;
+    stride = stride_;
+    sig = sig_ + j;
+    flag = flag_ + j;
+    each = 0;
+    valid = j >= N ? -1 : (int)max((int64_t)0, min((int64_t)8, K - p8));
+    out = Bs + j * K_pad + p8;
+    plane = N_pad * K_pad;
+  }
+  __device__ __forceinline__ void run(const Plan *plan) {
+    const int n = plan->S, W = plan->W;
     uint32_t dw[8][4];
+    bool any = false;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) digit_words(y[e], dw[e]);
-    for_each_residue_word(dw, 0, n, W, put);
-  } else {  // padding or flagged rows only: every residue zero
-    for (int sl = 0; sl < n; ++sl) put(sl, 0);
-  }
-}
-
-// B (k x n column-major view) -> Bs[t][j][p]: entries p8 .. p8+7 of column j.
-__device__ __forceinline__ void crt_slice_b_one(const double *__restrict__ B, int64_t K, int64_t N,
-                                                int64_t stride, int64_t N_pad, int64_t K_pad, const int *sig,
-                                                const int *flag, const Plan *plan, int8_t *__restrict__ Bs,
-                                                int64_t j, int64_t p8) {
-  const int n = plan->S, W = plan->W;
-  const bool col_ok = j < N && !flag[j < N ? j : 0];
-  const int tau = j < N ? sig[j] : 0;
-  uint32_t y[8][4];
+    for (int e = 0; e < 8; ++e) {
+      uint32_t y[4];
+      if (e < valid && !flag[e * each]) {
+        const double2 v = __ldg(src + e * stride);
+        biased_bytes(v.x, v.y, sig[e * each], W, y);
+        any = true;
+      } else {
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    int64_t p = p8 + e;
-    if (col_ok && p < K) {
-      double2 v = __ldg(reinterpret_cast<const double2 *>(B) + (j * K + p) * stride);
-      biased_bytes(v.x, v.y, tau, W, y[e]);
-    } else {
-#pragma unroll
-      for (int w = 0; w < 4; ++w) y[e][w] = bias_word(w);
+        for (int w = 0; w < 4; ++w) y[w] = bias_word(w);  // X = 0: every residue zero
+      }
+      digit_words(y, dw[e]);
     }
+    if (valid < 0) return;
+    auto put = [&](int t, uint64_t word) { *reinterpret_cast<uint64_t *>(out + t * plane) = word; };
+    if (any)
+      for_each_residue_word(dw, 0, n, W, put);
+    else  // padding or flagged entries only
+      for (int t = 0; t < n; ++t) put(t, 0);
   }
-  auto put = [&](int sl, uint64_t word) {
-    *reinterpret_cast<uint64_t *>(Bs + (((int64_t)sl * N_pad + j) * K_pad + p8)) = word;
-  };
-  if (col_ok && p8 < K) {
-    uint32_t dw[8][4];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) digit_words(y[e], dw[e]);
-    for_each_residue_word(dw, 0, n, W, put);
-  } else {  // padding only: every residue zero
-    for (int sl = 0; sl < n; ++sl) put(sl, 0);
-  }
-}
+};
 
 // Residue layout of one product (modulus t, K chunk kc): N_pad x M_pad bytes,
 // four consecutive columns interleaved per row -- byte (j, i) at

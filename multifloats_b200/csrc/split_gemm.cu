@@ -866,21 +866,21 @@ __global__ void __launch_bounds__(COMBINE_THREADS, COMBINE_BLOCKS)
 // columns past the operand are padding no output depends on): a thread per 8
 // consecutive rows of a K index (A, MN-major planes) or per 8 consecutive K
 // indices of a column (B: columns j0 .. of it).
-__global__ void __launch_bounds__(256) crt_slice_kernel(const __grid_constant__ Operands ops, const Plan *plan,
-                                                        unsigned j0, unsigned j1) {
+__global__ void __launch_bounds__(CRT_SLICE_THREADS)
+    crt_slice_kernel(const __grid_constant__ Operands ops, const Plan *plan, unsigned j0, unsigned j1) {
   const Operand &op = operand_of(ops, blockIdx.x);
-  const unsigned t = (blockIdx.x - op.first) * 256 + threadIdx.x;
+  const unsigned t = (blockIdx.x - op.first) * CRT_SLICE_THREADS + threadIdx.x;
+  CrtSlice c;
   if (op.b_side) {
     const unsigned per_col = (unsigned)(ops.k_pad / 8), j = j0 + t / per_col;
-    if (j < j1 && j < op.rows)
-      crt_slice_b_one(op.p, ops.k, op.rows, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, plan, op.slices, j,
-                      (int64_t)(t % per_col) * 8);
+    c.b(op.p, ops.k, op.rows, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, op.slices, j < j1 ? j : op.rows,
+        (int64_t)(t % per_col) * 8);
   } else {
     const unsigned per_k = (unsigned)((op.rows + 7) / 8), kp = t / per_k;
-    if (kp < ops.k_pad)
-      crt_slice_a_mn_one(op.p, op.rows, ops.k, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, plan, op.slices,
-                         (int64_t)(t % per_k) * 8, kp);
+    c.a(op.p, op.rows, ops.k, op.stride, op.rows_pad, ops.k_pad, op.sig, op.flag, op.slices,
+        (int64_t)(t % per_k) * 8, kp);
   }
+  c.run(plan);
 }
 // Reconstruction fed by TMA (crt_recon_body): persistent, one CTA per SM;
 // units of 32 rows x one column quad (crt_recon_body).  Dynamic shared memory
@@ -1325,12 +1325,13 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
     const int tn_cols = BN * L.nsub;
     const int ntn_all = (int)(L.N_pad / tn_cols);
     const int npan = (sink && crt && L.pair) ? std::max(1, std::min(sink->panels, ntn_all)) : 1;
+    const int per = crt ? CRT_SLICE_THREADS : 256;
     auto slice_blocks = [&](const Operand &op) {  // flat: a thread per 8 entries
-      return (op.b_side ? op.rows * (L.K_pad / 8) : (op.rows + 7) / 8 * L.K_pad) / 256 + 1;
+      return (op.b_side ? op.rows * (L.K_pad / 8) : (op.rows + 7) / 8 * L.K_pad) / per + 1;
     };
     if (crt) {  // with column panels B's residues follow panel by panel
       const unsigned blocks = lay_out(0, npan > 1 ? nA : nops, slice_blocks);
-      crt_slice_kernel<<<blocks, 256, 0, s>>>(ops, plan, 0, (unsigned)L.N_pad);
+      crt_slice_kernel<<<blocks, CRT_SLICE_THREADS, 0, s>>>(ops, plan, 0, (unsigned)L.N_pad);
     } else {
       const unsigned blocks = lay_out(0, nops, [&](const Operand &op) {
         return op.b_side ? slice_blocks(op) : (op.rows + 31) / 32 * (L.K_pad / 64);
@@ -1366,8 +1367,8 @@ static int run_products(const double *const *aview, const int64_t *astride, int 
       if (npan > 1) {  // this panel's columns of B (padding columns included)
         const unsigned c0 = (unsigned)(tn0 * tn_cols), c1 = (unsigned)(tn1 * tn_cols);
         const unsigned blocks = lay_out(
-            nA, nops, [&](const Operand &) { return ((int64_t)(c1 - c0) * (L.K_pad / 8) + 255) / 256; });
-        crt_slice_kernel<<<blocks, 256, 0, s>>>(ops, plan, c0, c1);
+            nA, nops, [&](const Operand &) { return ((int64_t)(c1 - c0) * (L.K_pad / 8) + CRT_SLICE_THREADS - 1) / CRT_SLICE_THREADS; });
+        crt_slice_kernel<<<blocks, CRT_SLICE_THREADS, 0, s>>>(ops, plan, c0, c1);
       }
       int pgrid = grid;
       if (L.pair && npan > 1) {
