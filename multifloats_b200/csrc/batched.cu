@@ -204,6 +204,9 @@ struct SProb {
 };
 // phases with a per-problem block count (and the items, with their prefix sums); the
 // recombination runs in two launches: stores first, then the - / + updates
+// K indices whose digits or residues the tensor cores read: whole steps of 32.
+__host__ __device__ constexpr int64_t k_fill(int64_t k) { return k < 1 ? 32 : (k + 31) / 32 * 32; }
+
 enum { PH_SCAN_A, PH_SCAN_B, PH_SLICE_A, PH_SLICE_B, PH_COMBINE, PH_COMBINE2, PH_ITEMS, PH_COUNT };
 
 // A block's problem and its index among the problem's blocks of the phase, from
@@ -266,25 +269,26 @@ __global__ void __launch_bounds__(256) g_crt_slice_a(const SProb *probs, const O
   const int64_t per_k = (P.m + 7) / 8;
   const int64_t kp = t / per_k;
   CrtSlice c;
-  c.a(P.A, P.m, P.k, P.astride, P.M_pad, P.K_pad, P.sigA, P.flagA, P.As, (t % per_k) * 8, kp);
+  c.a(P.A, P.m, P.k, P.astride, P.M_pad, P.K_pad, P.sigA, P.flagA, P.As, (t % per_k) * 8,
+      kp < k_fill(P.k) ? kp : P.K_pad);
   c.run(P.plan);
 }
 __global__ void __launch_bounds__(256) g_crt_slice_b(const SProb *probs, const Owner *owner) {
   const Owner own = owner[blockIdx.x];
   const SProb &P = probs[own.p];
   const int64_t t = (int64_t)own.local * 256 + threadIdx.x;
-  const int64_t per_col = P.K_pad / 8;
+  const int64_t per_col = k_fill(P.k) / 8;
   const int64_t j = t / per_col;
   CrtSlice c;
   c.b(P.B, P.k, P.n, P.bstride, P.N_pad, P.K_pad, P.sigB, P.flagB, P.Bs, j, (t % per_col) * 8);
   c.run(P.plan);
 }
-// flat: thread t of the problem takes column t / (K_pad / 8), entries 8 (t % (K_pad / 8)) .. + 7
+// flat: thread t of the problem takes column t / (k_fill / 8), entries 8 (t % (k_fill / 8)) .. + 7
 __global__ void __launch_bounds__(256) g_slice_b(const SProb *probs, const Owner *owner) {
   const Owner own = owner[blockIdx.x];
   const SProb &P = probs[own.p];
   const int64_t t = (int64_t)own.local * 256 + threadIdx.x;
-  const int64_t per_col = P.K_pad / 8;
+  const int64_t per_col = k_fill(P.k) / 8;
   const int64_t j = t / per_col;
   if (j < P.n)
     slice_b_one(P.B, P.k, P.n, P.bstride, P.N_pad, P.K_pad, P.sigB, P.flagB, P.plan, P.Bs, j, (t % per_col) * 8);
@@ -331,8 +335,10 @@ struct __align__(16) GItem {
   int g, nd;       // digits: diagonals g, g - 1, ... (nd of them); CRT: modulus g, nd = 1; nd = 0: beyond the plan
   int kb0, kb1;    // K blocks
   int a_row, b_row;  // first row of A and column of B
-  int bn;
-  int M_pad, pad[3];
+  int bn;          // columns of the tile: those of the output, rounded up to 32
+  int M_pad;
+  int rows;        // rows of the tile that the output has
+  int klast, pad;  // K steps of 32 of block kb1 - 1: those of the operands
   int32_t *dst;    // D of diagonal / modulus g, K chunk and tile
   int64_t gstride;  // INT32 sums between diagonals
 };
@@ -345,7 +351,7 @@ __device__ __forceinline__ GItem load_item(const GItem *items, int64_t w, int64_
   if (w < n) {
     const int4 *src = reinterpret_cast<const int4 *>(items + w);
     const int4 a = __ldg(src), b = __ldg(src + 1);
-    const int2 c = __ldg(reinterpret_cast<const int2 *>(src + 2));
+    const int4 c = __ldg(src + 2);
     const longlong2 e = __ldg(reinterpret_cast<const longlong2 *>(src + 3));
     it.p = a.x;
     it.g = a.y;
@@ -356,11 +362,20 @@ __device__ __forceinline__ GItem load_item(const GItem *items, int64_t w, int64_
     it.b_row = b.z;
     it.bn = b.w;
     it.M_pad = c.x;
+    it.rows = c.y;
+    it.klast = c.z;
     it.dst = reinterpret_cast<int32_t *>(e.x);
     it.gstride = e.y;
   }
   return it;
 }
+// Tiles come in boxes of 64 rows, only those the output has, and the MMAs, the
+// drain and the slicers stop at the same bounds (columns rounded up to 32, K to the
+// 32 of a step): the problems of a batch are small, and whole tiles of 128 x 256 x
+// 128 were 2.3 times the work.  B200, whole tiles -> these, us: 2000 problems up to
+// 1024 digits 10950 -> 10560, CRT 13760 -> 12690; 300 up to 256 330 -> 313, 514 ->
+// 448; 1000 up to 64 458 -> 442, 708 -> 553.
+constexpr int G_BOX = 64;
 // Diagonals of an item of the digit-sliced form.
 constexpr int GD_DIAGS = 2;
 __host__ __device__ constexpr int g_groups(int nsl, bool crt) { return crt ? nsl : (nsl + GD_DIAGS - 1) / GD_DIAGS; }
@@ -378,9 +393,11 @@ __global__ void __launch_bounds__(128) g_items(const SProb *probs, const int64_t
     it.kb1 = min(P.kblocks, it.kb0 + P.kcb);
     it.a_row = tile % P.ntm * BM;
     it.b_row = tile / P.ntm * P.bn;
-    it.bn = P.bn;
+    it.bn = ((int)min((int64_t)P.bn, P.n - it.b_row) + 31) / 32 * 32;
     it.M_pad = (int)P.M_pad;
-    it.pad[0] = it.pad[1] = it.pad[2] = 0;
+    it.rows = (int)min((int64_t)BM, P.m - it.a_row);
+    it.klast = it.kb1 < P.kblocks ? BK / UMMA_K : (int)(k_fill(P.k) - (int64_t)(P.kblocks - 1) * BK) / UMMA_K;
+    it.pad = 0;
     it.gstride = (int64_t)P.nkc * P.N_pad * P.M_pad;
     const int64_t off = (int64_t)max(it.g, 0) * it.gstride + ((int64_t)kc * P.N_pad + it.b_row) * P.M_pad + it.a_row;
     // CRT: one byte per output, four columns per 32-bit word (crt_device.cuh)
@@ -449,7 +466,8 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         const GItem it = next;
         next = load_item(items, w + gridDim.x, nitems);
         if (!it.nd) continue;
-        const uint32_t bytes = (uint32_t)(A_STAGE + it.bn * BK);
+        const int nb = (it.bn + G_BOX - 1) / G_BOX;
+        const uint32_t bytes = (uint32_t)(A_STAGE + nb * G_BOX * BK);
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
           if (!wait_bar(&empty[stage], phase ^ 1, abort_flag, wait_ns)) {
             fail(1);
@@ -459,7 +477,9 @@ __global__ void __launch_bounds__(G_THREADS, 1)
           mftc::mbar_arrive_expect_tx(&full[stage], bytes);
           // A: MN-major residue planes (row, K index, modulus)
           mftc::tma_load_3d(sA + stage * A_STAGE, &maps[2 * it.p], &full[stage], it.a_row, kb * BK, it.g);
-          mftc::tma_load_3d(sB + stage * B_STAGE, &maps[2 * it.p + 1], &full[stage], kb * BK, it.b_row, it.g);
+          for (int b = 0; b < nb; ++b)
+            mftc::tma_load_3d(sB + stage * B_STAGE + b * G_BOX * BK, &maps[2 * it.p + 1], &full[stage], kb * BK,
+                              it.b_row + b * G_BOX, it.g);
           arm.arm(stage, phase);
           if (++stage == NSTAGE) {
             stage = 0;
@@ -498,8 +518,10 @@ __global__ void __launch_bounds__(G_THREADS, 1)
           mftc::tc_fence_after();
           const uint32_t a0 = mftc::smem_u32(sA + stage * A_STAGE);
           const uint32_t b0 = mftc::smem_u32(sB + stage * B_STAGE);
+          const int ks = kb == it.kb1 - 1 ? it.klast : BK / UMMA_K;
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+            if (kk >= ks) break;
             mftc::umma_i8(d_tmem, mftc::smem_desc_k_sw128(a0 + kk * a_kstep),
                           mftc::smem_desc_k_sw128(b0 + kk * UMMA_K), idesc, accumulate);
             accumulate = 1;
@@ -539,10 +561,10 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         break;
       }
       mftc::tc_fence_after();
-      const int nch = it.bn / 64, ch0 = half * nch;  // this warp's 32-column chunks
-      // residues modulo m_g, four columns per 32-bit word (crt_device.cuh)
-      uint32_t *dst = reinterpret_cast<uint32_t *>(it.dst) + row + (int64_t)ch0 * 8 * it.M_pad;
-      for (int chunk = ch0; chunk < ch0 + nch; ++chunk) {
+      const int nch = quad * 32 < it.rows ? it.bn / 32 : 0;  // 32-column chunks, every other one this warp's
+      for (int chunk = half; chunk < nch; chunk += 2) {
+        // residues modulo m_g, four columns per 32-bit word (crt_device.cuh)
+        uint32_t *dst = reinterpret_cast<uint32_t *>(it.dst) + row + (int64_t)chunk * 8 * it.M_pad;
         uint32_t r[32];
         mftc::tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN + chunk * 32), r);
         mftc::tmem_wait_ld();
@@ -587,8 +609,8 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 // each to the other roles through a small ring in shared memory): dealt round
 // robin the busiest CTA had 16 % more work than the mean.
 //
-// Bound: the tensor pipe while an item runs (two thirds of the issuing
-// thread's time goes into MMAs waiting for it), then the drain, hidden only
+// Bound: the operands from L2 (45 GB for 2000 products up to 1024: 7.5 of about
+// 9 TB/s; the MMAs alone would take 2.6 ms), then the drain, hidden only
 // behind the next item's loads (the accumulators fill tensor memory; they are
 // handed back one by one in the order the next item needs them).  Four
 // diagonals on 128 x 128 tiles load less, but a 128-column MMA takes 102 cycles
@@ -696,7 +718,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         rw.advance();
         if (end) break;
         const CUtensorMap *ma = &maps[2 * it.p], *mb = ma + 1;
-        const uint32_t b_bytes = (uint32_t)(it.bn * BK);
+        const int na = (it.rows + G_BOX - 1) / G_BOX, nb = (it.bn + G_BOX - 1) / G_BOX;
         for (int kb = it.kb0; kb < it.kb1 && ok; ++kb) {
           int t = it.g;  // next slice of B
           for (int s = 0; s <= it.g && ok; ++s) {
@@ -705,8 +727,10 @@ __global__ void __launch_bounds__(G_THREADS, 1)
               ok = false;
               break;
             }
-            mftc::mbar_arrive_expect_tx(&fullA[ra.slot], GD_TILE_A);
-            mftc::tma_load_3d(sA + ra.slot * GD_TILE_A, ma, &fullA[ra.slot], kb * BK, it.a_row, s);
+            mftc::mbar_arrive_expect_tx(&fullA[ra.slot], na * G_BOX * BK);
+            for (int b = 0; b < na; ++b)
+              mftc::tma_load_3d(sA + ra.slot * GD_TILE_A + b * G_BOX * BK, ma, &fullA[ra.slot], kb * BK,
+                                it.a_row + b * G_BOX, s);
             armA.arm(ra.slot, ra.phase);
             ra.advance();
             for (; t >= 0 && t > it.g - s - it.nd; --t) {  // up to what step s multiplies
@@ -715,8 +739,10 @@ __global__ void __launch_bounds__(G_THREADS, 1)
                 ok = false;
                 break;
               }
-              mftc::mbar_arrive_expect_tx(&fullB[rb.slot], b_bytes);
-              mftc::tma_load_3d(sB + rb.slot * GD_TILE_B, mb, &fullB[rb.slot], kb * BK, it.b_row, t);
+              mftc::mbar_arrive_expect_tx(&fullB[rb.slot], nb * G_BOX * BK);
+              for (int b = 0; b < nb; ++b)
+                mftc::tma_load_3d(sB + rb.slot * GD_TILE_B + b * G_BOX * BK, mb, &fullB[rb.slot], kb * BK,
+                                  it.b_row + b * G_BOX, t);
               armB.arm(rb.slot, rb.phase);
               rb.advance();
             }
@@ -739,13 +765,14 @@ __global__ void __launch_bounds__(G_THREADS, 1)
           break;
         }
         const int g = work[rw.slot].g, it_nd = work[rw.slot].nd, kb0 = work[rw.slot].kb0, kb1 = work[rw.slot].kb1,
-                  bn = work[rw.slot].bn;
+                  bn = work[rw.slot].bn, klast = work[rw.slot].klast;
         mftc::mbar_arrive(&wempty[rw.slot]);
         rw.advance();
         if (!it_nd) break;
         const uint32_t idesc = mftc::idesc_i8(BM, bn);
         uint32_t accumulate = 0;
         for (int kb = kb0; kb < kb1 && ok; ++kb) {
+          const int ks = kb == kb1 - 1 ? klast : BK / UMMA_K;
           int landed = 0;  // B tiles from rb on known to have landed
           for (int s = 0; s <= g; ++s) {
             const int nd = min(it_nd, g - s + 1);
@@ -774,7 +801,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
               const uint32_t acc = tmem_base + (uint32_t)(d * GD_BN);
 #pragma unroll
               for (int kk = 0; kk < BK / UMMA_K; ++kk)
-                mftc::umma_i8(acc, ad + (uint64_t)(kk * UMMA_K / 16), bd + (uint64_t)(kk * UMMA_K / 16), idesc,
+                if (kk < ks) mftc::umma_i8(acc, ad + (uint64_t)(kk * UMMA_K / 16), bd + (uint64_t)(kk * UMMA_K / 16), idesc,
                               kk == 0 ? accumulate : 1u);
             }
             if (!ok) break;
@@ -808,7 +835,9 @@ __global__ void __launch_bounds__(G_THREADS, 1)
       }
       int32_t *const it_dst = work[rw.slot].dst;
       const int64_t gstride = work[rw.slot].gstride;
-      const int nd = work[rw.slot].nd, bn = work[rw.slot].bn, M_pad = work[rw.slot].M_pad;
+      const int nd = work[rw.slot].nd, M_pad = work[rw.slot].M_pad;
+      // 32-column chunks, every other one this warp's
+      const int nch = quad * 32 < work[rw.slot].rows ? work[rw.slot].bn / 32 : 0;
       __syncwarp();
       if (lane == 0) mftc::mbar_arrive(&wempty[rw.slot]);
       rw.advance();
@@ -820,10 +849,9 @@ __global__ void __launch_bounds__(G_THREADS, 1)
       }
       item_phase ^= 1;
       mftc::tc_fence_after();
-      const int nch = bn / 64, ch0 = half * nch;  // this warp's 32-column chunks
       for (int d = 0; d < nd; ++d) {
-        int32_t *dst = it_dst - d * gstride + (int64_t)ch0 * 32 * M_pad + row;
-        for (int chunk = ch0; chunk < ch0 + nch; ++chunk) {
+        for (int chunk = half; chunk < nch; chunk += 2) {
+          int32_t *dst = it_dst - d * gstride + (int64_t)chunk * 32 * M_pad + row;
           uint32_t r[32];
           mftc::tmem_ld_32x32b_x32(
               tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(d * GD_BN + chunk * 32), r);
@@ -1194,8 +1222,8 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
     const int64_t blocks[PH_COUNT] = {
         P.own_a ? ((P.m + 255) / 256) * ((P.k + 63) / 64) : 0,
         P.own_b && P.k > 0 ? (P.n + 7) / 8 : 0,
-        P.own_a ? (crt ? (P.K_pad * ((P.m + 7) / 8) + 255) / 256 : ((P.m + 31) / 32) * (P.K_pad / 64)) : 0,
-        P.own_b ? (P.n * (P.K_pad / 8) + 255) / 256 : 0,
+        P.own_a ? (crt ? (k_fill(P.k) * ((P.m + 7) / 8) + 255) / 256 : ((P.m + 31) / 32) * ((k_fill(P.k) + 63) / 64)) : 0,
+        P.own_b ? (P.n * (k_fill(P.k) / 8) + 255) / 256 : 0,
         P.mode == 0 ? comb : 0,
         P.mode != 0 ? comb : 0,
         (int64_t)g_groups(P.nsl, crt) * P.nkc * P.ntm * P.ntn};
@@ -1278,8 +1306,8 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
     P.sigB2 = g.plan_b2 >= 0 ? probs[g.plan_b2].sigB : nullptr;
     P.muB2 = g.plan_b2 >= 0 ? probs[g.plan_b2].muB : nullptr;
     if (!(crt ? make_map_mn(&maps[2 * q], P.As, P.M_pad, P.K_pad, P.nsl)
-              : make_map(&maps[2 * q], P.As, P.M_pad, P.K_pad, BM, P.nsl)) ||
-        !make_map(&maps[2 * q + 1], P.Bs, P.N_pad, P.K_pad, (uint32_t)P.bn, P.nsl)) {
+              : make_map(&maps[2 * q], P.As, P.M_pad, P.K_pad, G_BOX, P.nsl)) ||
+        !make_map(&maps[2 * q + 1], P.Bs, P.N_pad, P.K_pad, G_BOX, P.nsl)) {
       destroy(b);
       return MFCUDA_ERR_CUDA;
     }

@@ -75,3 +75,17 @@ def test_many_items(dev):
     for (m, k, n), (a, b), got in list(zip(shapes, host, out))[::7]:
         want, _ = O.split_gemm(a, b, m, k, n, kc=kc)
         assert O.same_bits(got, want).all(), (m, k, n)
+
+
+# where loads, MMAs and drain stop: rows 32 / 64, columns 32 / 64 of a tile, K steps
+# of 32 of the last block; large problems first, so that the rings hold their tiles
+TRIM = [(200, 300, 300), (31, 31, 31), (32, 32, 32), (33, 33, 33), (64, 96, 64), (65, 97, 65), (63, 129, 95),
+        (96, 160, 96), (97, 161, 97), (128, 64, 160), (129, 65, 161), (160, 128, 288), (161, 95, 289), (192, 1, 193)]
+
+
+@pytest.mark.parametrize("form", ["split", "crt"])
+def test_trimmed_tiles(dev, form):
+    host, out, kc = _run(dev, TRIM, form, 0, R=3)
+    for (m, k, n), (a, b), got in zip(TRIM, host, out):
+        want, _ = O.split_gemm(a, b, m, k, n, kc=kc) if form == "split" else O.crt_gemm(a, b, m, k, n)
+        assert O.same_bits(got, want).all(), (m, k, n)
