@@ -357,18 +357,19 @@ __device__ __forceinline__ void slice_a_body(const double *__restrict__ A, int64
   const int64_t i = i0 + ii;
   const bool row_ok = i < M && !flag[i < M ? i : 0];
   const int sigma = i < M ? sig[i] : 0;
-  uint32_t y[8][4];
+  // All entries on their way before the first is rounded (a zero entry has zero
+  // digits, so none needs a branch of its own): waiting for loads was half of the
+  // time between a warp's instructions.  Digits of 2000 problems up to 1024: the whole batch
+  // 10560 -> 10320 us.  The residue slicers gain nothing by it (12740 -> 12770).
+  double2 v[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    int64_t p = p0 + grp * 8 + e;
-    if (row_ok && p < K) {
-      double2 v = __ldg(reinterpret_cast<const double2 *>(A) + (p * M + i) * stride);
-      biased_bytes(v.x, v.y, sigma, W, y[e]);
-    } else {
-#pragma unroll
-      for (int w = 0; w < 4; ++w) y[e][w] = bias_word(w);  // X = 0: all digits zero
-    }
+    const int64_t p = p0 + grp * 8 + e;
+    v[e] = row_ok && p < K ? __ldg(reinterpret_cast<const double2 *>(A) + (p * M + i) * stride) : make_double2(0.0, 0.0);
   }
+  uint32_t y[8][4];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) biased_bytes(v[e].x, v[e].y, sigma, W, y[e]);
   for_each_slice_word(y, S, [&](int sl, uint64_t word) {
     *reinterpret_cast<uint64_t *>(&tile[sl][ii * SA_STRIDE + grp * 8]) = word;
   });
@@ -391,18 +392,15 @@ __device__ __forceinline__ void slice_b_one(const double *__restrict__ B, int64_
   const int S = plan->S, W = plan->W;
   const bool col_ok = j < N && !flag[j < N ? j : 0];
   const int tau = j < N ? sig[j] : 0;
-  uint32_t y[8][4];
+  double2 v[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    int64_t p = p8 + e;
-    if (col_ok && p < K) {
-      double2 v = __ldg(reinterpret_cast<const double2 *>(B) + (j * K + p) * stride);
-      biased_bytes(v.x, v.y, tau, W, y[e]);
-    } else {
-#pragma unroll
-      for (int w = 0; w < 4; ++w) y[e][w] = bias_word(w);
-    }
+    const int64_t p = p8 + e;
+    v[e] = col_ok && p < K ? __ldg(reinterpret_cast<const double2 *>(B) + (j * K + p) * stride) : make_double2(0.0, 0.0);
   }
+  uint32_t y[8][4];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) biased_bytes(v[e].x, v[e].y, tau, W, y[e]);
   for_each_slice_word(y, S, [&](int sl, uint64_t word) {
     *reinterpret_cast<uint64_t *>(Bs + (((int64_t)sl * N_pad + j) * K_pad + p8)) = word;
   });
