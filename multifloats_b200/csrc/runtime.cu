@@ -149,8 +149,20 @@ CtxGetId ctx_get_id() {
   return fn;
 }
 
-// The current context's pool, made on first use; nullptr where there is none
-// (the device's default pool serves then).
+// Making or trimming a pool touches no stream, but a stream capture in its global
+// or thread-local mode refuses such calls and is lost by them.  In the relaxed
+// mode, which is this thread's alone, it allows them.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { exchange(); }
+  ~RelaxedCapture() { exchange(); }
+  void exchange() {
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) (void)cudaGetLastError();
+  }
+};
+
+// The current context's pool, made on first use (which may be inside a stream
+// capture); nullptr where there is none (the device's default pool serves then).
 cudaMemPool_t workspace_pool(bool create) {
   unsigned long long id = 0;
   const CtxGetId fn = ctx_get_id();
@@ -159,6 +171,7 @@ cudaMemPool_t workspace_pool(bool create) {
   for (int i = 0; i < g_npools; ++i)
     if (g_pools[i].ctx == id) return g_pools[i].pool;
   if (!create || g_npools == kMaxPools) return nullptr;
+  RelaxedCapture relaxed;
   int dev = 0;
   cudaMemPool_t pool = nullptr;
   cudaMemPoolProps props = {};
