@@ -252,6 +252,16 @@ MULTIFLOATS_CUDA_API int mfcuda_cmatmuldd_mm_split(const complex64x2 *a, const c
                                                    size_t workspace_bytes, int *info_out,
                                                    void *stream);
 
+/* Device calls given no workspace allocate it on their stream from a pool that
+ * belongs to the library, one per context.  The pool keeps up to 4 GiB of free
+ * memory between calls (what is above goes back at the next synchronisation).
+ * An allocation of the same process that needs this memory gets it; another
+ * process on the GPU cannot have it.  mfcuda_release_workspace gives all that is
+ * free in the pool of the current device back to the system.  What calls still
+ * running use stays, so synchronise their streams first.  Later calls work as
+ * before; the first ones pay for mapping their workspace again. */
+MULTIFLOATS_CUDA_API int mfcuda_release_workspace(void);
+
 /* Phase profiling of the split form for the calling host thread.  Between
  * begin and end, every mfcuda_matmuldd_mm_split / matmuldd_mm_split call
  * records events (owned by the library) on its stream around its phases;

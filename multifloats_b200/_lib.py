@@ -89,6 +89,7 @@ SIGNATURES = {
     "mfcuda_unary_dd_ragged": (C.c_int, [C.c_int, P, P, P, I64, P]),
     "mfcuda_phase_profile_begin": (None, []),
     "mfcuda_phase_profile_end": (C.c_int, [C.POINTER(C.c_double), C.POINTER(I64)]),
+    "mfcuda_release_workspace": (C.c_int, []),
     "mfcuda_set_wait_limit_ns": (C.c_uint64, [C.c_uint64]),
     "mfcuda_shard_bounds": (None, [I64, C.c_int, C.c_int, C.POINTER(I64), C.POINTER(I64)]),
     "mfcuda_nccl_available": (C.c_int, []),

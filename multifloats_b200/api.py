@@ -199,6 +199,13 @@ def cmatmuldd_mm_crt(a, b, m: int, k: int, n: int, bits: int = 0, target: float 
     return _split_call("crt", True, a, b, m, k, n, bits, target, out)
 
 
+def release_workspace():
+    """Gives the free memory of the library's workspace pool on the current
+    device (at most 4 GiB, kept between calls) back to the system.  Synchronise
+    the streams of the calls in question first."""
+    check(lib().mfcuda_release_workspace(), "mfcuda_release_workspace")
+
+
 # ---- batch plans (no reference counterpart) ------------------------------------------
 FORM = {"plain": 0, "split": 1, "crt": 2}
 

@@ -118,8 +118,10 @@ int staging_acquire(Staging &st, const size_t bytes[4]) {
 // workspace again: 1.6 GB at 4096^3, 20 ms on a 2.2 ms product.  The library
 // therefore allocates from a pool of its own that keeps up to kWorkspaceKeep
 // bytes of free memory; what is above that goes back at the next
-// synchronisation, and everything free goes back when one of the library's own
-// allocations fails.  Allocation stays stream-ordered, so any number of threads
+// synchronisation.  A request of this process that needs the free memory gets it
+// (tried with larger workspaces, cudaMalloc, cuMemCreate and the default pool);
+// for other processes mfcuda_release_workspace gives it back.  Allocation stays
+// stream-ordered, so any number of threads
 // and streams may use the pool.  A pool belongs to the context it was made
 // under (contexts are told apart by their id, which is never reused), so one
 // that died with a device reset is never touched again.
@@ -200,17 +202,19 @@ cudaMemPool_t workspace_pool(bool create) {
 }
 }  // namespace
 
-void ws_release_free() {
+static int ws_release_free() {
   if (cudaMemPool_t pool = workspace_pool(false)) {
-    if (cudaMemPoolTrimTo(pool, 0) != cudaSuccess) (void)cudaGetLastError();
+    RelaxedCapture relaxed;
+    MF_TRY_CUDA(cudaMemPoolTrimTo(pool, 0));
   }
+  return MFCUDA_OK;
 }
 
 cudaError_t device_malloc(void **p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation) {  // free workspace memory may be what is missing
     (void)cudaGetLastError();
-    ws_release_free();
+    (void)ws_release_free();
     e = cudaMalloc(p, bytes);
   }
   return e;
@@ -253,6 +257,11 @@ MULTIFLOATS_CUDA_API const char *mfcuda_error_string(int code) {
 }
 
 MULTIFLOATS_CUDA_API const char *mfcuda_version(void) { return "0.1.0"; }
+
+MULTIFLOATS_CUDA_API int mfcuda_release_workspace(void) {
+  MF_TRY(mfcuda::require_device());
+  return mfcuda::ws_release_free();
+}
 
 MULTIFLOATS_CUDA_API uint64_t mfcuda_set_wait_limit_ns(uint64_t ns) {
   return mfcuda::g_wait_limit_ns.exchange(ns);
