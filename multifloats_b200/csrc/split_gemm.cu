@@ -947,13 +947,16 @@ static bool use_pair(int64_t m) {
 // 195, 1500 x 2500 x 700 116 -> 79 (n = 700 pads to 768, not 1024);
 // digit-sliced 1500 x 2500 x 700 378 -> 211.  MFCUDA_SPLIT_NSUB=1 or 2
 // overrides.
-static int pair_nsub(int64_t m, int64_t n, int64_t kblocks, int64_t nkc, int nsl, bool crt) {
-  static const int forced = [] {
+static int forced_nsub() {
+  static const int v = [] {
     const char *e = getenv("MFCUDA_SPLIT_NSUB");
     return e && (e[0] == '1' || e[0] == '2') ? e[0] - '0' : 0;
   }();
+  return v;
+}
+static int pair_nsub(int64_t m, int64_t n, int64_t kblocks, int64_t nkc, int nsl, bool crt) {
   if (n <= BN) return 1;
-  if (forced) return forced;
+  if (const int forced = forced_nsub()) return forced;
   const int64_t pairs = sm_count() / 2, per_tile = (crt ? nsl : (nsl + 1) / 2) * nkc;
   const int64_t ntm = (m + BM_PAIR - 1) / BM_PAIR;
   auto rounds = [&](int64_t cols) { return (per_tile * ntm * ((n + cols - 1) / cols) + pairs - 1) / pairs; };
@@ -961,14 +964,19 @@ static int pair_nsub(int64_t m, int64_t n, int64_t kblocks, int64_t nkc, int nsl
   return rounds(BN) * half < rounds(2 * BN) * 2000 ? 1 : 2;
 }
 
-static Layout layout(int64_t m, int64_t k, int64_t n, int nA, int nB, int nsl = SMAX, bool crt = false) {
+// widest: with two halves wherever the rule may choose two.  Workspace sizes are
+// given for that layout: the rule's choice depends on the device and on rounds of
+// work, so the need of a call is not monotone in its shape, but a workspace of
+// the widest layout serves every shape that is no larger in any extent (the
+// digit-sliced form of 1028 x 97 x 591 wants more than that of 1309 x 97 x 666).
+static Layout layout(int64_t m, int64_t k, int64_t n, int nA, int nB, int nsl, bool crt, bool widest = false) {
   Layout L;
   L.nsl = nsl;
   L.pair = use_pair(m);
   L.K_pad = round_up(k < 1 ? 1 : k, BK);
   L.kblocks = L.K_pad / BK;
   L.nkc = (L.kblocks + KC_BLOCKS - 1) / KC_BLOCKS;
-  L.nsub = L.pair ? pair_nsub(m, n, L.kblocks, L.nkc, nsl, crt) : 1;
+  L.nsub = !L.pair ? 1 : !widest ? pair_nsub(m, n, L.kblocks, L.nkc, nsl, crt) : n > BN && forced_nsub() != 1 ? 2 : 1;
   L.M_pad = round_up(m < 1 ? 1 : m, L.pair ? BM_PAIR : BM);
   L.N_pad = round_up(n < 1 ? 1 : n, BN * L.nsub);
   L.nA = nA;
@@ -1014,12 +1022,13 @@ static bool layout_ok(const Layout &L) {
   return L.M_pad <= INT32_MAX / 2 && L.N_pad <= INT32_MAX / 2 && L.kblocks <= INT32_MAX / 2 && L.N_pad <= 65535 &&
          L.K_pad / 64 <= 65535;
 }
-static Joint joint_layout(int64_t m, int64_t k, int64_t n, int nsl, bool crt) {
+static Joint joint_layout(int64_t m, int64_t k, int64_t n, int nsl, bool crt, bool widest = false) {
   Joint J;
   J.ro = round_up(m, 32);  // row blocks of the reconstruction and of A's slicers
   J.co = round_up(n, 4);   // column quads
-  J.L = layout(J.ro + m, k, J.co + n, 1, 1, nsl, crt);
-  J.ok = layout_ok(J.L) && J.L.total - J.L.off_D <= JOINT_MAX;
+  const Layout W = layout(J.ro + m, k, J.co + n, 1, 1, nsl, crt, true);
+  J.L = widest ? W : layout(J.ro + m, k, J.co + n, 1, 1, nsl, crt);
+  J.ok = layout_ok(W) && W.total - W.off_D <= JOINT_MAX;
   return J;
 }
 
@@ -1129,9 +1138,9 @@ int profile_end(double *sums, int64_t *calls) {
 
 static size_t call_bytes(int64_t m, int64_t k, int64_t n, bool complex_operands, int nsl, bool crt) {
   const int no = complex_operands ? 2 : 1;
-  size_t total = layout(m, k, n, no, no, nsl, crt).total;
+  size_t total = layout(m, k, n, no, no, nsl, crt, true).total;
   if (complex_operands) {
-    const Joint J = joint_layout(m, k, n, nsl, crt);
+    const Joint J = joint_layout(m, k, n, nsl, crt, true);
     if (J.ok) total = std::max(total, J.L.total);
   }
   return total;
