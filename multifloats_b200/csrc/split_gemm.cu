@@ -1145,6 +1145,16 @@ static size_t call_bytes(int64_t m, int64_t k, int64_t n, bool complex_operands,
   }
   return total;
 }
+// What a call takes on this device: the four products of a complex one at once
+// (joint, where the rule allows it), or one at a time.
+static size_t call_need(int64_t m, int64_t k, int64_t n, bool complex_operands, int nsl, bool crt, bool joint) {
+  if (complex_operands && joint) {
+    const Joint J = joint_layout(m, k, n, nsl, crt);
+    if (J.ok) return J.L.total;
+  }
+  const int no = complex_operands ? 2 : 1;
+  return layout(m, k, n, no, no, nsl, crt).total;
+}
 size_t workspace_size(int64_t m, int64_t k, int64_t n, bool complex_operands) {
   return call_bytes(m, k, n, complex_operands, SMAX, false);
 }
@@ -1613,10 +1623,17 @@ static int split_host(const void *a, const void *b, void *c, int64_t m, int64_t 
   if (!c || (k > 0 && (!a || !b))) return MFCUDA_ERR_INVALID_ARG;
   MF_TRY(require_device());
   size_t ba = (size_t)(m * k) * elem, bb = (size_t)(k * n) * elem, bc = (size_t)(m * n) * elem;
-  size_t wsb = split::workspace_size(m, k, n, CPLX);
+  size_t wsb = split::call_need(m, k, n, CPLX, split::SMAX, false, true);
   size_t sz[4] = {ba, bb, bc, wsb};
   Staging st;
-  MF_TRY(staging_acquire(st, sz));
+  int rc = staging_acquire(st, sz);
+  const size_t one = split::call_need(m, k, n, CPLX, split::SMAX, false, false);
+  if (rc == MFCUDA_ERR_ALLOC && one < wsb) {  // no room for the four products at once
+    st = Staging();
+    sz[3] = wsb = one;
+    rc = staging_acquire(st, sz);
+  }
+  MF_TRY(rc);
   if (ba) MF_TRY_CUDA(cudaMemcpyAsync(st.buf[0], a, ba, cudaMemcpyHostToDevice, st.stream));
   if (bb) MF_TRY_CUDA(cudaMemcpyAsync(st.buf[1], b, bb, cudaMemcpyHostToDevice, st.stream));
   int info[3] = {0, 0, 0};
@@ -1681,7 +1698,8 @@ static int crt_host(const void *a, const void *b, void *c, int64_t m, int64_t k,
   if (!c || (k > 0 && (!a || !b))) return MFCUDA_ERR_INVALID_ARG;
   MF_TRY(require_device());
   size_t ba = (size_t)(m * k) * elem, bb = (size_t)(k * n) * elem, bc = (size_t)(m * n) * elem;
-  size_t wsb = split::crt_workspace_size(m, k, n, bits, CPLX);
+  // a call with a sink takes the products one at a time
+  size_t wsb = split::call_need(m, k, n, CPLX, split::crt_slices_max(k, bits), true, false);
   size_t sz[4] = {ba, bb, bc, wsb};
   Staging st;
   MF_TRY(staging_acquire(st, sz));
