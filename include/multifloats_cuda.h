@@ -405,7 +405,8 @@ MULTIFLOATS_CUDA_API int mfcuda_reduce_combine(int kind, const void *parts, int6
  * tune != 0 times the candidate tile shapes of every new shape bucket on
  * synthetic problems and caches the winners in MFCUDA_AUTOTUNE_CACHE (default
  * $HOME/.cache/multifloats_b200/autotune.txt); tune == 0 uses cached winners or
- * a built-in heuristic. */
+ * a built-in heuristic.  Winners that another version of the tiles' kernels was
+ * timed with are ignored. */
 typedef struct mfcuda_gemm_desc {
   const void *a; /* float64x2, column-major m x k */
   const void *b; /* float64x2, column-major k x n */

@@ -1572,6 +1572,10 @@ static int tune_bucket(int form, const Bucket &bk, int64_t ri) {
   return best;
 }
 
+// Part of a winner's key, raised with every change of the tiles' kernels: a winner
+// timed on other kernels says nothing about these (cache files outlive the library
+// that wrote them; entries without this number are from before it was there).
+constexpr int kTuneGeneration = 2;
 static std::string bucket_key(int form, const Bucket &b) {
   char dev[256] = "gpu";
   cudaDeviceProp prop;
@@ -1581,8 +1585,8 @@ static std::string bucket_key(int form, const Bucket &b) {
   for (char *c = dev; *c; ++c)
     if (*c == ' ') *c = '_';
   char key[512];
-  std::snprintf(key, sizeof key, "%s:%s:%d:%d:%d", dev, form == 0 ? "plain" : form == 1 ? "split" : "crt", b.bm,
-                b.bn, b.bk);
+  std::snprintf(key, sizeof key, "%s:%s:%d:%d:%d:g%d", dev, form == 0 ? "plain" : form == 1 ? "split" : "crt", b.bm,
+                b.bn, b.bk, kTuneGeneration);
   return key;
 }
 
