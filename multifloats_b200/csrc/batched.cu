@@ -937,25 +937,27 @@ static int64_t ru(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// Tiles of a plain batch without the tuner: 32 x 32, or 16 x 16 for problems
-// under 24 rows or columns and where one tile's k loop outlasts the batch.  With
+// Tiles of a plain batch: the tuner's winner, or 32 x 32, or 16 x 16 for problems
+// under 24 rows or columns; smaller ones where a tile's k loop outlasts the batch,
+// which the tuner, timing a bucket alone at one k, cannot see.  With
 // two CTAs per SM a tile of 32 costs its SM 0.139 us per step and takes 0.28 us
 // to do one, a tile of 16 0.043 and 0.087 (measured): a problem whose k steps
 // of 0.28 us exceed the whole batch's work spread over the SMs would set the
 // time alone.  Tiles of 64 do the same work 2 % cheaper but take 1.0 us a step:
 // 2000 problems up to 1024 29.1 ms with 64, 29.0 with 32; 30 up to 600 603 us
 // against 222 by this rule, 60 up to 300 308 against 96, 20 up to 200 105
-// against 23.
-constexpr double kStep32 = 0.139, kLatency32 = 0.28;
+// against 23; tuned ones 603 -> 223, 307 -> 102, 105 -> 23.
+constexpr double kStep32 = 0.139, kLatency32 = 0.28, kLatency64 = 1.0;
 static int plain_heuristic(int64_t m, int64_t n) { return std::min(m, n) >= 24 ? 1 : 2; }
-static void plain_small_tiles(const mfcuda_gemm_desc *d, int64_t count, std::vector<int> &cfg,
-                              const std::vector<bool> &tuned) {
+static void plain_small_tiles(const mfcuda_gemm_desc *d, int64_t count, std::vector<int> &cfg) {
   double work = 0.0;
   for (int64_t p = 0; p < count; ++p)
     work += (double)((d[p].m + 31) / 32) * (double)((d[p].n + 31) / 32) * (double)d[p].k * kStep32;
   const double balanced = work / sm_count();
-  for (int64_t p = 0; p < count; ++p)
-    if (!tuned[p] && (double)d[p].k * kLatency32 > balanced) cfg[p] = 2;
+  for (int64_t p = 0; p < count; ++p) {
+    if (cfg[p] == 0 && (double)d[p].k * kLatency64 > balanced) cfg[p] = 1;
+    if (cfg[p] == 1 && (double)d[p].k * kLatency32 > balanced) cfg[p] = 2;
+  }
 }
 
 // Plan memory: one device allocation holding the tables and the workspace.
@@ -1629,19 +1631,17 @@ static std::vector<int> choose(int form, const mfcuda_gemm_desc *d, int64_t coun
     }
     if (dirty) tune_save();
   }
-  std::vector<bool> tuned(count, false);
   for (int64_t p = 0; p < count; ++p) {
     auto it = win.find(bucket_of(d[p]));
     if (it != win.end()) {
       cfg[p] = it->second;
-      tuned[p] = true;
     } else if (form == 0) {
       cfg[p] = plain_heuristic(d[p].m, d[p].n);
     } else {
       cfg[p] = d[p].n <= 64 ? 64 : d[p].n <= 128 ? 128 : 256;
     }
   }
-  if (form == 0) plain_small_tiles(d, count, cfg, tuned);
+  if (form == 0) plain_small_tiles(d, count, cfg);
   return cfg;
 }
 

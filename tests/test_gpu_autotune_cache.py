@@ -55,3 +55,15 @@ def test_former_winners_are_ignored(dev, tmp_path, form, shape, stored, reported
     assert _config(planted, form, shape) == heuristic
     _config(planted, form, shape, tune=True)
     assert set(_entries(planted)) == {key, former}
+
+
+@pytest.mark.parametrize("stored", ["0", "1"])
+def test_winner_whose_tiles_outlast_the_batch(dev, tmp_path, stored):
+    """Two products of 100 x 2000 x 100: a tile of 64 or 32 runs its k loop alone
+    when the SMs have long finished the rest, whatever won for the bucket."""
+    fresh, planted = tmp_path / "fresh.txt", tmp_path / "planted.txt"
+    shape = (100, 2000, 100, 2)
+    _config(fresh, "plain", shape, tune=True)
+    (key, _), = _entries(fresh).items()
+    planted.write_text(f"{key} {stored}\n")
+    assert _config(planted, "plain", shape) == _config(tmp_path / "none.txt", "plain", shape) == 16
