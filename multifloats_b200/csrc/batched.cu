@@ -65,7 +65,7 @@ struct PItem {
 constexpr int kPlainCfgs = 3;  // 0: 64x64 (4x4 per thread), 1: 32x32 (2x2), 2: 16x16 (1x1)
 static int cfg_edge(int cfg) { return cfg == 0 ? 64 : cfg == 1 ? 32 : 16; }
 
-template <bool ALIGNED>
+template <bool ALIGNED, bool SHORT>
 __global__ void __launch_bounds__(256, 2)
     plain_grouped_kernel(const PProb *__restrict__ probs, const PItem *__restrict__ items, int nitems,
                          int64_t ri, int *counter) {
@@ -81,16 +81,16 @@ __global__ void __launch_bounds__(256, 2)
     const PProb p = probs[it.prob];
     switch (it.cfg) {
       case 0:
-        gtile::gemm_tile<4, 4, ALIGNED>(p.A, p.B, p.C, p.m, p.k, p.n, ri, (int64_t)it.tm * 64,
-                                        (int64_t)it.tn * 64, sm);
+        gtile::gemm_tile<4, 4, ALIGNED, SHORT>(p.A, p.B, p.C, p.m, p.k, p.n, ri, (int64_t)it.tm * 64,
+                                               (int64_t)it.tn * 64, sm);
         break;
       case 1:
-        gtile::gemm_tile<2, 2, ALIGNED>(p.A, p.B, p.C, p.m, p.k, p.n, ri, (int64_t)it.tm * 32,
-                                        (int64_t)it.tn * 32, sm);
+        gtile::gemm_tile<2, 2, ALIGNED, SHORT>(p.A, p.B, p.C, p.m, p.k, p.n, ri, (int64_t)it.tm * 32,
+                                               (int64_t)it.tn * 32, sm);
         break;
       default:
-        gtile::gemm_tile<1, 1, ALIGNED>(p.A, p.B, p.C, p.m, p.k, p.n, ri, (int64_t)it.tm * 16,
-                                        (int64_t)it.tn * 16, sm);
+        gtile::gemm_tile<1, 1, ALIGNED, SHORT>(p.A, p.B, p.C, p.m, p.k, p.n, ri, (int64_t)it.tm * 16,
+                                               (int64_t)it.tn * 16, sm);
         break;
     }
   }
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(256, 2)
 
 // Complex problems (complex64x2): every 32 x 32 output tile runs the
 // single-problem complex tile code (gtile::cgemm_tile).
-template <bool ALIGNED>
+template <bool ALIGNED, bool SHORT>
 __global__ void __launch_bounds__(256, 2)
     cplain_grouped_kernel(const PProb *__restrict__ probs, const PItem *__restrict__ items, int nitems,
                           int64_t ri, int *counter) {
@@ -112,7 +112,8 @@ __global__ void __launch_bounds__(256, 2)
     if (w >= nitems) break;
     const PItem it = items[w];
     const PProb p = probs[it.prob];
-    gtile::cgemm_tile<2, 2, ALIGNED>(p.A, p.B, p.C, p.m, p.k, p.n, ri, (int64_t)it.tm * 32, (int64_t)it.tn * 32, sm);
+    gtile::cgemm_tile<2, 2, ALIGNED, SHORT>(p.A, p.B, p.C, p.m, p.k, p.n, ri, (int64_t)it.tm * 32,
+                                            (int64_t)it.tn * 32, sm);
   }
 }
 
@@ -1073,18 +1074,16 @@ static int create_plain(const mfcuda_gemm_desc *d, int64_t count, int64_t ri, co
   const int nitems = (int)items.size();
   int grid = sm_count() * 2;
   if (grid > nitems) grid = nitems > 0 ? nitems : 1;
+  auto pick = [&](auto al, auto sh) {
+    return complex ? cplain_grouped_kernel<al, sh> : plain_grouped_kernel<al, sh>;
+  };
+  const std::true_type yes;
+  const std::false_type no;
+  const bool sh = gtile::short_interval(ri);
+  auto *kernel = aligned ? (sh ? pick(yes, yes) : pick(yes, no)) : sh ? pick(no, yes) : pick(no, no);
   int rc = capture(b, [&](cudaStream_t cs) {
     cudaMemsetAsync(ctr, 0, sizeof(int), cs);
-    if (complex) {
-      if (aligned)
-        cplain_grouped_kernel<true><<<grid, 256, 0, cs>>>(dp, di, nitems, ri, ctr);
-      else
-        cplain_grouped_kernel<false><<<grid, 256, 0, cs>>>(dp, di, nitems, ri, ctr);
-    } else if (aligned) {
-      plain_grouped_kernel<true><<<grid, 256, 0, cs>>>(dp, di, nitems, ri, ctr);
-    } else {
-      plain_grouped_kernel<false><<<grid, 256, 0, cs>>>(dp, di, nitems, ri, ctr);
-    }
+    kernel<<<grid, 256, 0, cs>>>(dp, di, nitems, ri, ctr);
   });
   if (rc != MFCUDA_OK) {
     destroy(b);

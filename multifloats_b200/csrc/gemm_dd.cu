@@ -99,7 +99,7 @@ __device__ __forceinline__ void piece_origin(int q, int side, int E, int64_t &m0
 // Real GEMM.  Mixed: blocks 0 .. whole - 1 own a 64 x 64 tile (4 x 4 outputs
 // per thread), the others a piece of the tiles after those.
 // ---------------------------------------------------------------------------
-template <bool ALIGNED>
+template <bool ALIGNED, bool SHORT>
 __global__ void __launch_bounds__(kThreads, 2)
     gemm_dd_kernel(const double *__restrict__ A, const double *__restrict__ B,
                    double *__restrict__ C, int64_t M, int64_t K, int64_t N, int64_t ri,
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   int64_t b = blockIdx.x, m0, n0;
   if (b < whole) {
     tile_origin(b, gx, 64, m0, n0);
-    gtile::gemm_tile<4, 4, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+    gtile::gemm_tile<4, 4, ALIGNED, SHORT>(A, B, C, M, K, N, ri, m0, n0, sm);
     return;
   }
   b -= whole;
@@ -117,27 +117,27 @@ __global__ void __launch_bounds__(kThreads, 2)
   tile_origin(whole + b / cut, gx, 64, m0, n0);
   if (cut == 4) {
     piece_origin(q, 2, 32, m0, n0);
-    if (m0 < M && n0 < N) gtile::gemm_tile<2, 2, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+    if (m0 < M && n0 < N) gtile::gemm_tile<2, 2, ALIGNED, SHORT>(A, B, C, M, K, N, ri, m0, n0, sm);
   } else {
     piece_origin(q, 4, 16, m0, n0);
-    if (m0 < M && n0 < N) gtile::gemm_tile<1, 1, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+    if (m0 < M && n0 < N) gtile::gemm_tile<1, 1, ALIGNED, SHORT>(A, B, C, M, K, N, ri, m0, n0, sm);
   }
 }
 // Uniform tiles of edge 16 T (three CTAs of edge 32 per SM, four of edge 16).
-template <int T, bool ALIGNED>
+template <int T, bool ALIGNED, bool SHORT>
 __global__ void __launch_bounds__(kThreads, T == 2 ? 3 : 4)
     gemm_dd_small_kernel(const double *__restrict__ A, const double *__restrict__ B,
                          double *__restrict__ C, int64_t M, int64_t K, int64_t N, int64_t ri) {
   __shared__ gtile::Smem sm;
   int64_t m0, n0;
   tile_origin(blockIdx.x, (M + 16 * T - 1) / (16 * T), 16 * T, m0, n0);
-  gtile::gemm_tile<T, T, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+  gtile::gemm_tile<T, T, ALIGNED, SHORT>(A, B, C, M, K, N, ri, m0, n0, sm);
 }
 
 // ---------------------------------------------------------------------------
 // Complex GEMM (gtile::cgemm_tile): the same with tiles of 32 and 16.
 // ---------------------------------------------------------------------------
-template <bool ALIGNED>
+template <bool ALIGNED, bool SHORT>
 __global__ void __launch_bounds__(kThreads, 2)
     cgemm_dd_kernel(const double *__restrict__ A, const double *__restrict__ B,
                     double *__restrict__ C, int64_t M, int64_t K, int64_t N, int64_t ri,
@@ -147,22 +147,22 @@ __global__ void __launch_bounds__(kThreads, 2)
   int64_t b = blockIdx.x, m0, n0;
   if (b < whole) {
     tile_origin(b, gx, 32, m0, n0);
-    gtile::cgemm_tile<2, 2, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+    gtile::cgemm_tile<2, 2, ALIGNED, SHORT>(A, B, C, M, K, N, ri, m0, n0, sm);
     return;
   }
   b -= whole;
   tile_origin(whole + b / cut, gx, 32, m0, n0);
   piece_origin((int)(b % cut), 2, 16, m0, n0);
-  if (m0 < M && n0 < N) gtile::cgemm_tile<1, 1, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+  if (m0 < M && n0 < N) gtile::cgemm_tile<1, 1, ALIGNED, SHORT>(A, B, C, M, K, N, ri, m0, n0, sm);
 }
-template <bool ALIGNED>
+template <bool ALIGNED, bool SHORT>
 __global__ void __launch_bounds__(kThreads, 4)
     cgemm_dd_small_kernel(const double *__restrict__ A, const double *__restrict__ B,
                           double *__restrict__ C, int64_t M, int64_t K, int64_t N, int64_t ri) {
   __shared__ gtile::CSmem sm;
   int64_t m0, n0;
   tile_origin(blockIdx.x, (M + 15) / 16, 16, m0, n0);
-  gtile::cgemm_tile<1, 1, ALIGNED>(A, B, C, M, K, N, ri, m0, n0, sm);
+  gtile::cgemm_tile<1, 1, ALIGNED, SHORT>(A, B, C, M, K, N, ri, m0, n0, sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -427,25 +427,25 @@ static int zero_fill(double *p, int64_t ndoubles, cudaStream_t s) {
   return MFCUDA_OK;
 }
 
-template <bool ALIGNED>
+template <bool ALIGNED, bool SHORT>
 static void launch_gemm(const TilePick &p, const double *A, const double *B, double *C, int64_t m, int64_t k,
                         int64_t n, int64_t ri, cudaStream_t s) {
   const unsigned g = (unsigned)p.blocks;
   if (p.edge == 64)
-    gemm_dd_kernel<ALIGNED><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri, p.cut ? p.whole : p.blocks, p.cut);
+    gemm_dd_kernel<ALIGNED, SHORT><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri, p.cut ? p.whole : p.blocks, p.cut);
   else if (p.edge == 32)
-    gemm_dd_small_kernel<2, ALIGNED><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
+    gemm_dd_small_kernel<2, ALIGNED, SHORT><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
   else
-    gemm_dd_small_kernel<1, ALIGNED><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
+    gemm_dd_small_kernel<1, ALIGNED, SHORT><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
 }
-template <bool ALIGNED>
+template <bool ALIGNED, bool SHORT>
 static void launch_cgemm(const TilePick &p, const double *A, const double *B, double *C, int64_t m, int64_t k,
                          int64_t n, int64_t ri, cudaStream_t s) {
   const unsigned g = (unsigned)p.blocks;
   if (p.edge == 32)
-    cgemm_dd_kernel<ALIGNED><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri, p.cut ? p.whole : p.blocks, p.cut);
+    cgemm_dd_kernel<ALIGNED, SHORT><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri, p.cut ? p.whole : p.blocks, p.cut);
   else
-    cgemm_dd_small_kernel<ALIGNED><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
+    cgemm_dd_small_kernel<ALIGNED, SHORT><<<g, kThreads, 0, s>>>(A, B, C, m, k, n, ri);
 }
 
 int gemm_dev(const float64x2 *a, const float64x2 *b, float64x2 *c, int64_t m, int64_t k,
@@ -461,10 +461,11 @@ int gemm_dev(const float64x2 *a, const float64x2 *b, float64x2 *c, int64_t m, in
   if ((n + 63) / 64 > 65535) return MFCUDA_ERR_UNSUPPORTED;
   const TilePick p = pick_tiles(m, n, kRealCost, 3, kRealCutCost);
   if (p.blocks <= 0 || p.blocks > INT32_MAX) return MFCUDA_ERR_UNSUPPORTED;
+  const bool sh = gtile::short_interval(ri);
   if (aligned16(a, b, c))
-    launch_gemm<true>(p, A, B, C, m, k, n, ri, s);
+    (sh ? launch_gemm<true, true> : launch_gemm<true, false>)(p, A, B, C, m, k, n, ri, s);
   else
-    launch_gemm<false>(p, A, B, C, m, k, n, ri, s);
+    (sh ? launch_gemm<false, true> : launch_gemm<false, false>)(p, A, B, C, m, k, n, ri, s);
   MF_TRY_CUDA(cudaGetLastError());
   return MFCUDA_OK;
 }
@@ -482,10 +483,11 @@ int cgemm_dev(const complex64x2 *a, const complex64x2 *b, complex64x2 *c, int64_
   if ((n + 31) / 32 > 65535) return MFCUDA_ERR_UNSUPPORTED;
   const TilePick p = pick_tiles(m, n, kCplxCost, 2, kCplxCutCost);
   if (p.blocks <= 0 || p.blocks > INT32_MAX) return MFCUDA_ERR_UNSUPPORTED;
+  const bool sh = gtile::short_interval(ri);
   if (aligned16(a, b, c))
-    launch_cgemm<true>(p, A, B, C, m, k, n, ri, s);
+    (sh ? launch_cgemm<true, true> : launch_cgemm<true, false>)(p, A, B, C, m, k, n, ri, s);
   else
-    launch_cgemm<false>(p, A, B, C, m, k, n, ri, s);
+    (sh ? launch_cgemm<false, true> : launch_cgemm<false, false>)(p, A, B, C, m, k, n, ri, s);
   MF_TRY_CUDA(cudaGetLastError());
   return MFCUDA_OK;
 }

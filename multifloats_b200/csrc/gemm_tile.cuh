@@ -16,7 +16,7 @@
 // registers at each merge, and the moves that took (8 of 26 issue cycles per
 // MAC) were paid on top of the FP64 issue -- 4096^3 66.6 -> 56.8 ms, FP64 pipe
 // 88 % busy.  An interval that is not a multiple of eight runs from chunk end
-// to chunk end in a counted loop.
+// to chunk end in a counted loop; the shortest ones have kernels of their own.
 #pragma once
 #include "dd_device.cuh"
 
@@ -83,9 +83,25 @@ struct Cadence {
     cnt = 0;
     return true;
   }
+  // one more MAC done, interval known to be positive: does a chunk end here?
+  __device__ __forceinline__ bool step_ends() {
+    const bool end = ++cnt == ri;
+    if (end) cnt = 0;
+    return end;
+  }
 };
+// Intervals of up to three steps have kernels of their own (SHORT): their chunks are
+// too short for a counted loop each.  Real tiles of 32 and 16 and complex ones of 16
+// test the chunk counter after every step of an unrolled group, complex tiles of 32
+// renormalise without a test where the interval is one.  Counted loops -> these, us:
+// 777 x 333 x 555 interval 1 376 -> 232, 2 261 -> 220; 256^3 interval 1 64 -> 35, 3
+// 39 -> 33; complex batches interval 1 a fifth less.  With four steps
+// and more the test costs the tiles of 32 up to 15 %; in the same kernel as the
+// longer intervals this code cost those up to 5 %.
+constexpr int kShort = 3;
+inline bool short_interval(int64_t ri) { return ri > 0 && ri <= kShort; }
 
-template <int TM, int TN, bool ALIGNED>
+template <int TM, int TN, bool ALIGNED, bool SHORT>
 __device__ __forceinline__ void gemm_tile(const double *__restrict__ A, const double *__restrict__ B,
                                           double *__restrict__ C, int64_t M, int64_t K, int64_t N,
                                           int64_t ri, int64_t m0, int64_t n0, Smem &sm) {
@@ -155,7 +171,16 @@ __device__ __forceinline__ void gemm_tile(const double *__restrict__ A, const do
     const int kmax = (K - k0) < BK ? (int)(K - k0) : BK;
     const double2 *as = sm.A[stage] + tx, *bs = sm.B[stage] + ty;
     int kk = 0;
-    if (cad.grouped) {
+    if constexpr (SHORT && TM * TN < 16) {  // whole groups with more steps after them
+#pragma unroll 1
+      for (; kk + kGroup <= kmax && k0 + kk + kGroup < K; kk += kGroup) {
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) {
+          step(as + (kk + u) * BM, bs + (kk + u) * PB);
+          if (cad.step_ends()) renorm_all();
+        }
+      }
+    } else if (!SHORT && cad.grouped) {
 #pragma unroll 1
       for (; kk + kGroup <= kmax; kk += kGroup) {
 #pragma unroll
@@ -208,7 +233,7 @@ struct CSmem {
   double2 B[2][2 * depth(32) * b_pitch(16)];
 };
 
-template <int TM, int TN, bool ALIGNED>
+template <int TM, int TN, bool ALIGNED, bool SHORT>
 __device__ __forceinline__ void cgemm_tile(const double *__restrict__ A, const double *__restrict__ B,
                                            double *__restrict__ C, int64_t M, int64_t K, int64_t N,
                                            int64_t ri, int64_t m0, int64_t n0, CSmem &sm) {
@@ -288,7 +313,25 @@ __device__ __forceinline__ void cgemm_tile(const double *__restrict__ A, const d
     const int kmax = (K - k0) < BK ? (int)(K - k0) : BK;
     const double2 *as = sm.A[stage] + 2 * tx, *bs = sm.B[stage] + 2 * ty;
     int kk = 0;
-    if (cad.grouped) {
+    if constexpr (SHORT && TM * TN >= 4) {
+      if (ri == 1) {
+        const int each = K - 1 - k0 < kmax ? (int)(K - 1 - k0) : kmax;  // steps with more after them
+#pragma unroll 2
+        for (; kk < each; ++kk) {
+          step(as + 2 * kk * BM, bs + 2 * kk * PB);
+          renorm_all();
+        }
+      }
+    } else if constexpr (SHORT) {  // whole groups with more steps after them
+#pragma unroll 1
+      for (; kk + kGroup <= kmax && k0 + kk + kGroup < K; kk += kGroup) {
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) {
+          step(as + 2 * (kk + u) * BM, bs + 2 * (kk + u) * PB);
+          if (cad.step_ends()) renorm_all();
+        }
+      }
+    } else if (!SHORT && cad.grouped) {
 #pragma unroll 1
       for (; kk + kGroup <= kmax; kk += kGroup) {
 #pragma unroll
