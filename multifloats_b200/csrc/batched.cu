@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(CTC_THREADS, 4) g_crt_combine(const SProb *pro
 // one: finding an item's problem by bisection and walking to its plan was a
 // dozen dependent loads per role and item, about 10 of the 13 us an item took.
 struct __align__(16) GItem {
-  int p;           // problem (tensor maps 2 p, 2 p + 1)
+  int p;           // problem (its tensor maps)
   int g, nd;       // digits: diagonals g, g - 1, ... (nd of them); CRT: modulus g, nd = 1; nd = 0: beyond the plan
   int kb0, kb1;    // K blocks
   int a_row, b_row;  // first row of A and column of B
@@ -377,6 +377,23 @@ __device__ __forceinline__ GItem load_item(const GItem *items, int64_t w, int64_
 // 1024 digits 10950 -> 10560, CRT 13760 -> 12690; 300 up to 256 330 -> 313, 514 ->
 // 448; 1000 up to 64 458 -> 442, 708 -> 553.
 constexpr int G_BOX = 64;
+// Tensor maps of a problem.  CRT: A (boxes of 128 rows), B (boxes of G_BOX columns).
+// Digits: boxes of 128 rows and of G_BOX for A, of G_BOX, 128 and 256 columns for B,
+// and a tile is loaded in as few as there are for it: a box costs the copy engine as
+// much as its bytes where one CTA's loads are the bound (100 x 500 x 200, 14 items:
+// 46 us in boxes of 64, 38 so).  The CRT form's items are short and gain nothing
+// (1000 products up to 64: 566 -> 576 us with the choice).
+enum { GM_A, GM_B, GM_CRT, GM_A_BOX = GM_CRT, GM_B128, GM_B256, GM_COUNT };
+// nb G_BOX columns of B (1 <= nb <= 4) from column b_row on.
+__device__ __forceinline__ void load_b(uint8_t *dst, const CUtensorMap *m, uint64_t *bar, int nb, int k, int b_row,
+                                       int slice) {
+  if (nb == 4) {
+    mftc::tma_load_3d(dst, m + GM_B256, bar, k, b_row, slice);
+    return;
+  }
+  if (nb >= 2) mftc::tma_load_3d(dst, m + GM_B128, bar, k, b_row, slice);
+  if (nb & 1) mftc::tma_load_3d(dst + (nb - 1) * G_BOX * BK, m + GM_B, bar, k, b_row + (nb - 1) * G_BOX, slice);
+}
 // Diagonals of an item of the digit-sliced form.
 constexpr int GD_DIAGS = 2;
 __host__ __device__ constexpr int g_groups(int nsl, bool crt) { return crt ? nsl : (nsl + GD_DIAGS - 1) / GD_DIAGS; }
@@ -477,9 +494,9 @@ __global__ void __launch_bounds__(G_THREADS, 1)
           }
           mftc::mbar_arrive_expect_tx(&full[stage], bytes);
           // A: MN-major residue planes (row, K index, modulus)
-          mftc::tma_load_3d(sA + stage * A_STAGE, &maps[2 * it.p], &full[stage], it.a_row, kb * BK, it.g);
+          mftc::tma_load_3d(sA + stage * A_STAGE, &maps[GM_CRT * it.p + GM_A], &full[stage], it.a_row, kb * BK, it.g);
           for (int b = 0; b < nb; ++b)
-            mftc::tma_load_3d(sB + stage * B_STAGE + b * G_BOX * BK, &maps[2 * it.p + 1], &full[stage], kb * BK,
+            mftc::tma_load_3d(sB + stage * B_STAGE + b * G_BOX * BK, &maps[GM_CRT * it.p + GM_B], &full[stage], kb * BK,
                               it.b_row + b * G_BOX, it.g);
           arm.arm(stage, phase);
           if (++stage == NSTAGE) {
@@ -603,8 +620,12 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 // K chunk, accumulated side by side in tensor memory.  Per K block the slices
 // come in the order A_0, B_g, B_{g-1}, A_1, B_{g-2}, ...: step s multiplies A_s
 // with B_{g-s} and B_{g-s-1}, one product per diagonal, and then lets A_s and
-// B_{g-s} go, so each slice is loaded once for both diagonals.  A and B have
-// rings of their own because a step holds two B tiles but one A tile.
+// B_{g-s} go, so each slice is loaded once for both diagonals.  B has more slots
+// than A because a step holds two B tiles but one A tile; as every step takes one
+// of each and frees one of each, the n-th tiles of both belong together: one
+// barrier says that what steps up to n multiply has landed (A_n and the B tiles
+// loaded with it, one ahead), one that the n-th tile of both is free, which with
+// one slot of B more also frees the one ahead.
 //
 // CTAs take items from a counter (the producer does, one item ahead, and hands
 // each to the other roles through a small ring in shared memory): dealt round
@@ -617,11 +638,15 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 // diagonals on 128 x 128 tiles load less, but a 128-column MMA takes 102 cycles
 // instead of its 64 (shared-memory reads).  2000 products of sizes up to 1024:
 // 9.0 ms with one diagonal at a time and items found by bisection, 7.8 four by
-// 128 columns, 6.0 two by 256.
+// 128 columns, 6.0 two by 256.  With barriers and commits of their own for A and B
+// a step cost 0.2 us more (the second commit waits for the tensor pipe once again):
+// the 2000 products, whole batch, 10.26 -> 9.18 ms with one; 100 x 500 x 200 alone,
+// this kernel, 52 -> 41 us.
 constexpr int GD_BN = BN, GD_NA = 4, GD_NB = 5, GD_NW = 4;
 constexpr int GD_TILE_A = A_STAGE, GD_TILE_B = B_STAGE;  // bytes of a slot
 constexpr int GD_SMEM = GD_NA * GD_TILE_A + GD_NB * GD_TILE_B + 1024 /*align*/ + 512 /*barriers, items*/;
-static_assert(GD_DIAGS * GD_BN == TMEM_COLS && GD_NB > GD_DIAGS, "accumulators fill tensor memory");
+static_assert(GD_DIAGS * GD_BN == TMEM_COLS, "accumulators fill tensor memory");
+static_assert(GD_NB >= GD_NA + GD_DIAGS - 1, "a free step of A means free slots of B");
 
 // Position in a ring of N slots and the parity of its current pass.
 template <int N>
@@ -635,7 +660,6 @@ struct RingPos {
     }
   }
   __device__ __forceinline__ int at(int d) const { return slot + d < N ? slot + d : slot + d - N; }
-  __device__ __forceinline__ uint32_t phase_at(int d) const { return slot + d < N ? phase : phase ^ 1; }
 };
 
 __global__ void __launch_bounds__(G_THREADS, 1)
@@ -644,11 +668,9 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t *sA = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t *sB = sA + GD_NA * GD_TILE_A;
-  uint64_t *fullA = reinterpret_cast<uint64_t *>(sB + GD_NB * GD_TILE_B);
-  uint64_t *emptyA = fullA + GD_NA;
-  uint64_t *fullB = emptyA + GD_NA;
-  uint64_t *emptyB = fullB + GD_NB;
-  uint64_t *tempty = emptyB + GD_NB;    // per accumulator
+  uint64_t *full = reinterpret_cast<uint64_t *>(sB + GD_NB * GD_TILE_B);
+  uint64_t *empty = full + GD_NA;
+  uint64_t *tempty = empty + GD_NA;     // per accumulator
   uint64_t *tfull = tempty + GD_DIAGS;  // the item's accumulators
   uint64_t *wfull = tfull + 1;  // the ring of items
   uint64_t *wempty = wfull + GD_NW;
@@ -660,12 +682,8 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < GD_NA; ++s) {
-      mftc::mbar_init(&fullA[s], 1);
-      mftc::mbar_init(&emptyA[s], 1);
-    }
-    for (int s = 0; s < GD_NB; ++s) {
-      mftc::mbar_init(&fullB[s], 1);
-      mftc::mbar_init(&emptyB[s], 1);
+      mftc::mbar_init(&full[s], 1);
+      mftc::mbar_init(&empty[s], 1);
     }
     for (int d = 0; d < GD_DIAGS; ++d) mftc::mbar_init(&tempty[d], G_EPI_WARPS);
     mftc::mbar_init(tfull, 1);
@@ -689,10 +707,8 @@ __global__ void __launch_bounds__(G_THREADS, 1)
     *abort_flag = 1;
     record_abort(status, code);
   };
-  ArmedStages<GD_NA> armA;  // the producer's armed slots
-  ArmedStages<GD_NB> armB;
-  armA.clear();
-  armB.clear();
+  ArmedStages<GD_NA> arm;  // the producer's armed steps
+  arm.clear();
 
   if (warp == 0) {
     if (lane == 0) {  // ---- TMA producer
@@ -718,35 +734,26 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         mftc::mbar_arrive(&wfull[rw.slot]);
         rw.advance();
         if (end) break;
-        const CUtensorMap *ma = &maps[2 * it.p], *mb = ma + 1;
+        const CUtensorMap *m = &maps[GM_COUNT * it.p];
         const int na = (it.rows + G_BOX - 1) / G_BOX, nb = (it.bn + G_BOX - 1) / G_BOX;
         for (int kb = it.kb0; kb < it.kb1 && ok; ++kb) {
           int t = it.g;  // next slice of B
-          for (int s = 0; s <= it.g && ok; ++s) {
-            if (!wait_bar(&emptyA[ra.slot], ra.phase ^ 1, abort_flag, wait_ns)) {
+          for (int s = 0; s <= it.g; ++s) {
+            if (!wait_bar(&empty[ra.slot], ra.phase ^ 1, abort_flag, wait_ns)) {
               fail(1);
               ok = false;
               break;
             }
-            mftc::mbar_arrive_expect_tx(&fullA[ra.slot], na * G_BOX * BK);
-            for (int b = 0; b < na; ++b)
-              mftc::tma_load_3d(sA + ra.slot * GD_TILE_A + b * G_BOX * BK, ma, &fullA[ra.slot], kb * BK,
-                                it.a_row + b * G_BOX, s);
-            armA.arm(ra.slot, ra.phase);
-            ra.advance();
-            for (; t >= 0 && t > it.g - s - it.nd; --t) {  // up to what step s multiplies
-              if (!wait_bar(&emptyB[rb.slot], rb.phase ^ 1, abort_flag, wait_ns)) {
-                fail(1);
-                ok = false;
-                break;
-              }
-              mftc::mbar_arrive_expect_tx(&fullB[rb.slot], nb * G_BOX * BK);
-              for (int b = 0; b < nb; ++b)
-                mftc::tma_load_3d(sB + rb.slot * GD_TILE_B + b * G_BOX * BK, mb, &fullB[rb.slot], kb * BK,
-                                  it.b_row + b * G_BOX, t);
-              armB.arm(rb.slot, rb.phase);
+            const int upto = max(it.g - s - it.nd + 1, 0);  // the last slice of B that step s multiplies
+            mftc::mbar_arrive_expect_tx(&full[ra.slot], (uint32_t)((na + (t - upto + 1) * nb) * G_BOX * BK));
+            mftc::tma_load_3d(sA + ra.slot * GD_TILE_A, m + (na == 1 ? GM_A_BOX : GM_A), &full[ra.slot], kb * BK,
+                              it.a_row, s);
+            for (; t >= upto; --t) {
+              load_b(sB + rb.slot * GD_TILE_B, m, &full[ra.slot], nb, kb * BK, it.b_row, t);
               rb.advance();
             }
+            arm.arm(ra.slot, ra.phase);
+            ra.advance();
           }
         }
       }
@@ -774,14 +781,11 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         uint32_t accumulate = 0;
         for (int kb = kb0; kb < kb1 && ok; ++kb) {
           const int ks = kb == kb1 - 1 ? klast : BK / UMMA_K;
-          int landed = 0;  // B tiles from rb on known to have landed
           for (int s = 0; s <= g; ++s) {
             const int nd = min(it_nd, g - s + 1);
-            ok = wait_bar(&fullA[ra.slot], ra.phase, abort_flag, wait_ns);
-            for (; ok && landed < nd; ++landed)
-              ok = wait_bar(&fullB[rb.at(landed)], rb.phase_at(landed), abort_flag, wait_ns);
-            if (!ok) {
+            if (!wait_bar(&full[ra.slot], ra.phase, abort_flag, wait_ns)) {
               fail(4);
+              ok = false;
               break;
             }
             mftc::tc_fence_after();
@@ -807,11 +811,9 @@ __global__ void __launch_bounds__(G_THREADS, 1)
             }
             if (!ok) break;
             accumulate = 1;
-            mftc::umma_commit(&emptyA[ra.slot]);
-            mftc::umma_commit(&emptyB[rb.slot]);
+            mftc::umma_commit(&empty[ra.slot]);
             ra.advance();
             rb.advance();
-            --landed;
           }
         }
         if (!ok) break;
@@ -874,10 +876,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   mftc::tc_fence_after();
   if (*abort_flag) {  // read after the barrier: the same value in every thread
     // copies in flight that no MMA consumed land before shared memory is released
-    if (warp == 0 && lane == 0) {
-      armA.drain(fullA, GD_NA);
-      armB.drain(fullB, GD_NB);
-    }
+    if (warp == 0 && lane == 0) arm.drain(full, GD_NA);
     __syncthreads();
   }
   if (warp == 1) {
@@ -1167,7 +1166,8 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
   Arena ar;
   size_t o_probs = ar.take(sizeof(SProb) * std::max(np, 1));
   size_t o_prefix = ar.take(sizeof(int64_t) * std::max(np, 1));
-  size_t o_maps = ar.take(sizeof(CUtensorMap) * 2 * std::max(np, 1), 128);
+  const size_t nmaps = crt ? GM_CRT : GM_COUNT;  // per problem
+  size_t o_maps = ar.take(sizeof(CUtensorMap) * nmaps * std::max(np, 1), 128);
   size_t o_status = ar.take(2 * sizeof(int));  // abort codes, the digit kernel's item counter
   std::vector<size_t> o_plan(np, 0), o_cc(np, 0), o_as(np, 0), o_bs(np, 0), o_d(np);
   std::vector<int64_t> rowA(np, -1), rowB(np, -1);  // statistics rows of owned operands
@@ -1280,7 +1280,7 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
     }
     P.D = reinterpret_cast<int32_t *>(base + o_d[q]);
   }
-  std::vector<CUtensorMap> maps(2 * (size_t)std::max(np, 1));
+  std::vector<CUtensorMap> maps(nmaps * std::max(np, 1));
   for (int q = 0; q < np; ++q) {
     SProb &P = probs[q];
     const Spec &g = sp[q];
@@ -1306,9 +1306,15 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
     P.muA2 = g.plan_a2 >= 0 ? probs[g.plan_a2].muA : nullptr;
     P.sigB2 = g.plan_b2 >= 0 ? probs[g.plan_b2].sigB : nullptr;
     P.muB2 = g.plan_b2 >= 0 ? probs[g.plan_b2].muB : nullptr;
-    if (!(crt ? make_map_mn(&maps[2 * q], P.As, P.M_pad, P.K_pad, P.nsl)
-              : make_map(&maps[2 * q], P.As, P.M_pad, P.K_pad, G_BOX, P.nsl)) ||
-        !make_map(&maps[2 * q + 1], P.Bs, P.N_pad, P.K_pad, G_BOX, P.nsl)) {
+    CUtensorMap *m = &maps[nmaps * q];
+    bool made = (crt ? make_map_mn(m + GM_A, P.As, P.M_pad, P.K_pad, P.nsl)
+                     : make_map(m + GM_A, P.As, P.M_pad, P.K_pad, BM, P.nsl)) &&
+                make_map(m + GM_B, P.Bs, P.N_pad, P.K_pad, G_BOX, P.nsl);
+    if (!crt)
+      made = made && make_map(m + GM_A_BOX, P.As, P.M_pad, P.K_pad, G_BOX, P.nsl) &&
+             (P.bn < 128 || make_map(m + GM_B128, P.Bs, P.N_pad, P.K_pad, 128, P.nsl)) &&
+             (P.bn < 256 || make_map(m + GM_B256, P.Bs, P.N_pad, P.K_pad, 256, P.nsl));
+    if (!made) {
       destroy(b);
       return MFCUDA_ERR_CUDA;
     }
@@ -1329,7 +1335,7 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
   if (np > 0 && (cudaMemcpy(dp, probs.data(), sizeof(SProb) * np, cudaMemcpyHostToDevice) != cudaSuccess ||
                  cudaMemcpy(dprefix, prefix.data(), sizeof(int64_t) * np, cudaMemcpyHostToDevice) != cudaSuccess ||
                  !copied ||
-                 cudaMemcpy(dmaps, maps.data(), sizeof(CUtensorMap) * 2 * np, cudaMemcpyHostToDevice) !=
+                 cudaMemcpy(dmaps, maps.data(), sizeof(CUtensorMap) * nmaps * np, cudaMemcpyHostToDevice) !=
                      cudaSuccess)) {
     destroy(b);
     return MFCUDA_ERR_CUDA;
