@@ -201,6 +201,7 @@ struct SProb {
   Plan *plan;
   int crt;       // CRT form (crt_device.cuh): slices are residues, items single products
   int nsl;       // slice slots per operand: SMAX digits, or the most moduli the CRT plan can use
+  int diags;     // diagonals of an item (CRT: 1, the product of one modulus)
   CrtConst *cc;  // the plan's reconstruction constants (CRT form)
 };
 // phases with a per-problem block count (and the items, with their prefix sums); the
@@ -394,19 +395,25 @@ __device__ __forceinline__ void load_b(uint8_t *dst, const CUtensorMap *m, uint6
   if (nb >= 2) mftc::tma_load_3d(dst, m + GM_B128, bar, k, b_row, slice);
   if (nb & 1) mftc::tma_load_3d(dst + (nb - 1) * G_BOX * BK, m + GM_B, bar, k, b_row + (nb - 1) * G_BOX, slice);
 }
-// Diagonals of an item of the digit-sliced form.
+// Diagonals of an item of the digit-sliced form: two, or one in a batch that has at
+// most 1.5 single ones per SM (`items` of them).  There the longest item sets the
+// time, and half of it is gone with the second diagonal; with more items the loads
+// that two diagonals share count for more.  B200, two -> one, us: 512^3 82 -> 71, 5 of
+// 100 x 500 x 200 (0.5 per SM) 82 -> 70, 11 of 128^3 (1.04) 55 -> 53, complex 512^3 of
+// 6 slices (1.3) 103 -> 98; 16 of 128^3 (1.5) 55 -> 59, 42 of 200 x 1000 x 300 (16) 651 -> 714.
 constexpr int GD_DIAGS = 2;
-__host__ __device__ constexpr int g_groups(int nsl, bool crt) { return crt ? nsl : (nsl + GD_DIAGS - 1) / GD_DIAGS; }
+static int digit_diags(int64_t items) { return 2 * items <= 3 * (int64_t)sm_count() ? 1 : GD_DIAGS; }
+__host__ __device__ constexpr int g_groups(int nsl, int diags) { return (nsl + diags - 1) / diags; }
 // A block per problem: its items, the longest first.
 __global__ void __launch_bounds__(128) g_items(const SProb *probs, const int64_t *prefix, GItem *items) {
   const SProb &P = probs[blockIdx.x];
-  const int G = P.plan->G, ntiles = P.ntm * P.ntn, per_g = P.nkc * ntiles, groups = g_groups(P.nsl, P.crt != 0);
+  const int G = P.plan->G, ntiles = P.ntm * P.ntn, per_g = P.nkc * ntiles, groups = g_groups(P.nsl, P.diags);
   for (int64_t l = threadIdx.x; l < (int64_t)groups * per_g; l += blockDim.x) {
     GItem it;
     const int q = (int)(l / per_g), r = (int)(l % per_g), kc = r / ntiles, tile = r % ntiles;
     it.p = (int)blockIdx.x;
-    it.g = P.crt ? P.nsl - 1 - q : G - GD_DIAGS * q;
-    it.nd = P.crt ? (it.g <= G ? 1 : 0) : max(0, min(GD_DIAGS, it.g + 1));
+    it.g = P.crt ? P.nsl - 1 - q : G - P.diags * q;
+    it.nd = P.crt ? (it.g <= G ? 1 : 0) : max(0, min(P.diags, it.g + 1));
     it.kb0 = kc * P.kcb;
     it.kb1 = min(P.kblocks, it.kb0 + P.kcb);
     it.a_row = tile % P.ntm * BM;
@@ -615,8 +622,8 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   }
 }
 
-// Persistent tensor-core kernel of the digit-sliced form.  An item is two
-// consecutive diagonals g, g - 1 of one tile (128 rows x bn <= 256 columns) and
+// Persistent tensor-core kernel of the digit-sliced form.  An item is one diagonal g
+// (digit_diags), or two consecutive ones g, g - 1, of one tile (128 rows x bn <= 256 columns) and
 // K chunk, accumulated side by side in tensor memory.  Per K block the slices
 // come in the order A_0, B_g, B_{g-1}, A_1, B_{g-2}, ...: step s multiplies A_s
 // with B_{g-s} and B_{g-s-1}, one product per diagonal, and then lets A_s and
@@ -1175,6 +1182,12 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
   std::vector<int64_t> prefix((size_t)std::max(np, 1), 0);  // of the items
   std::vector<Owner> owner[PH_ITEMS];                         // of the blocks of the other phases
   int64_t total[PH_COUNT] = {0, 0, 0, 0, 0, 0, 0};
+  int64_t singles = 0;  // items of one diagonal each, at the most slices a plan may take
+  for (const Spec &g : sp) {
+    const int64_t kblocks = ru(g.k < 1 ? 1 : g.k, BK) / BK, kcb = std::min(kcb_all, KC_BLOCKS);
+    singles += (slices > 0 ? slices : SMAX) * ((kblocks + kcb - 1) / kcb) * (ru(g.m, BM) / BM) * (ru(g.n, g.bn) / g.bn);
+  }
+  const int diags = crt ? 1 : digit_diags(singles);
   for (int q = 0; q < np; ++q) {
     const Spec &g = sp[q];
     SProb &P = probs[q];
@@ -1202,6 +1215,7 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
     P.ntn = (int)(P.N_pad / P.bn);
     P.crt = crt ? 1 : 0;
     P.nsl = crt ? crt_slices_max(g.k < 1 ? 1 : g.k, slices) : SMAX;
+    P.diags = diags;
     P.cc = nullptr;
     if (P.own_plan) {
       o_plan[q] = ar.take(sizeof(Plan));
@@ -1227,7 +1241,7 @@ static int create_split_specs(std::vector<Spec> specs, int64_t count, int slices
         P.own_b ? (P.n * (k_fill(P.k) / 8) + 255) / 256 : 0,
         P.mode == 0 ? comb : 0,
         P.mode != 0 ? comb : 0,
-        (int64_t)g_groups(P.nsl, crt) * P.nkc * P.ntm * P.ntn};
+        (int64_t)g_groups(P.nsl, P.diags) * P.nkc * P.ntm * P.ntn};
     prefix[q] = total[PH_ITEMS];
     for (int ph = 0; ph < PH_COUNT; ++ph) {
       total[ph] += blocks[ph];
