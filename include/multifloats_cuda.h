@@ -393,8 +393,8 @@ MULTIFLOATS_CUDA_API int mfcuda_reduce_combine(int kind, const void *parts, int6
  *     tile shape of 64x64, 32x32 or 16x16 outputs.  renorm_interval as in
  *     matmuldd_mm; slices/target unused.
  *   form MFCUDA_FORM_SPLIT: the split-INT8 pipeline, each phase one grouped
- *     launch; one persistent tcgen05 kernel over every (diagonal, K chunk, tile)
- *     item of every problem; per problem a tile width N of 256, 128 or 64 and a
+ *     launch; one persistent tcgen05 kernel over every item (one or two diagonals
+ *     of a K chunk and tile) of every problem; per problem a tile width N of 256, 128 or 64 and a
  *     shared K chunk (split-K when the batch is too small to fill the GPU);
  *     slices/target as in mfcuda_matmuldd_mm_split.  Operands 16-byte aligned.
  *   form MFCUDA_FORM_CRT: the CRT (modular) split pipeline of

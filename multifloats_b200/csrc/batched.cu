@@ -11,10 +11,12 @@
 //    bit-identical to matmuldd_mm.
 //  * split-INT8 DD GEMMs: each phase of the split pipeline (exponent scan,
 //    plan, slicing, tcgen05 MMA, recombination) is one grouped launch over all
-//    problems; the tensor-core phase is one persistent kernel whose work list
-//    holds every (diagonal, K chunk, tile) item of every problem.  Per problem:
-//    slice count from its plan, tile width N (256/128/64) and K chunk from the
-//    autotuner.  Results are bit-identical to mfcuda_matmuldd_mm_split.
+//    problems; the tensor-core phase is one persistent kernel whose work list,
+//    written on the device from the plans, holds every problem's items: one or
+//    two diagonals (digits) or one modulus (CRT) of a K chunk and tile.  Per
+//    problem: slice count from its plan, tile width N (256/128/64) from the
+//    autotuner; one K chunk for the whole plan.  Results are bit-identical to
+//    mfcuda_matmuldd_mm_split with that K chunk.
 //  * ragged elementwise arrays: one grid-stride launch over the concatenated
 //    index space.
 //
@@ -204,11 +206,11 @@ struct SProb {
   int diags;     // diagonals of an item (CRT: 1, the product of one modulus)
   CrtConst *cc;  // the plan's reconstruction constants (CRT form)
 };
-// phases with a per-problem block count (and the items, with their prefix sums); the
-// recombination runs in two launches: stores first, then the - / + updates
 // K indices whose digits or residues the tensor cores read: whole steps of 32.
 __host__ __device__ constexpr int64_t k_fill(int64_t k) { return k < 1 ? 32 : (k + 31) / 32 * 32; }
 
+// phases with a per-problem block count (and the items, with their prefix sums); the
+// recombination runs in two launches: stores first, then the - / + updates
 enum { PH_SCAN_A, PH_SCAN_B, PH_SLICE_A, PH_SLICE_B, PH_COMBINE, PH_COMBINE2, PH_ITEMS, PH_COUNT };
 
 // A block's problem and its index among the problem's blocks of the phase, from
@@ -1665,9 +1667,11 @@ static std::vector<int> choose(int form, const mfcuda_gemm_desc *d, int64_t coun
 }
 
 // Split-K rule: K chunks of at most KC_BLOCKS blocks (the INT32 bound); when
-// the whole batch has fewer items than four per SM, shorter chunks raise the
-// item count (the chunks' INT32 partials are summed exactly in the combine).
-// nsl(k): slice slots (and so items per tile) of a product with inner size k.
+// the whole batch has fewer than four products of one diagonal or modulus per SM,
+// shorter chunks raise their number (the chunks' INT32 partials are summed exactly
+// in the combine).  The results depend on the chunk (the combine rounds once per
+// chunk), so it follows from shapes alone and not from how many diagonals an item has.
+// nsl(k): slice slots (and so products per tile) of a product with inner size k.
 template <class SlotFn>
 static int choose_kcb(const mfcuda_gemm_desc *d, int64_t count, const std::vector<int> &cfg, int prods, SlotFn nsl) {
   int64_t items = 0, kmax = 1;

@@ -127,7 +127,7 @@ __device__ __forceinline__ dd dd_div(dd x, dd y) {
 }
 
 // ---- the operators' general paths, for operands known to take them -----------
-// dd_add / dd_sub / dd_mul without the short-circuit tests: bit-identical where
+// dd_add / dd_mul without the short-circuit tests: bit-identical where
 // the leading sum or product is finite and (addition) the two high limbs are
 // not both zero.  dd_add_ord needs |x.hi| >= |y.hi| besides: 17 FP64
 // instructions instead of 20.  The polynomial kernels of exp, log, sin and cos
@@ -148,7 +148,6 @@ __device__ __forceinline__ dd dd_add_gen(dd x, dd y) {
   two_sum(x.lo, y.lo, c, d);
   return dd_add_tail(a, b, c, d);
 }
-__device__ __forceinline__ dd dd_sub_gen(dd x, dd y) { return dd_add_gen(x, neg(y)); }
 __device__ __forceinline__ dd dd_add_ord(dd x, dd y) {
   double a, b, c, d;
   two_sum_ord(x.hi, y.hi, a, b);

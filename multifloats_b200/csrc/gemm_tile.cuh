@@ -14,8 +14,9 @@
 // issue cycles each.  The steps run in branch-free groups of eight: with the
 // chunk counter tested after every step the accumulators had to sit in fixed
 // registers at each merge, and the moves that took (8 of 26 issue cycles per
-// MAC) were paid on top of the FP64 issue -- 4096^3 66.6 -> 56.8 ms, FP64 pipe
-// 88 % busy.  An interval that is not a multiple of eight runs from chunk end
+// MAC) were paid on top of the FP64 issue -- 4096^3 66.6 -> 56.8 ms, 16.6 of the
+// pipe's 18.6 T instructions/s (64 a cycle and SM at 1.965 GHz; a chain-free loop
+// of multiply-adds alone reaches 17.1).  An interval that is not a multiple of eight runs from chunk end
 // to chunk end in a counted loop; the shortest ones have kernels of their own.
 #pragma once
 #include "dd_device.cuh"
