@@ -39,8 +39,10 @@ def test_diagonals(dev, slices, more, cplx):
         out = [to_host(p[2]) for p in probs[:len(SHAPES)]]
         kc = api.lib().mfcuda_batch_kchunk(plan._plan)
         items = api.lib().mfcuda_batch_work_items(plan._plan)
+        width = [api.lib().mfcuda_batch_config(plan._plan, i) for i in range(len(probs))]
     # groups of diagonals over the 14 slices there may be: 14 of one, 7 of two
-    tiles = (4 if cplx else 1) * (1 + 2 * -(-600 // kc) + 1 + more)
+    tiles = (4 if cplx else 1) * sum(-(-m // 128) * -(-n // width[i]) * -(-k // kc)
+                                     for i, (_, _, _, m, k, n) in enumerate(probs))
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     assert items == tiles * (14 if 2 * tiles * (slices or 14) <= 3 * sms else 7)
     for (m, k, n), (a, b), got in zip(SHAPES, host, out):
