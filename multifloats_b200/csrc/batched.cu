@@ -398,13 +398,16 @@ __device__ __forceinline__ void load_b(uint8_t *dst, const CUtensorMap *m, uint6
   if (nb & 1) mftc::tma_load_3d(dst + (nb - 1) * G_BOX * BK, m + GM_B, bar, k, b_row + (nb - 1) * G_BOX, slice);
 }
 // Diagonals of an item of the digit-sliced form: two, or one in a batch that has at
-// most 1.5 single ones per SM (`items` of them).  There the longest item sets the
-// time, and half of it is gone with the second diagonal; with more items the loads
-// that two diagonals share count for more.  B200, two -> one, us: 512^3 82 -> 71, 5 of
-// 100 x 500 x 200 (0.5 per SM) 82 -> 70, 11 of 128^3 (1.04) 55 -> 53, complex 512^3 of
-// 6 slices (1.3) 103 -> 98; 16 of 128^3 (1.5) 55 -> 59, 42 of 200 x 1000 x 300 (16) 651 -> 714.
+// most five single ones per SM (`items` of them).  Two share their loads and take 7/8
+// of the time of two single items where a batch is long; but the longest item, which
+// by chance starts last, is 1.75 times as long as a single one, and in a short batch
+// that counts for more: with the mean item half as long as the longest, up to
+// five or six per SM.  260 random batches, one against two by single items per SM: up to 1
+// 0.93, 1 to 3 0.96, 3 to 5 0.97, 5 to 7 1.00, 7 to 17 1.05.  B200, two -> one, us: 512^3
+// 82 -> 71, 5 of 100 x 500 x 200 (0.5) 82 -> 70, 4 of 465 x 559 x 22 (3) 109 -> 94, 42
+// of 200 x 1000 x 300 (16) 651 -> 714.
 constexpr int GD_DIAGS = 2;
-static int digit_diags(int64_t items) { return 2 * items <= 3 * (int64_t)sm_count() ? 1 : GD_DIAGS; }
+static int digit_diags(int64_t items) { return items <= 5 * (int64_t)sm_count() ? 1 : GD_DIAGS; }
 __host__ __device__ constexpr int g_groups(int nsl, int diags) { return (nsl + diags - 1) / diags; }
 // A block per problem: its items, the longest first.
 __global__ void __launch_bounds__(128) g_items(const SProb *probs, const int64_t *prefix, GItem *items) {
