@@ -643,17 +643,16 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 // each to the other roles through a small ring in shared memory): dealt round
 // robin the busiest CTA had 16 % more work than the mean.
 //
-// Bound: the operands from L2 (45 GB for 2000 products up to 1024: 7.5 of about
-// 9 TB/s; the MMAs alone would take 2.6 ms), then the drain, hidden only
+// Bound: the operands from L2 (45 GB for 2000 products up to 1024: 10 TB/s; the MMAs
+// alone would take 2.6 ms of the 4.5), then the drain, hidden only
 // behind the next item's loads (the accumulators fill tensor memory; they are
 // handed back one by one in the order the next item needs them).  Four
 // diagonals on 128 x 128 tiles load less, but a 128-column MMA takes 102 cycles
 // instead of its 64 (shared-memory reads).  2000 products of sizes up to 1024:
 // 9.0 ms with one diagonal at a time and items found by bisection, 7.8 four by
 // 128 columns, 6.0 two by 256.  With barriers and commits of their own for A and B
-// a step cost 0.2 us more (the second commit waits for the tensor pipe once again):
-// the 2000 products, whole batch, 10.26 -> 9.18 ms with one; 100 x 500 x 200 alone,
-// this kernel, 52 -> 41 us.
+// a step cost 0.2 us more: 5.65 -> 4.50 ms with one (under ncu, both); 100 x 500 x 200
+// alone 52 -> 41 us.
 constexpr int GD_BN = BN, GD_NA = 4, GD_NB = 5, GD_NW = 4;
 constexpr int GD_TILE_A = A_STAGE, GD_TILE_B = B_STAGE;  // bytes of a slot
 constexpr int GD_SMEM = GD_NA * GD_TILE_A + GD_NB * GD_TILE_B + 1024 /*align*/ + 512 /*barriers, items*/;
